@@ -72,7 +72,7 @@ int mode_number(int i, int n, ModeConvention conv = kModesP2) {
 }
 
 std::vector<double2> twiddles(int n) {
-    std::vector<double2> t(n > 1 ? n / 2 : 1);
+    std::vector<double2> t(n);
     for (int m = 0; m < (int)t.size(); ++m) {
         const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)m / (long double)n;
         t[m] = make_double2((double)cosl(a), (double)sinl(a));
@@ -419,14 +419,67 @@ PushArgs push_args(upic_ctx* c, const ParticleSoA& p, long np, bool uniform) {
     return a;
 }
 
+// Fields are paired in the transforms of the FP64 form on grids of at least
+// two cells along each axis (explicit.cu).  The mixed form transforms them one
+// by one: a different rounding of the FP64 spectra would move single FP32
+// node records by an ulp, and the particles with them.
+KGrid kgrid(const upic_ctx* c) {
+    return KGrid{c->nx, c->ny, c->lny, c->nx > 1 && c->ny > 1 && !c->mixed, c->d_kx, c->d_ky, c->d_k2};
+}
+
+// Transforms of the deposited fields and of the gathered ones (explicit.cu
+// bdf_kspace_kernel): pairs of real fields, or one by one on a grid one cell
+// high or wide.  Returns their number.
+int current_map(const upic_ctx* c, FftMap& m) {
+    m = fft_identity_map(3);
+    if (!paired_grid(kgrid(c))) return 3;
+    m.im[0] = 1;
+    m.re[1] = 2;
+    return 2;
+}
+int gather_map(const upic_ctx* c, FftMap& m) {
+    m = fft_identity_map(kGF);
+    if (!paired_grid(kgrid(c))) return kGF;
+    const signed char re[6] = {0, 2, 3, 5, 7, 9}, im[6] = {1, -1, 4, 6, 8, 10};
+    for (int k = 0; k < 6; ++k) {
+        m.re[k] = re[k];
+        m.im[k] = im[k];
+    }
+    return 6;
+}
+
+// J^n (and rho^n with `charge`) of the accumulators and their spectra.
+int transform_deposit(upic_ctx* c, bool charge) {
+    FftAccIn in{};
+    in.acc = c->d_acc;
+    for (int k = 0; k < 4; ++k) in.scale[k] = c->scale[k];
+    in.J = c->d_J;
+    in.rho = c->d_rho;
+    in.n0 = c->cfg.n0;
+    in.bg = c->d_bg;
+    in.single = c->mixed ? 1 : 0;
+    FftMap m;
+    int n = current_map(c, m);
+    if (charge) {
+        // the charge goes to slot 3 of the spectra: transform 2 when paired
+        m.re[n] = 3;
+        m.im[n] = -1;
+        ++n;
+    }
+    UPIC_CUDA(c, fft2d_from_acc(c->plan, c->d_spec, n, m, in, c->st));
+    return 0;
+}
+
+// Spectrum of the naive charge after transform_deposit(c, true).
+const double2* charge_spectrum(const upic_ctx* c) {
+    return c->d_spec + (paired_grid(kgrid(c)) ? 2 : 3) * (size_t)c->N;
+}
+
 // Diagnostics row of the current spectra (hist slot_new with derivatives
 // against slot_prev0) into c->h_row.
-int run_diag(upic_ctx* c, int slot_new, int slot_prev0, int na, const double* acoef) {
-    DiagKArgs d{};
-    d.N = c->N;
-    d.kx = c->d_kx;
-    d.ky = c->d_ky;
-    d.k2 = c->d_k2;
+DiagArgs diag_args(upic_ctx* c, int slot_new, int slot_prev0, int na, const double* acoef) {
+    DiagArgs d{};
+    d.g = kgrid(c);
     d.Jhat = c->d_spec;
     d.hist = c->d_hist;
     d.R = kHistSlots;
@@ -437,25 +490,20 @@ int run_diag(upic_ctx* c, int slot_new, int slot_prev0, int na, const double* ac
     d.dt = c->cfg.dt;
     d.c = c->cfg.c;
     d.eps0 = c->cfg.eps0;
-    d.out = c->d_dspec;
-    UPIC_CUDA(c, launch_diag_kspace(d, c->st));
-    UPIC_CUDA(c, fft2d_batched(c->plan, c->d_dspec, kDiagFields, 1, c->st, nullptr, 1, c->d_dreal));
-    DiagReduceArgs r{};
-    r.N = c->N;
-    r.dfields = c->d_dreal;
-    r.J = c->d_J;
-    r.partials = c->d_partials;
-    r.grid = kRedGrid;
-    r.pdiag = c->d_pdiag;
-    r.pcount = c->push_grid;
-    r.np = c->np;
-    r.dA = c->dA;
-    r.eps0 = c->cfg.eps0;
-    r.mu0 = c->cfg.mu0;
-    r.row = c->d_row;
-    UPIC_CUDA(c, launch_diag_reduce(r, c->st));
-    UPIC_CUDA(c, cudaMemcpyAsync(c->h_row, c->d_row, sizeof(double) * UPIC_DIAG_COUNT,
-                                 cudaMemcpyDeviceToHost, c->st));
+    d.mu0 = c->cfg.mu0;
+    d.dA = c->dA;
+    return d;
+}
+int run_diag(upic_ctx* c, int slot_new, int slot_prev0, int na, const double* acoef) {
+    DiagArgs d = diag_args(c, slot_new, slot_prev0, na, acoef);
+    d.partials = c->d_partials;
+    d.max_blocks = kRedGrid;
+    d.done = c->d_done;
+    d.pdiag = c->d_pdiag;
+    d.pcount = c->push_grid;
+    d.np = c->np;
+    d.row = c->h_row;
+    UPIC_CUDA(c, launch_diag_reduce(d, c->st));
     return 0;
 }
 
@@ -737,7 +785,7 @@ int upic_create(const upic_config* cfg, upic_ctx** out) {
         (rc = dalloc(c, &c->d_dreal, (size_t)kDiagFields * N)) ||
         (rc = dalloc(c, &c->d_partials, (size_t)kRedGrid * 16)) ||
         (rc = dalloc(c, &c->d_pdiag, (size_t)c->push_grid * kDiagPart)) ||
-        (rc = dalloc(c, &c->d_row, UPIC_DIAG_COUNT)) || (rc = dalloc(c, &c->d_scan, 3)) ||
+        (rc = dalloc(c, &c->d_done, 1)) || (rc = dalloc(c, &c->d_scan, 3)) ||
         (c->mixed && (rc = dalloc(c, &c->d_gf32, (size_t)kGFStride * N))))
         return bail(rc);
     if (cudaMallocHost(&c->h_row, sizeof(double) * UPIC_DIAG_COUNT) != cudaSuccess ||
@@ -767,6 +815,7 @@ int upic_create(const upic_config* cfg, upic_ctx** out) {
         cudaMemcpy(c->d_kx, kx.data(), sizeof(double) * N, cudaMemcpyHostToDevice) ||
         cudaMemcpy(c->d_ky, ky.data(), sizeof(double) * N, cudaMemcpyHostToDevice) ||
         cudaMemcpy(c->d_k2, k2.data(), sizeof(double) * N, cudaMemcpyHostToDevice) ||
+        cudaMemset(c->d_done, 0, sizeof(unsigned)) ||
         cudaMemset(c->d_acc, 0, sizeof(unsigned long long) * 8 * (size_t)N))
         return bail(fail(c, UPIC_ERR_CUDA, "initial device copies failed"));
     c->plan.nx = c->nx;
@@ -1230,7 +1279,9 @@ int upic_init_fields(upic_ctx* c, double* diag_row) {
     UPIC_CUDA(c, launch_fill_hist(H + 4 * fs, kHistSlots, N, sp + 3 * (size_t)N, c->st));
     c->head = 0;
     // J0 spectra for the step-0 diagnostics
-    UPIC_CUDA(c, fft2d_batched(c->plan, sp, 3, 0, c->st, c->d_J));
+    FftMap jmap;
+    const int jn = current_map(c, jmap);
+    UPIC_CUDA(c, fft2d_mapped(c->plan, sp, jn, jmap, 0, c->st, c->d_J, 0, nullptr, 0, 0));
     if (diag_row) {
         const double a1[3] = {1.0, -1.0, 0.0};
         if ((rc = run_diag(c, c->head, c->head, 2, a1))) return rc;
@@ -1279,26 +1330,15 @@ int explicit_advance(upic_ctx* c, int nsteps, int diag_stride, double* diag, boo
             if ((rc = sort_active(c, c->cfg.dt))) return rc;
         }
         // J^n (and rho^n) were deposited by the previous particle kernel
-        if (c->mixed)
-            UPIC_CUDA(c, launch_convert_acc1(c->d_acc, N, c->scale, c->d_J, c->d_rho, c->cfg.n0, naive ? 3 : 1,
-                                             c->st, c->d_bg));
-        else
-            UPIC_CUDA(c, launch_convert_acc(c->d_acc, N, c->scale, c->d_J, c->d_rho, c->cfg.n0, naive ? 3 : 1,
-                                            c->st, c->d_bg));
-        UPIC_CUDA(c, fft2d_batched(c->plan, sp, 3, 0, c->st, c->d_J));
-        if (naive) UPIC_CUDA(c, fft2d_batched(c->plan, sp + 3 * (size_t)N, 1, 0, c->st, c->d_rho));
+        if ((rc = transform_deposit(c, naive))) return rc;
         KspaceArgs k{};
-        k.N = N;
-        k.kx = c->d_kx;
-        k.ky = c->d_ky;
-        k.k2 = c->d_k2;
+        k.g = kgrid(c);
         k.Jhat = sp;
-        k.rho_dep = naive ? sp + 3 * (size_t)N : nullptr;
+        k.rho_dep = naive ? charge_spectrum(c) : nullptr;
         k.hist = c->d_hist;
         k.R = kHistSlots;
         k.head = c->head;
         k.na = na;
-        k.nb = nb;
         for (int i = 0; i < 3; ++i) k.a[i] = a[i];
         for (int i = 0; i < 5; ++i) k.b[i] = b[i];
         k.dt = c->cfg.dt;
@@ -1308,12 +1348,10 @@ int explicit_advance(upic_ctx* c, int nsteps, int diag_stride, double* diag, boo
         k.conserving = naive ? 0 : 1;
         k.gspec = sp + 4 * (size_t)N;
         UPIC_CUDA(c, launch_bdf_kspace(k, c->st));
-        if (c->mixed)
-            UPIC_CUDA(c, fft2d_batched(c->plan, sp + 4 * (size_t)N, kGF, 1, c->st, nullptr, 3,
-                                       reinterpret_cast<double*>(c->d_gf32), kGFStride, 0));
-        else
-            UPIC_CUDA(c, fft2d_batched(c->plan, sp + 4 * (size_t)N, kGF, 1, c->st, nullptr, 2, c->d_gf,
-                                       kGFStride, 0));
+        FftMap gmap;
+        const int gn = gather_map(c, gmap);
+        UPIC_CUDA(c, fft2d_mapped(c->plan, k.gspec, gn, gmap, 1, c->st, nullptr, c->mixed ? 3 : 2,
+                                  c->mixed ? static_cast<void*>(c->d_gf32) : static_cast<void*>(c->d_gf), kGFStride, 0));
         if (c->np > 0) {
             if ((rc = launch_push(c, kModePush, grid_ncomp(c), c->P[c->cur], c->np, c->uniform_qm, c->sw,
                                   c->d_pdiag)))
@@ -1418,26 +1456,10 @@ int upic_get_field(upic_ctx* c, int which, double* host) {
             bdf_coeffs(c->cfg.method, na, a, nb, b);
             prev = (c->head + 1) % kHistSlots;
         }
-        DiagKArgs d{};
-        d.N = N;
-        d.kx = c->d_kx;
-        d.ky = c->d_ky;
-        d.k2 = c->d_k2;
-        d.Jhat = c->d_spec;
-        d.hist = c->d_hist;
-        d.R = kHistSlots;
-        d.slot_new = c->head;
-        d.slot_prev0 = prev;
-        d.na = na;
-        for (int k = 0; k < 3; ++k) d.a[k] = a[k];
-        d.dt = c->cfg.dt;
-        d.c = c->cfg.c;
-        d.eps0 = c->cfg.eps0;
-        d.out = c->d_dspec;
-        UPIC_CUDA(c, launch_diag_kspace(d, c->st));
-        // diag_kspace output slots: E 1..3, B 6..8
+        const DiagArgs d = diag_args(c, c->head, prev, na, a);
         const int slot = which <= UPIC_FIELD_EZ ? 1 + which - UPIC_FIELD_EX : 6 + which - UPIC_FIELD_BX;
-        UPIC_CUDA(c, fft2d_batched(c->plan, c->d_dspec + (size_t)slot * N, 1, 1, c->st, nullptr, 1, c->d_dreal));
+        UPIC_CUDA(c, launch_diag_field(d, slot, c->d_dspec, c->st));
+        UPIC_CUDA(c, fft2d_batched(c->plan, c->d_dspec, 1, 1, c->st, nullptr, 1, c->d_dreal));
         UPIC_CUDA(c, cudaMemcpyAsync(host, c->d_dreal, sizeof(double) * N, cudaMemcpyDeviceToHost, c->st));
         return sync(c);
     }

@@ -74,9 +74,9 @@ struct upic_ctx {
     double* d_dreal = nullptr;
     double* d_partials = nullptr;
     double* d_pdiag = nullptr;
-    double* d_row = nullptr;
+    unsigned* d_done = nullptr;  // finished blocks of the diagnostics reduction (zero between launches)
     double* d_bg = nullptr;   // fixed background charge (upic_set_background) or null: uniform n0
-    double* h_row = nullptr;  // pinned
+    double* h_row = nullptr;  // pinned; the diagnostics reduction writes it
     // particle-state scan of upic_set_particles (non-finite count, largest
     // speed and velocity component bits): device words and their pinned copy
     unsigned long long* d_scan = nullptr;

@@ -511,135 +511,222 @@ UPIC_D double2 cscale(double s, double2 a) { return make_double2(s * a.x, s * a.
 // i*k*z
 UPIC_D double2 cik(double k, double2 z) { return make_double2(-k * z.y, k * z.x); }
 
+// ---- k-space step -----------------------------------------------------------
+// Real fields travel in pairs through the transforms: spectrum Z = F + i G of
+// two real fields gives F(k) = (Z(k) + conj Z(-k)) / 2 and
+// G(k) = (Z(k) - conj Z(-k)) / 2i, and the inverse transform of F + i G has F
+// in its real and G in its imaginary part.  A grid one cell high or wide is
+// not paired: its wave number there is that of mode -1
+// (spectral_pic_part3.cpp:320-330), so a derivative's spectrum is not that of
+// a real field and only the real part of each transform is wanted.
+UPIC_D double2 pair_re(double2 z, double2 m) { return make_double2(0.5 * (z.x + m.x), 0.5 * (z.y - m.y)); }
+UPIC_D double2 pair_im(double2 z, double2 m) { return make_double2(0.5 * (z.y + m.y), 0.5 * (m.x - z.x)); }
+// (i kx - ky) z: the pair of i kx z and i ky z
+UPIC_D double2 cgrad(double kx, double ky, double2 z) {
+    return make_double2(-kx * z.y - ky * z.x, kx * z.x - ky * z.y);
+}
+
+// Node (i, j)'s wave numbers from the axes' own rows and columns of the
+// grid-sized tables (16 B per node less to read): kx depends on i alone, ky
+// on j, and k2 = k2(i, 0) + k2(0, j) is the sum the host rounds.
+// The BDF combinations' roundings are written out: u - s h in one, so that
+// no instance of the kernel contracts them differently (the mixed form's FP32
+// records depend on them bit for bit).
+UPIC_D double2 cmul_add(double s, double2 h, double2 u) {
+    return make_double2(__fma_rn(s, h.x, u.x), __fma_rn(s, h.y, u.y));
+}
+
+struct Wave {
+    double kx, ky, k2;
+    int mirror;  // node of -k
+};
+UPIC_D Wave wave_at(const KGrid& g, int id) {
+    const int i = id >> g.lny, j = id & (g.ny - 1);
+    Wave w;
+    w.kx = __ldg(g.kx + (i << g.lny));
+    w.ky = __ldg(g.ky + j);
+    w.k2 = g.nx > 1 && g.ny > 1 ? __dadd_rn(__ldg(g.k2 + (i << g.lny)), __ldg(g.k2 + j)) : __ldg(g.k2 + id);
+    w.mirror = (((g.nx - i) & (g.nx - 1)) << g.lny) + ((g.ny - j) & (g.ny - 1));
+    return w;
+}
+
+// Current spectra of mode id.  Paired: transform 0 carries (Jx, Jy), 1 Jz.
+template <bool PAIRED>
+UPIC_D void current_at(const double2* __restrict__ Jhat, int N, int id, int mirror, double2* J) {
+    if (PAIRED) {
+        const double2 z = Jhat[id], m = Jhat[mirror];
+        J[0] = pair_re(z, m);
+        J[1] = pair_im(z, m);
+        J[2] = pair_re(Jhat[N + id], Jhat[N + mirror]);
+    } else {
+        for (int c = 0; c < 3; ++c) J[c] = Jhat[(size_t)c * N + id];
+    }
+}
+
 // k-space BDF step: continuity / naive charge, BDF Helmholtz solves for phi
 // and A (spectral_pic_part3.cpp:829-880, 1147-1164), spectra of the eleven
-// gathered fields (:1166-1168).
-__global__ void bdf_kspace_kernel(KspaceArgs a) {
-    const int N = a.N;
+// gathered fields (:1166-1168), in six transforms when paired: (Ax, Ay), Az,
+// grad phi, grad Ax, grad Ay, grad Az (fields that vanish together share a
+// transform, so a zero component stays exactly zero).  NA: BDF coefficients
+// (2 or 3; the Helmholtz solves take 2 NA - 1), which fixes the number of
+// history slots, so that all loads of a mode are in flight together.
+template <int NA, bool PAIRED>
+__global__ void __launch_bounds__(128) bdf_kspace_kernel(KspaceArgs a) {
+    constexpr int NB = 2 * NA - 1;
+    const int N = a.g.nx * a.g.ny;
     const double scale = 1.0 / (a.c * a.c * a.dt * a.dt);
-    const int snew = (a.head + a.R - 1) % a.R;
+    const int snew = a.head == 0 ? a.R - 1 : a.head - 1;
+    size_t slot[NB - 1];
+#pragma unroll
+    for (int l = 0; l < NB - 1; ++l) slot[l] = (size_t)(a.head + l < a.R ? a.head + l : a.head + l - a.R) * N;
+    const size_t FS = (size_t)a.R * N;  // one field's ring
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < N; id += gridDim.x * blockDim.x) {
-        const double kx = a.kx[id], ky = a.ky[id];
-        const double denom = scale * a.b[0] + a.k2[id];
-        const double2 J0 = a.Jhat[id], J1 = a.Jhat[N + id], J2 = a.Jhat[2 * (size_t)N + id];
-        auto H = [&](int field, int past) -> double2 {
-            const int slot = (a.head + past) % a.R;
-            return a.hist[((size_t)field * a.R + slot) * N + id];
-        };
+        const Wave w = wave_at(a.g, id);
+        const double kx = w.kx, ky = w.ky;
+        double2 J[3];
+        current_at<PAIRED>(a.Jhat, N, id, w.mirror, J);
+        double2 H[4][NB - 1];
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+#pragma unroll
+            for (int l = 0; l < NB - 1; ++l) H[f][l] = a.hist[f * FS + slot[l] + id];
         double2 rho_new;
         if (a.conserving) {
-            const double2 div = cik(1.0, make_double2(kx * J0.x + ky * J1.x, kx * J0.y + ky * J1.y));
+            const double2 div = cik(1.0, make_double2(kx * J[0].x + ky * J[1].x, kx * J[0].y + ky * J[1].y));
             double2 hs = make_double2(0.0, 0.0);
-            for (int l = 1; l < a.na; ++l) hs = cadd(hs, cscale(a.a[l], H(4, l - 1)));
-            const double2 num = cadd(cscale(a.dt, div), hs);
+#pragma unroll
+            for (int l = 1; l < NA; ++l) hs = cmul_add(a.a[l], a.hist[4 * FS + slot[l - 1] + id], hs);
+            const double2 num = cmul_add(a.dt, div, hs);
             rho_new = make_double2(-num.x / a.a[0], -num.y / a.a[0]);
         } else {
-            rho_new = a.rho_dep[id];
+            rho_new = PAIRED ? pair_re(a.rho_dep[id], a.rho_dep[w.mirror]) : a.rho_dep[id];
         }
-        // phi: (b0 s + k^2) phi = rho/eps0 - s sum b_l phi^{n+1-l}
-        double2 rhs = make_double2(rho_new.x / a.eps0, rho_new.y / a.eps0);
-        for (int l = 1; l < a.nb; ++l) rhs = csub(rhs, cscale(scale * a.b[l], H(0, l - 1)));
-        const double2 phi = make_double2(rhs.x / denom, rhs.y / denom);
-        double2 A[3];
-        const double2 J[3] = {J0, J1, J2};
+        const double denom = scale * a.b[0] + w.k2;
+        // (b0 s + k^2) u = source - s sum b_l u^{n+1-l}: phi from rho / eps0, A from mu0 J
+        double2 u[4];
+        u[0] = make_double2(rho_new.x / a.eps0, rho_new.y / a.eps0);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            double2 r = cscale(a.mu0, J[c]);
-            for (int l = 1; l < a.nb; ++l) r = csub(r, cscale(scale * a.b[l], H(1 + c, l - 1)));
-            A[c] = make_double2(r.x / denom, r.y / denom);
+        for (int c = 0; c < 3; ++c)
+            u[1 + c] = make_double2(__dmul_rn(a.mu0, J[c].x), __dmul_rn(a.mu0, J[c].y));
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+#pragma unroll
+            for (int l = 1; l < NB; ++l) u[f] = cmul_add(-(scale * a.b[l]), H[f][l - 1], u[f]);
+            u[f] = make_double2(u[f].x / denom, u[f].y / denom);
+            a.hist[f * FS + (size_t)snew * N + id] = u[f];
         }
-        a.hist[((size_t)0 * a.R + snew) * N + id] = phi;
-        for (int c = 0; c < 3; ++c) a.hist[((size_t)(1 + c) * a.R + snew) * N + id] = A[c];
-        a.hist[((size_t)4 * a.R + snew) * N + id] = rho_new;
-        if (a.gspec) {
-            double2* g = a.gspec;
-            g[0 * (size_t)N + id] = A[0];
-            g[1 * (size_t)N + id] = A[1];
-            g[2 * (size_t)N + id] = A[2];
-            g[3 * (size_t)N + id] = cik(kx, phi);
-            g[4 * (size_t)N + id] = cik(ky, phi);
+        a.hist[4 * FS + (size_t)snew * N + id] = rho_new;
+        double2* g = a.gspec;
+        if (PAIRED) {
+            g[id] = make_double2(u[1].x - u[2].y, u[1].y + u[2].x);
+            g[(size_t)N + id] = u[3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                g[(5 + 2 * c) * (size_t)N + id] = cik(kx, A[c]);
-                g[(6 + 2 * c) * (size_t)N + id] = cik(ky, A[c]);
+            for (int f = 0; f < 4; ++f) g[(2 + f) * (size_t)N + id] = cgrad(kx, ky, u[f]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) g[(size_t)c * N + id] = u[1 + c];
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                g[(3 + 2 * f) * (size_t)N + id] = cik(kx, u[f]);
+                g[(4 + 2 * f) * (size_t)N + id] = cik(ky, u[f]);
             }
         }
     }
 }
 
-// Diagnostics spectra (spectral_pic_part3.cpp:902-948): gauge, E, gauss,
-// continuity, B = curl A, rho, using BDF first derivatives of the histories.
-__global__ void diag_kspace_kernel(DiagKArgs a) {
-    const int N = a.N;
+// ---- diagnostics --------------------------------------------------------------
+// Spectra of one mode's diagnostics fields (spectral_pic_part3.cpp:902-948):
+// gauge, E (3), gauss, continuity, B = curl A (3), rho, using BDF first
+// derivatives of the histories; J (3) after them.
+constexpr int kDiagTerms = 13;
+
+template <bool PAIRED>
+UPIC_D void diag_terms(const DiagArgs& a, int id, double2* o) {
+    const int N = a.g.nx * a.g.ny;
+    const Wave w = wave_at(a.g, id);
+    const double kx = w.kx, ky = w.ky;
+    auto H = [&](int field, int slot) -> double2 { return a.hist[((size_t)field * a.R + slot) * N + id]; };
+    auto ddt = [&](int field) -> double2 {
+        double2 r = cscale(a.a[0], H(field, a.slot_new));
+        for (int l = 1; l < a.na; ++l) {
+            const int sl = a.slot_prev0 + l - 1;
+            r = cadd(r, cscale(a.a[l], H(field, sl < a.R ? sl : sl - a.R)));
+        }
+        return make_double2(r.x / a.dt, r.y / a.dt);
+    };
+    double2* J = o + 10;
+    current_at<PAIRED>(a.Jhat, N, id, w.mirror, J);
+    const double2 phi = H(0, a.slot_new);
+    const double2 Ax = H(1, a.slot_new), Ay = H(2, a.slot_new), Az = H(3, a.slot_new);
+    const double2 rho = H(4, a.slot_new);
+    const double2 phit = ddt(0);
+    const double2 divA = cik(1.0, make_double2(kx * Ax.x + ky * Ay.x, kx * Ax.y + ky * Ay.y));
+    const double c2 = a.c * a.c;
+    o[0] = cadd(make_double2(phit.x / c2, phit.y / c2), divA);
+    const double2 Atx = ddt(1), Aty = ddt(2), Atz = ddt(3);
+    const double2 gpx = cik(kx, phi), gpy = cik(ky, phi);
+    o[1] = make_double2(-gpx.x - Atx.x, -gpx.y - Atx.y);
+    o[2] = make_double2(-gpy.x - Aty.x, -gpy.y - Aty.y);
+    o[3] = make_double2(-Atz.x, -Atz.y);
+    const double2 divE = cik(1.0, make_double2(kx * o[1].x + ky * o[2].x, kx * o[1].y + ky * o[2].y));
+    o[4] = csub(divE, make_double2(rho.x / a.eps0, rho.y / a.eps0));
+    const double2 divJ = cik(1.0, make_double2(kx * J[0].x + ky * J[1].x, kx * J[0].y + ky * J[1].y));
+    o[5] = cadd(ddt(4), divJ);
+    o[6] = cik(ky, Az);
+    o[7] = cik(-kx, Az);
+    o[8] = csub(cik(kx, Ay), cik(ky, Ax));
+    o[9] = rho;
+}
+
+// Spectrum of one diagnostics field (upic_get_field).
+template <bool PAIRED>
+__global__ void diag_field_kernel(DiagArgs a, int which, double2* out) {
+    const int N = a.g.nx * a.g.ny;
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < N; id += gridDim.x * blockDim.x) {
-        const double kx = a.kx[id], ky = a.ky[id];
-        auto H = [&](int field, int slot) -> double2 {
-            return a.hist[((size_t)field * a.R + slot) * N + id];
-        };
-        auto ddt = [&](int field) -> double2 {
-            double2 r = cscale(a.a[0], H(field, a.slot_new));
-            for (int l = 1; l < a.na; ++l) r = cadd(r, cscale(a.a[l], H(field, (a.slot_prev0 + l - 1) % a.R)));
-            return make_double2(r.x / a.dt, r.y / a.dt);
-        };
-        const double2 phi = H(0, a.slot_new);
-        const double2 Ax = H(1, a.slot_new), Ay = H(2, a.slot_new), Az = H(3, a.slot_new);
-        const double2 rho = H(4, a.slot_new);
-        const double2 phit = ddt(0);
-        const double2 divA = cik(1.0, make_double2(kx * Ax.x + ky * Ay.x, kx * Ax.y + ky * Ay.y));
-        const double c2 = a.c * a.c;
-        const double2 gauge = cadd(make_double2(phit.x / c2, phit.y / c2), divA);
-        const double2 Atx = ddt(1), Aty = ddt(2), Atz = ddt(3);
-        const double2 gpx = cik(kx, phi), gpy = cik(ky, phi);
-        const double2 Ex = make_double2(-gpx.x - Atx.x, -gpx.y - Atx.y);
-        const double2 Ey = make_double2(-gpy.x - Aty.x, -gpy.y - Aty.y);
-        const double2 Ez = make_double2(-Atz.x, -Atz.y);
-        const double2 divE = cik(1.0, make_double2(kx * Ex.x + ky * Ey.x, kx * Ex.y + ky * Ey.y));
-        const double2 gauss = csub(divE, make_double2(rho.x / a.eps0, rho.y / a.eps0));
-        const double2 J0 = a.Jhat[id], J1 = a.Jhat[N + id];
-        const double2 divJ = cik(1.0, make_double2(kx * J0.x + ky * J1.x, kx * J0.y + ky * J1.y));
-        const double2 cont = cadd(ddt(4), divJ);
-        const double2 Bx = cik(ky, Az);
-        const double2 gAzx = cik(kx, Az);
-        const double2 By = make_double2(-gAzx.x, -gAzx.y);
-        const double2 Bz = csub(cik(kx, Ay), cik(ky, Ax));
-        double2* o = a.out;
-        o[0 * (size_t)N + id] = gauge;
-        o[1 * (size_t)N + id] = Ex;
-        o[2 * (size_t)N + id] = Ey;
-        o[3 * (size_t)N + id] = Ez;
-        o[4 * (size_t)N + id] = gauss;
-        o[5 * (size_t)N + id] = cont;
-        o[6 * (size_t)N + id] = Bx;
-        o[7 * (size_t)N + id] = By;
-        o[8 * (size_t)N + id] = Bz;
-        o[9 * (size_t)N + id] = rho;
+        double2 o[kDiagTerms];
+        diag_terms<PAIRED>(a, id, o);
+        double2 r = o[0];
+#pragma unroll
+        for (int k = 1; k < 10; ++k)
+            if (k == which) r = o[k];
+        out[id] = r;
     }
 }
 
 constexpr int kRedThreads = 256;
 constexpr int kNSums = 8;  // gauge, gauss, cont, Bz, B, E, rho, J
 
-__global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagReduceArgs a) {
-    const int N = a.N;
-    const double* f = a.dfields;
+// The diagnostics row.  Sums of squares over the grid are taken in k-space,
+// sum_x f^2 = (1/N) sum_k |f_hat|^2 (Parseval; double-double, fixed order), so
+// that no field is transformed back: at 64 x 64 the ten inverse transforms,
+// the reduction over their results and its one-warp finish took 60 of a
+// step's 231 us, this launch takes about 6.  Without pairing (a one-cell
+// axis) a field is the real part of its transform, whose spectrum is
+// (f(k) + conj f(-k)) / 2.  The last block to finish adds the blocks'
+// partials and the push kernel's particle partials in index order and writes
+// the row (page-locked host memory).
+template <bool PAIRED>
+__global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagArgs a) {
+    const int N = a.g.nx * a.g.ny;
     DD s[kNSums];
 #pragma unroll
     for (int k = 0; k < kNSums; ++k) s[k] = DD{0.0, 0.0};
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < N; id += gridDim.x * blockDim.x) {
-        const double gauge = f[id], Ex = f[N + id], Ey = f[2 * (size_t)N + id];
-        const double Ez = f[3 * (size_t)N + id], gauss = f[4 * (size_t)N + id];
-        const double cont = f[5 * (size_t)N + id], Bx = f[6 * (size_t)N + id];
-        const double By = f[7 * (size_t)N + id], Bz = f[8 * (size_t)N + id];
-        const double rho = f[9 * (size_t)N + id];
-        const double Jx = a.J[id], Jy = a.J[N + id], Jz = a.J[2 * (size_t)N + id];
-        s[0] = dd_add_dd(s[0], dd_sq(gauge));
-        s[1] = dd_add_dd(s[1], dd_sq(gauss));
-        s[2] = dd_add_dd(s[2], dd_sq(cont));
-        s[3] = dd_add_dd(s[3], dd_sq(Bz));
-        s[4] = dd_add_dd(dd_add_dd(dd_add_dd(s[4], dd_sq(Bx)), dd_sq(By)), dd_sq(Bz));
-        s[5] = dd_add_dd(dd_add_dd(dd_add_dd(s[5], dd_sq(Ex)), dd_sq(Ey)), dd_sq(Ez));
-        s[6] = dd_add_dd(s[6], dd_sq(rho));
-        s[7] = dd_add_dd(dd_add_dd(dd_add_dd(s[7], dd_sq(Jx)), dd_sq(Jy)), dd_sq(Jz));
+        double2 o[kDiagTerms];
+        diag_terms<PAIRED>(a, id, o);
+        if (!PAIRED) {
+            double2 m[kDiagTerms];
+            diag_terms<PAIRED>(a, wave_at(a.g, id).mirror, m);
+#pragma unroll
+            for (int k = 0; k < kDiagTerms; ++k) o[k] = pair_re(o[k], m[k]);
+        }
+        constexpr int which[kDiagTerms] = {0, 5, 5, 5, 1, 2, 4, 4, 4, 6, 7, 7, 7};
+#pragma unroll
+        for (int k = 0; k < kDiagTerms; ++k) {
+            DD& t = s[which[k]];
+            t = dd_add_dd(dd_add_dd(t, dd_sq(o[k].x)), dd_sq(o[k].y));
+        }
+        s[3] = dd_add_dd(dd_add_dd(s[3], dd_sq(o[8].x)), dd_sq(o[8].y));
     }
     __shared__ double red[kRedThreads / kWarp][kNSums * 2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -659,24 +746,35 @@ __global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagReduceArgs
         a.partials[(size_t)blockIdx.x * 16 + 2 * threadIdx.x] = t.hi;
         a.partials[(size_t)blockIdx.x * 16 + 2 * threadIdx.x + 1] = t.lo;
     }
-}
-
-// Final reduction in a fixed order: lane l sums blocks l, l+32, ... and the
-// 32 lane sums are combined by a fixed butterfly; then thread 0 forms the row.
-__global__ void diag_final_kernel(DiagReduceArgs a) {
-    const int lane = threadIdx.x;
-    __shared__ double sums[kNSums + 2][2];
-    __shared__ double svmax;
-    for (int k = 0; k < kNSums; ++k) {
-        DD s{0.0, 0.0};
-        for (int b = lane; b < a.grid; b += 32)
-            s = dd_add_dd(s, DD{a.partials[b * 16 + 2 * k], a.partials[b * 16 + 2 * k + 1]});
-        s = warp_sum_dd(s);
-        if (lane == 0) { sums[k][0] = s.hi; sums[k][1] = s.lo; }
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(a.done, 1u) == gridDim.x - 1;
+        if (last) *a.done = 0u;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // one warp per field sum; the particle sums' partials are shared by all
+    // warps and combined in warp order
+    __shared__ double sums[kNSums][2];
+    __shared__ double part[kRedThreads / kWarp][kDiagPart];
+    {
+        DD t{0.0, 0.0};
+        for (int b = lane; b < (int)gridDim.x; b += 32) {
+            const volatile double* p = a.partials + (size_t)b * 16 + 2 * warp;
+            t = dd_add_dd(t, DD{p[0], p[1]});
+        }
+        t = warp_sum_dd(t);
+        if (lane == 0) {
+            sums[warp][0] = t.hi;
+            sums[warp][1] = t.lo;
+        }
     }
     DD kin{0.0, 0.0}, gs{0.0, 0.0};
     double vmax = 0.0;
-    for (int b = lane; b < a.pcount; b += 32) {
+    for (int b = threadIdx.x; b < a.pcount; b += blockDim.x) {
         const double* p = a.pdiag + (size_t)b * kDiagPart;
         kin = dd_add_dd(kin, DD{p[0], p[1]});
         gs = dd_add_dd(gs, DD{p[2], p[3]});
@@ -686,21 +784,32 @@ __global__ void diag_final_kernel(DiagReduceArgs a) {
     gs = warp_sum_dd(gs);
     vmax = warp_max(vmax);
     if (lane == 0) {
-        sums[kNSums][0] = kin.hi; sums[kNSums][1] = kin.lo;
-        sums[kNSums + 1][0] = gs.hi; sums[kNSums + 1][1] = gs.lo;
-        svmax = vmax;
+        part[warp][0] = kin.hi;
+        part[warp][1] = kin.lo;
+        part[warp][2] = gs.hi;
+        part[warp][3] = gs.lo;
+        part[warp][4] = vmax;
     }
-    __syncwarp();
-    if (lane != 0) return;
-    const double invN = 1.0 / (double)a.N;
-    auto tot = [&](int k) { return sums[k][0] + sums[k][1]; };
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    kin = gs = DD{0.0, 0.0};
+    vmax = 0.0;
+    for (int w = 0; w < kRedThreads / kWarp; ++w) {
+        kin = dd_add_dd(kin, DD{part[w][0], part[w][1]});
+        gs = dd_add_dd(gs, DD{part[w][2], part[w][3]});
+        vmax = fmax(vmax, part[w][4]);
+    }
+    const double invN = 1.0 / (double)N;
+    auto tot = [&](int k) { return (sums[k][0] + sums[k][1]) * invN; };  // sum over the nodes
     double* r = a.row;
     for (int k = 0; k < kNSums; ++k) r[k] = sqrt(tot(k) * invN);
-    r[8] = 0.5 * a.eps0 * (tot(5) * a.dA) + 0.5 / a.mu0 * (tot(4) * a.dA);
-    r[9] = tot(kNSums);
-    r[10] = r[8] + r[9];
-    r[11] = svmax;
-    r[12] = a.np > 0 ? tot(kNSums + 1) / (double)a.np : 0.0;
+    const double field = 0.5 * a.eps0 * (tot(5) * a.dA) + 0.5 / a.mu0 * (tot(4) * a.dA);
+    const double kinetic = kin.hi + kin.lo;
+    r[8] = field;
+    r[9] = kinetic;
+    r[10] = field + kinetic;
+    r[11] = vmax;
+    r[12] = a.np > 0 ? (gs.hi + gs.lo) / (double)a.np : 0.0;
 }
 
 __global__ void poisson_kspace_kernel(int N, const double* k2, const double2* rh, double eps0,
@@ -922,21 +1031,32 @@ cudaError_t launch_convert_acc(unsigned long long* acc, int N, const double* sca
 }
 
 cudaError_t launch_bdf_kspace(const KspaceArgs& a, cudaStream_t st) {
-    bdf_kspace_kernel<<<grid_for(a.N, 256), 256, 0, st>>>(a);
+    const int grid = grid_for((long)a.g.nx * a.g.ny, 128);
+    if (a.na == 3) {
+        if (paired_grid(a.g)) bdf_kspace_kernel<3, true><<<grid, 128, 0, st>>>(a);
+        else bdf_kspace_kernel<3, false><<<grid, 128, 0, st>>>(a);
+    } else {
+        if (paired_grid(a.g)) bdf_kspace_kernel<2, true><<<grid, 128, 0, st>>>(a);
+        else bdf_kspace_kernel<2, false><<<grid, 128, 0, st>>>(a);
+    }
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_diag_kspace(const DiagKArgs& a, cudaStream_t st) {
-    diag_kspace_kernel<<<grid_for(a.N, 256), 256, 0, st>>>(a);
+cudaError_t launch_diag_field(const DiagArgs& a, int which, double2* out, cudaStream_t st) {
+    const int grid = grid_for((long)a.g.nx * a.g.ny, 256);
+    if (paired_grid(a.g)) diag_field_kernel<true><<<grid, 256, 0, st>>>(a, which, out);
+    else diag_field_kernel<false><<<grid, 256, 0, st>>>(a, which, out);
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_diag_reduce(const DiagReduceArgs& a, cudaStream_t st) {
-    diag_reduce_kernel<<<a.grid, kRedThreads, 0, st>>>(a);
-    diag_final_kernel<<<1, 32, 0, st>>>(a);
-    count_launches(2);
+cudaError_t launch_diag_reduce(const DiagArgs& a, cudaStream_t st) {
+    long blocks = ((long)a.g.nx * a.g.ny + kRedThreads - 1) / kRedThreads;
+    const int grid = (int)(blocks < a.max_blocks ? blocks : a.max_blocks);
+    if (paired_grid(a.g)) diag_reduce_kernel<true><<<grid, kRedThreads, 0, st>>>(a);
+    else diag_reduce_kernel<false><<<grid, kRedThreads, 0, st>>>(a);
+    count_launches(1);
     return cudaGetLastError();
 }
 

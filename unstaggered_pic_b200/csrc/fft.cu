@@ -1,4 +1,4 @@
-// Batched radix-2 complex FFT for the collocated periodic grid (sm_100a).
+// Batched complex FFT for the collocated periodic grid (sm_100a).
 //
 // Replaces the reference's fft1d/fft2d (Project2/spectral_pic_part3.cpp:372-424;
 // Project3/ec_pic_nyquist_projected.cpp:1566-1670): forward
@@ -6,11 +6,24 @@
 // each 1D pass, and a 2D transform is the y-line pass followed by the x-line
 // pass, as in the reference.
 //
-// Each CTA stages whole lines in shared memory (bit-reversed on load, then
-// log2(n) in-place radix-2 butterfly passes, twiddles from an accurate table
-// rather than the reference's w *= wlen recurrence).  y lines are contiguous;
-// an x-pass CTA loads a block of adjacent columns so every global access is a
-// coalesced run along y.
+// A line of n points belongs to n/8 threads with eight points each in
+// registers.  The log2 n decimation-in-time levels run three at a time (2 2 or
+// 2 at the end where 3 does not divide log2 n), with one shared-memory
+// exchange between such passes and none before the first (whose eight
+// bit-reversed points are a stride apart, so it loads them from global
+// memory) or after the last (which ends in natural order).  The levels and
+// their twiddles (accurate table, exp(-2 pi i m/n)) are those of the plain
+// radix-2 transform, so the results do not depend on the grouping.  A
+// 512-point line then takes two exchanges; one level at a time in shared
+// memory took nine, and a 64 x 64 grid kept 11 CTAs busy where it now fills
+// 44.  Per launch, eleven inverse transforms before and after: 64 x 64
+// 13.8-16.2 -> 2.4-3.2 us, 1024 x 1024 226-256 -> 79-125 us.
+// Lines that fit a warp exchange without block barriers.  An x pass CTA takes
+// a few adjacent columns, so its global accesses are runs along y.
+//
+// What bounds it: at 1024 x 1024 and above the memory passes (16 B read and
+// 16 B written per point and pass), at small grids the latency of one load,
+// the passes and one store.
 #include "kernels.h"
 #include "upic_common.cuh"
 
@@ -18,109 +31,245 @@ namespace upic {
 
 namespace {
 
-constexpr int kFftThreads = 256;
-// Complex elements staged per CTA (64 KB of shared memory); a single line
-// longer than this stages alone (up to 8192 elements, 128 KB).
-constexpr int kFftSmemElems = 4096;
-constexpr int kFftMaxN = 8192;
+constexpr int kFftMaxLog = 13;
 
-__device__ __forceinline__ unsigned bitrev(unsigned v, int bits) {
-    return bits == 0 ? 0u : (__brev(v) >> (32 - bits));
+// Points per thread and threads per line.
+template <int LOGN>
+struct Shape {
+    static constexpr int n = 1 << LOGN;
+    static constexpr int E = n < 8 ? n : 8;
+    static constexpr int T = n / E;
+    // y pass: lines per CTA for about 128 threads
+    static constexpr int ylines = T >= 128 ? 1 : 128 / T;
+    static constexpr int ythreads = ylines * T;
+    // x pass: columns per CTA for about 256 threads, at most 16
+    static constexpr int xcols = T >= 512 ? 1 : T >= 128 ? 2 : T <= 16 ? 16 : 256 / T;
+    static constexpr int xthreads = xcols * T;
+    static constexpr bool exchanges = LOGN > 3;
+};
+
+// a b, its roundings written out so that forward and inverse, whose twiddles
+// differ in the sign of the imaginary part, contract alike.
+UPIC_D double2 cmul(double2 a, double2 b) {
+    return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// Shared-memory slot of point i: the low three bits exclusive-ored with all
+// higher groups of three, so that eight points that differ in any three
+// adjacent bits (a pass' stores and loads by consecutive threads) lie in
+// different 16-byte banks.
+UPIC_D int swizzle(int i) { return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9) ^ (i >> 12)) & 7); }
+
+template <int BITS>
+UPIC_D int reverse_bits(int v) {
+    if constexpr (BITS == 0) return 0;
+    else return (int)(__brev((unsigned)v) >> (32 - BITS));
+}
+constexpr int reverse_const(int v, int bits) {
+    int r = 0;
+    for (int k = 0; k < bits; ++k) r |= ((v >> k) & 1) << (bits - 1 - k);
+    return r;
 }
 
-// In-place radix-2 DIT passes over `lines` bit-reversed lines of length n
-// stored contiguously in s.  tw[m] = exp(-2 pi i m / n), m < n/2.
-__device__ void butterflies(double2* s, int lines, int n, int log2n, const double2* __restrict__ tw,
-                            bool inverse) {
-    const int half_total = lines * (n >> 1);
-    for (int st = 1; st <= log2n; ++st) {
-        const int half = 1 << (st - 1);
-        const int tstride = n >> st;  // twiddle index step
-        for (int b = threadIdx.x; b < half_total; b += blockDim.x) {
-            const int line = b >> (log2n - 1);
-            const int k = b & ((n >> 1) - 1);
-            const int j = k & (half - 1);
-            const int grp = k >> (st - 1);
-            const int i0 = line * n + grp * 2 * half + j;
-            const int i1 = i0 + half;
-            double2 w = __ldg(&tw[j * tstride]);
-            if (inverse) w.y = -w.y;
-            const double2 u = s[i0];
-            const double2 v = cmul(s[i1], w);
-            s[i0] = make_double2(u.x + v.x, u.y + v.y);
-            s[i1] = make_double2(u.x - v.x, u.y - v.y);
+// Levels of the decimation-in-time transform of one line from 2^LNS on, RB at
+// a time.  A group of 2^RB points that these levels combine is the points
+// block 2^(LNS+RB) + j + m 2^LNS of the bit-reversed order, j < 2^LNS; thread
+// t holds groups t + h T, point m of group h in v[h + B m].  addr(i): slot of
+// point i in shared memory; sync(): barrier of the line's threads.  On entry
+// (LNS = 0) v[e] is point t + e T of the input, on return of the output.
+template <int LOGN, int LNS, bool INV, class Addr, class Sync>
+UPIC_D void line_passes(double2* v, int t, double2* sm, const double2* __restrict__ tw, Addr addr, Sync sync) {
+    constexpr int E = Shape<LOGN>::E, T = Shape<LOGN>::T;
+    constexpr int REM = LOGN - LNS;
+    if constexpr (REM > 0) {
+        constexpr int RB = REM == 4 || REM == 2 ? 2 : (REM < 3 ? REM : 3);
+        constexpr int R = 1 << RB, B = E / R;
+#pragma unroll
+        for (int h = 0; h < B; ++h) {
+            const int j = (t + h * T) & ((1 << LNS) - 1);
+            // the first pass holds its points in input order: point m of the
+            // bit-reversed group is input point reverse(m)
+            auto at = [&](int m) -> double2& { return v[h + B * (LNS == 0 ? reverse_const(m, RB) : m)]; };
+#pragma unroll
+            for (int l = 0; l < RB; ++l) {
+#pragma unroll
+                for (int m = 0; m < R; ++m) {
+                    if (m & (1 << l)) continue;
+                    // partner m + 2^l, twiddle index (j + (m mod 2^l) 2^LNS) n / 2^(LNS+l+1)
+                    double2 w = __ldg(&tw[(j + ((m & ((1 << l) - 1)) << LNS)) << (LOGN - LNS - l - 1)]);
+                    if (INV) w.y = -w.y;
+                    double2 &a = at(m), &b = at(m + (1 << l));
+                    const double2 u = a;
+                    const double2 x = cmul(b, w);
+                    a = make_double2(u.x + x.x, u.y + x.y);
+                    b = make_double2(u.x - x.x, u.y - x.y);
+                }
+            }
         }
-        __syncthreads();
+        if constexpr (LNS + RB < LOGN) {
+#pragma unroll
+            for (int h = 0; h < B; ++h) {
+                const int q = t + h * T;
+                const int block = LNS == 0 ? reverse_bits<LOGN - RB>(q) : q >> LNS;
+                const int base = (block << (LNS + RB)) + (q & ((1 << LNS) - 1));
+#pragma unroll
+                for (int m = 0; m < R; ++m)
+                    sm[addr(base + (m << LNS))] = v[h + B * (LNS == 0 ? reverse_const(m, RB) : m)];
+            }
+            sync();
+            constexpr int LN2 = LNS + RB, REM2 = LOGN - LN2;
+            constexpr int RB2 = REM2 == 4 || REM2 == 2 ? 2 : (REM2 < 3 ? REM2 : 3);
+            constexpr int R2 = 1 << RB2, B2 = E / R2;
+#pragma unroll
+            for (int h = 0; h < B2; ++h) {
+                const int q = t + h * T;
+                const int base = ((q >> LN2) << (LN2 + RB2)) + (q & ((1 << LN2) - 1));
+#pragma unroll
+                for (int m = 0; m < R2; ++m) v[h + B2 * m] = sm[addr(base + (m << LN2))];
+            }
+            if constexpr (LN2 + RB2 < LOGN) sync();  // another exchange follows
+            line_passes<LOGN, LN2, INV>(v, t, sm, tw, addr, sync);
+        } else if constexpr (LNS == 0) {
+            // the only pass of a short line: from input to natural order
+            double2 o[E];
+#pragma unroll
+            for (int m = 0; m < E; ++m) o[m] = v[reverse_const(m, RB)];
+#pragma unroll
+            for (int m = 0; m < E; ++m) v[m] = o[m];
+        }
     }
 }
 
-// y-lines: line index L in [0, ncomp*nx), elements contiguous (stride 1).
-// in_mode 0: complex in place; 1: real planar input (imag = 0) from `rin`
-// (component stride N).  out_mode 0: complex to `data`.
-__global__ void __launch_bounds__(kFftThreads)
-fft_y_kernel(double2* __restrict__ data, const double* __restrict__ rin, int in_mode, int nlines,
-             int n, int log2n, int lines_per_cta, const double2* __restrict__ tw, int inverse) {
-    extern __shared__ double2 smem[];
-    const int line0 = blockIdx.x * lines_per_cta;
-    const int lines = min(lines_per_cta, nlines - line0);
-    if (lines <= 0) return;
-    const int total = lines * n;
-    const size_t base = (size_t)line0 * n;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-        const int l = e / n, j = e - l * n;
-        double2 v;
-        if (in_mode == 1) v = make_double2(rin[base + e], 0.0);
-        else v = data[base + e];
-        smem[l * n + bitrev(j, log2n)] = v;
+struct FftArgs {
+    double2* data;
+    int nlines;               // y pass: transforms * nx; x pass: transforms
+    int lognx, logny;
+    const double2* tw;
+    FftMap map;
+    const double* rin;        // forward: real planar input or null
+    int out_mode;             // inverse
+    void* rout;
+    int rec_stride, comp_offset;
+    FftAccIn acc;             // y forward from accumulators
+};
+
+enum YPass { kForward = 0, kInverse = 1, kForwardAcc = 2, kForwardAcc1 = 3 };
+
+// Value of component c at a node from the accumulators, which are cleared.
+template <bool SINGLE>
+UPIC_D double take_acc(const FftAccIn& a, int c, size_t N, size_t node) {
+    unsigned long long* h = a.acc + (size_t)(2 * c) * N + node;
+    double v;
+    if (SINGLE) {
+        v = (double)(long long)*h / a.scale[c];
+    } else {
+        unsigned long long* l = h + N;
+        v = from_fixed(*h, *l, 1.0 / a.scale[c]);
+        *l = 0ull;
     }
-    __syncthreads();
-    butterflies(smem, lines, n, log2n, tw, inverse != 0);
-    const double sc = inverse ? 1.0 / (double)n : 1.0;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-        double2 v = smem[e];
-        if (inverse) { v.x *= sc; v.y *= sc; }
-        data[base + e] = v;
+    *h = 0ull;
+    if (c == 3) {
+        v += a.bg ? a.bg[node] : a.n0;
+        a.rho[node] = v;
+    } else {
+        a.J[c * N + node] = v;
     }
+    return v;
 }
 
-// x-lines: for component c and column block [j0, j0+cols), element i of
-// column j lives at c*N + i*ny + j.  out_mode 0: complex in place;
-// 1: real part to rout[(c*N + node) ...] planar (rout_comp_stride = N,
-// rout_node_stride = 1); 2: real part to interleaved records
-// rout[node*rec_stride + comp_offset + c]; 3: the same records in FP32 (rout
-// then points to floats).
-__global__ void __launch_bounds__(kFftThreads)
-fft_x_kernel(double2* __restrict__ data, int ncomp, int nx, int ny, int log2nx, int cols_per_cta,
-             const double2* __restrict__ tw, int inverse, int out_mode, double* __restrict__ rout,
-             int rec_stride, int comp_offset) {
+// y lines (contiguous), the first pass.  Forward: complex, real planar or
+// accumulators in; inverse: complex in.  Complex out, in `data`.
+template <int LOGN, int PASS>
+__global__ void __launch_bounds__(Shape<LOGN>::ythreads) fft_y_kernel(FftArgs a) {
+    using S = Shape<LOGN>;
+    constexpr bool INV = PASS == kInverse;
     extern __shared__ double2 smem[];
-    const int blocks_per_comp = ny / cols_per_cta;
-    const int c = blockIdx.x / blocks_per_comp;
-    const int j0 = (blockIdx.x - c * blocks_per_comp) * cols_per_cta;
-    if (c >= ncomp) return;
-    const size_t N = (size_t)nx * ny;
-    double2* d = data + c * N;
-    const int total = nx * cols_per_cta;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-        const int i = e / cols_per_cta, cc = e - i * cols_per_cta;
-        smem[cc * nx + bitrev(i, log2nx)] = d[(size_t)i * ny + j0 + cc];
+    const int l = threadIdx.x / S::T, t = threadIdx.x % S::T;
+    const int line = blockIdx.x * S::ylines + l;
+    const bool on = line < a.nlines;
+    const int p = line >> a.lognx, row = line & ((1 << a.lognx) - 1);
+    const size_t N = (size_t)1 << (a.lognx + LOGN);
+    double2* d = a.data + (size_t)line * S::n;
+    double2 v[S::E];
+#pragma unroll
+    for (int e = 0; e < S::E; ++e) v[e] = make_double2(0.0, 0.0);
+    if (on) {
+        const int cr = a.map.re[p], ci = a.map.im[p];
+        if constexpr (PASS == kForwardAcc || PASS == kForwardAcc1) {
+            constexpr bool single = PASS == kForwardAcc1;
+#pragma unroll
+            for (int e = 0; e < S::E; ++e) {
+                const size_t node = (size_t)row * S::n + t + e * S::T;
+                v[e].x = take_acc<single>(a.acc, cr, N, node);
+                if (ci >= 0) v[e].y = take_acc<single>(a.acc, ci, N, node);
+            }
+        } else if (!INV && a.rin) {
+            const double* r = a.rin + cr * N + (size_t)row * S::n;
+#pragma unroll
+            for (int e = 0; e < S::E; ++e) v[e].x = r[t + e * S::T];
+            if (ci >= 0) {
+                const double* q = a.rin + ci * N + (size_t)row * S::n;
+#pragma unroll
+                for (int e = 0; e < S::E; ++e) v[e].y = q[t + e * S::T];
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < S::E; ++e) v[e] = d[t + e * S::T];
+        }
     }
-    __syncthreads();
-    butterflies(smem, cols_per_cta, nx, log2nx, tw, inverse != 0);
-    const double sc = inverse ? 1.0 / (double)nx : 1.0;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-        const int i = e / cols_per_cta, cc = e - i * cols_per_cta;
-        double2 v = smem[cc * nx + i];
-        if (inverse) { v.x *= sc; v.y *= sc; }
-        const size_t node = (size_t)i * ny + j0 + cc;
-        if (out_mode == 0) d[node] = v;
-        else if (out_mode == 1) rout[c * N + node] = v.x;
-        else if (out_mode == 2) rout[node * rec_stride + comp_offset + c] = v.x;
-        else reinterpret_cast<float*>(rout)[node * rec_stride + comp_offset + c] = (float)v.x;
+    // lines of fewer than eight threads share a bank phase: they start in different banks
+    const int shift = S::T < 8 ? (l * S::T) & 7 : 0;
+    line_passes<LOGN, 0, INV>(
+        v, t, smem + l * S::n, a.tw, [shift](int i) { return swizzle(i) ^ shift; },
+        [] {
+            if (S::T <= 32) __syncwarp();
+            else __syncthreads();
+        });
+    if (!on) return;
+    constexpr double sc = INV ? 1.0 / (double)S::n : 1.0;
+#pragma unroll
+    for (int e = 0; e < S::E; ++e) d[t + e * S::T] = make_double2(sc * v[e].x, sc * v[e].y);
+}
+
+// x lines, the second pass: element i of column j of transform c is at
+// c N + i ny + j; a CTA takes 2^logcols adjacent columns.  Forward: complex in
+// place; inverse: out_mode out.
+template <int LOGN, bool INV>
+__global__ void __launch_bounds__(Shape<LOGN>::xthreads) fft_x_kernel(FftArgs a, int logcols) {
+    using S = Shape<LOGN>;
+    extern __shared__ double2 smem[];
+    const int col = threadIdx.x & ((1 << logcols) - 1), t = threadIdx.x >> logcols;
+    const int logblocks = a.logny - logcols;
+    const int p = blockIdx.x >> logblocks;
+    const int j = ((blockIdx.x & ((1 << logblocks) - 1)) << logcols) + col;
+    const size_t N = (size_t)1 << (LOGN + a.logny);
+    double2* d = a.data + p * N + j;
+    double2 v[S::E];
+#pragma unroll
+    for (int e = 0; e < S::E; ++e) v[e] = d[(size_t)(t + e * S::T) << a.logny];
+    line_passes<LOGN, 0, INV>(
+        v, t, smem, a.tw, [logcols, col](int i) { return (swizzle(i) << logcols) + col; }, [] { __syncthreads(); });
+    constexpr double sc = INV ? 1.0 / (double)S::n : 1.0;
+    const int cr = a.map.re[p], ci = a.map.im[p];
+#pragma unroll
+    for (int e = 0; e < S::E; ++e) {
+        const size_t at = (size_t)(t + e * S::T) << a.logny, node = at + j;
+        const double re = sc * v[e].x, im = sc * v[e].y;
+        if (!INV || a.out_mode == 0) {
+            d[at] = make_double2(re, im);
+        } else if (a.out_mode == 1) {
+            double* o = static_cast<double*>(a.rout);
+            o[cr * N + node] = re;
+            if (ci >= 0) o[ci * N + node] = im;
+        } else if (a.out_mode == 2) {
+            double* o = static_cast<double*>(a.rout) + node * a.rec_stride + a.comp_offset;
+            o[cr] = re;
+            if (ci >= 0) o[ci] = im;
+        } else {
+            float* o = static_cast<float*>(a.rout) + node * a.rec_stride + a.comp_offset;
+            o[cr] = (float)re;
+            if (ci >= 0) o[ci] = (float)im;
+        }
     }
 }
 
@@ -130,40 +279,139 @@ int ilog2(int n) {
     return l;
 }
 
+template <int LOGN>
+int y_smem() {
+    return Shape<LOGN>::exchanges ? (int)sizeof(double2) * Shape<LOGN>::ylines * Shape<LOGN>::n : 0;
+}
+template <int LOGN>
+int x_smem(int cols) {
+    return Shape<LOGN>::exchanges ? (int)sizeof(double2) * cols * Shape<LOGN>::n : 0;
+}
+
+using YKernel = void (*)(FftArgs);
+template <int LOGN>
+YKernel y_kernel(int pass) {
+    switch (pass) {
+        case kInverse: return fft_y_kernel<LOGN, kInverse>;
+        case kForwardAcc: return fft_y_kernel<LOGN, kForwardAcc>;
+        case kForwardAcc1: return fft_y_kernel<LOGN, kForwardAcc1>;
+        default: return fft_y_kernel<LOGN, kForward>;
+    }
+}
+
+template <int LOGN>
+void launch_y(const FftArgs& a, int pass, cudaStream_t st) {
+    using S = Shape<LOGN>;
+    const int grid = (a.nlines + S::ylines - 1) / S::ylines;
+    y_kernel<LOGN>(pass)<<<grid, S::ythreads, y_smem<LOGN>(), st>>>(a);
+}
+
+template <int LOGN>
+void launch_x(const FftArgs& a, bool inverse, cudaStream_t st) {
+    using S = Shape<LOGN>;
+    const int ny = 1 << a.logny;
+    const int cols = S::xcols < ny ? S::xcols : ny;
+    const int grid = a.nlines * (ny / cols);
+    if (inverse) fft_x_kernel<LOGN, true><<<grid, cols * S::T, x_smem<LOGN>(cols), st>>>(a, ilog2(cols));
+    else fft_x_kernel<LOGN, false><<<grid, cols * S::T, x_smem<LOGN>(cols), st>>>(a, ilog2(cols));
+}
+
+template <int LOGN>
+cudaError_t raise_one() {
+    cudaError_t e = cudaSuccess;
+    if constexpr (LOGN >= 0) {
+        for (int pass = kForward; pass <= kForwardAcc1 && y_smem<LOGN>() > 48 * 1024 && e == cudaSuccess; ++pass)
+            e = raise_smem_limit(reinterpret_cast<const void*>(y_kernel<LOGN>(pass)), y_smem<LOGN>());
+        if (x_smem<LOGN>(Shape<LOGN>::xcols) > 48 * 1024) {
+            const int b = x_smem<LOGN>(Shape<LOGN>::xcols);
+            if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(fft_x_kernel<LOGN, false>), b);
+            if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(fft_x_kernel<LOGN, true>), b);
+        }
+        if (e == cudaSuccess) e = raise_one<LOGN - 1>();
+    }
+    return e;
+}
+
+#define UPIC_FFT_SIZES(F) F(0) F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13)
+
+void run_y(int logn, const FftArgs& a, int pass, cudaStream_t st) {
+    switch (logn) {
+#define UPIC_CASE(L) case L: launch_y<L>(a, pass, st); break;
+        UPIC_FFT_SIZES(UPIC_CASE)
+#undef UPIC_CASE
+    }
+}
+
+void run_x(int logn, const FftArgs& a, bool inverse, cudaStream_t st) {
+    switch (logn) {
+#define UPIC_CASE(L) case L: launch_x<L>(a, inverse, st); break;
+        UPIC_FFT_SIZES(UPIC_CASE)
+#undef UPIC_CASE
+    }
+}
+
 }  // namespace
 
-// Lines-per-CTA choices keep every CTA at <= kFftSmemElems staged elements.
-static int y_lines_per_cta(int ny) { return ny >= kFftSmemElems ? 1 : kFftSmemElems / ny; }
-static int x_cols_per_cta(int nx, int ny) {
-    int c = nx >= kFftSmemElems ? 1 : kFftSmemElems / nx;
-    if (c > ny) c = ny;
-    return c;
+FftMap fft_identity_map(int ncomp) {
+    FftMap m{};
+    for (int c = 0; c < ncomp && c < kFftMaxTransforms; ++c) {
+        m.re[c] = (signed char)c;
+        m.im[c] = -1;
+    }
+    return m;
+}
+
+namespace {
+
+// Both passes of `a` (its plan-dependent members are filled in here).
+cudaError_t run_2d(const FftPlan& p, FftArgs a, int ntransforms, int pass, cudaStream_t st) {
+    const int lx = ilog2(p.nx), ly = ilog2(p.ny);
+    if (ntransforms > kFftMaxTransforms || lx > kFftMaxLog || ly > kFftMaxLog) return cudaErrorInvalidValue;
+    a.lognx = lx;
+    a.logny = ly;
+    FftArgs x = a;
+    a.nlines = ntransforms << lx;
+    a.tw = p.tw_y;
+    x.nlines = ntransforms;
+    x.tw = p.tw_x;
+    run_y(ly, a, pass, st);
+    run_x(lx, x, pass == kInverse, st);
+    count_launches(2);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t fft2d_mapped(const FftPlan& p, double2* data, int ntransforms, const FftMap& map, int inverse,
+                         cudaStream_t st, const double* real_in, int out_mode, void* real_out, int rec_stride,
+                         int comp_offset) {
+    FftArgs a{};
+    a.data = data;
+    a.map = map;
+    a.rin = inverse ? nullptr : real_in;
+    a.out_mode = out_mode;
+    a.rout = real_out;
+    a.rec_stride = rec_stride;
+    a.comp_offset = comp_offset;
+    return run_2d(p, a, ntransforms, inverse ? kInverse : kForward, st);
+}
+
+cudaError_t fft2d_from_acc(const FftPlan& p, double2* data, int ntransforms, const FftMap& map, const FftAccIn& acc,
+                           cudaStream_t st) {
+    FftArgs a{};
+    a.data = data;
+    a.map = map;
+    a.acc = acc;
+    return run_2d(p, a, ntransforms, acc.single ? kForwardAcc1 : kForwardAcc, st);
 }
 
 cudaError_t fft2d_batched(const FftPlan& p, double2* data, int ncomp, int inverse, cudaStream_t st,
                           const double* real_in, int out_mode, double* real_out, int rec_stride,
                           int comp_offset) {
-    const int nx = p.nx, ny = p.ny;
-    const int nl = ncomp * nx;
-    const int lpc = y_lines_per_cta(ny);
-    const int gy = (nl + lpc - 1) / lpc;
-    const size_t smy = sizeof(double2) * (size_t)lpc * ny;
-    fft_y_kernel<<<gy, kFftThreads, smy, st>>>(data, real_in, real_in ? 1 : 0, nl, ny, ilog2(ny),
-                                               lpc, p.tw_y, inverse);
-    const int cpc = x_cols_per_cta(nx, ny);
-    const int gx = ncomp * (ny / cpc);
-    const size_t smx = sizeof(double2) * (size_t)cpc * nx;
-    fft_x_kernel<<<gx, kFftThreads, smx, st>>>(data, ncomp, nx, ny, ilog2(nx), cpc, p.tw_x, inverse,
-                                               out_mode, real_out, rec_stride, comp_offset);
-    count_launches(2);
-    return cudaGetLastError();
+    return fft2d_mapped(p, data, ncomp, fft_identity_map(ncomp), inverse, st, real_in, out_mode, real_out,
+                        rec_stride, comp_offset);
 }
 
-cudaError_t fft_configure_smem() {
-    const int bytes = (int)(sizeof(double2) * kFftMaxN);
-    cudaError_t e = cudaFuncSetAttribute(fft_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(fft_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
+cudaError_t fft_configure_smem() { return raise_one<kFftMaxLog>(); }
 
 }  // namespace upic

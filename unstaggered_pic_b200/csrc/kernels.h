@@ -20,16 +20,42 @@ cudaError_t raise_smem_limit(const void* func, int bytes);
 // FFT (fft.cu)
 struct FftPlan {
     int nx, ny;
-    const double2* tw_x;  // exp(-2 pi i m / nx), m < nx/2
-    const double2* tw_y;  // exp(-2 pi i m / ny), m < ny/2
+    const double2* tw_x;  // exp(-2 pi i m / nx), m < nx
+    const double2* tw_y;  // exp(-2 pi i m / ny), m < ny
 };
 
-// 2D transform of ncomp stacked complex grids (component stride nx*ny).
-// real_in != NULL: the input is the real planar array real_in (imag 0), the
-// transform result lands in data.  out_mode 0: complex result in data;
-// 1: real part to real_out planar (component stride nx*ny); 2: real part to
-// interleaved records real_out[node*rec_stride + comp_offset + c]; 3: the
-// same records as floats (real_out then points to float storage).
+// Real components of a batch of transforms: transform p carries component
+// re[p] in its real part and im[p] (-1: none) in its imaginary part.
+constexpr int kFftMaxTransforms = 16;
+struct FftMap {
+    signed char re[kFftMaxTransforms], im[kFftMaxTransforms];
+};
+FftMap fft_identity_map(int ncomp);  // component p alone in transform p
+
+// 2D transforms of stacked complex grids (stride nx*ny).  Forward with
+// real_in != NULL: the input is the components of the real planar array
+// real_in that `map` names, the result lands in data.  Inverse, out_mode 0:
+// complex result in data; 1: the components to real_out planar (stride
+// nx*ny); 2: to interleaved records real_out[node*rec_stride + comp_offset +
+// component]; 3: the same records as floats (float storage).
+cudaError_t fft2d_mapped(const FftPlan& p, double2* data, int ntransforms, const FftMap& map, int inverse,
+                         cudaStream_t st, const double* real_in, int out_mode, void* real_out, int rec_stride,
+                         int comp_offset);
+// Forward transforms straight from the deposit accumulators: component c is
+// J_c (0..2) or rho (3), converted, stored to J / rho and cleared on the way
+// (launch_convert_acc, or launch_convert_acc1 with `single`).
+struct FftAccIn {
+    unsigned long long* acc;  // [slot 4][hi, lo][N]
+    double scale[4];
+    double *J, *rho;
+    double n0;
+    const double* bg;
+    int single;
+};
+cudaError_t fft2d_from_acc(const FftPlan& p, double2* data, int ntransforms, const FftMap& map, const FftAccIn& acc,
+                           cudaStream_t st);
+// The same with every component alone in its transform (at most
+// kFftMaxTransforms).
 cudaError_t fft2d_batched(const FftPlan& p, double2* data, int ncomp, int inverse, cudaStream_t st,
                           const double* real_in = nullptr, int out_mode = 0,
                           double* real_out = nullptr, int rec_stride = 0, int comp_offset = 0);
@@ -210,51 +236,52 @@ cudaError_t launch_convert_acc(unsigned long long* acc, int N, const double* sca
                                double* J, double* rho, double n0, int ncomp_mask,
                                cudaStream_t st, const double* bg = nullptr);
 
-struct KspaceArgs {
-    int N;
+// Grid and wave-number tables (nx x ny each) of the k-space kernels.
+struct KGrid {
+    int nx, ny, lny;  // lny = log2(ny)
+    int paired;       // real fields share transforms two by two (explicit.cu)
     const double *kx, *ky, *k2;
-    const double2* Jhat;       // 3 x N
-    const double2* rho_dep;    // N (naive charge spectrum) or null
+};
+
+inline bool paired_grid(const KGrid& g) { return g.paired != 0; }
+
+struct KspaceArgs {
+    KGrid g;
+    const double2* Jhat;       // (Jx, Jy), Jz transforms when paired, else Jx, Jy, Jz
+    const double2* rho_dep;    // naive charge spectrum or null
     double2* hist;             // ring: [field(5: phi, Ax, Ay, Az, rho)][slot R][N]
     int R, head;               // slots; head = slot of u^n
-    int na;                    // BDF coefficients a[0..na)
+    int na;                    // BDF coefficients a[0..na), 2 or 3
     double a[3];
-    int nb;
-    double b[5];
+    double b[5];               // their convolution, 2 na - 1 of them
     double dt, c, eps0, mu0;
     int conserving;
-    double2* gspec;            // 11 x N gather-field spectra (output) or null
+    double2* gspec;            // spectra of the gathered fields: 6 transforms when paired, else 11
 };
 cudaError_t launch_bdf_kspace(const KspaceArgs& a, cudaStream_t st);
 
-// Diagnostics spectra (10 x N): gauge, E (3), gauss, continuity, B (3), rho.
-struct DiagKArgs {
-    int N;
-    const double *kx, *ky, *k2;
-    const double2* Jhat;
+// Diagnostics of the histories: fields gauge 0, E 1..3, gauss 4, continuity
+// 5, B 6..8, rho 9.
+struct DiagArgs {
+    KGrid g;
+    const double2* Jhat;          // as in KspaceArgs
     const double2* hist;
     int R, slot_new, slot_prev0;  // u^{n+1} slot; past(0) slot
     int na;
     double a[3];
-    double dt, c, eps0;
-    double2* out;
-};
-cudaError_t launch_diag_kspace(const DiagKArgs& a, cudaStream_t st);
-
-// Sum-of-squares reductions over the diagnostics fields; writes the row.
-struct DiagReduceArgs {
-    int N;
-    const double* dfields;  // 10 x N real (gauge, Ex, Ey, Ez, gauss, cont, Bx, By, Bz, rho)
-    const double* J;        // 3 x N
-    double* partials;       // grid x 16
-    int grid;
-    const double* pdiag;    // particle partials (count x kDiagPart)
+    double dt, c, eps0, mu0, dA;
+    // reduction: partials of max_blocks blocks x 16, finished-block counter
+    // (zero between launches), particle partials (pcount x kDiagPart), row
+    double* partials;
+    int max_blocks;
+    unsigned* done;
+    const double* pdiag;
     int pcount;
     long np;
-    double dA, eps0, mu0;
-    double* row;            // 13 doubles (device)
+    double* row;                  // 13 doubles, device-visible
 };
-cudaError_t launch_diag_reduce(const DiagReduceArgs& a, cudaStream_t st);
+cudaError_t launch_diag_field(const DiagArgs& a, int which, double2* out, cudaStream_t st);
+cudaError_t launch_diag_reduce(const DiagArgs& a, cudaStream_t st);
 
 // phi_hat = rho_hat/(eps0 k2), 0 at k2 == 0 (into out).
 cudaError_t launch_poisson_kspace(int N, const double* k2, const double2* rho_hat, double eps0,
