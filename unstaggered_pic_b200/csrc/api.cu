@@ -110,6 +110,8 @@ TileGeom make_tiles(int nx, int ny, int tile, int guard, int lo, int hi) {
     g.key_origin_x = 0.0;
     g.key_origin_y = 0.0;
     g.key_shift = 0.5;
+    g.classes = 1;
+    g.class_dt = g.class_off = 0.0;
     return g;
 }
 

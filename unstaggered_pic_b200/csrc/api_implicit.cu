@@ -37,8 +37,9 @@ constexpr int kNormGrid = 296;
 constexpr int kMaxImplicitChunk = 1024;
 
 struct ImplicitState {
-    int order = 2, nq = 8, mnq = 8;
-    double* qtab = nullptr;  // Gauss rules (ImplicitMapArgs::qtab)
+    int order = 2, nq = 8;
+    bool closed = false;     // orbit integrals in closed form (ImplicitMapArgs::closed)
+    double* qtab = nullptr;  // Gauss rule (ImplicitMapArgs::qtab)
     double dx = 0, dy = 0, dV = 0;
     // particles: two sorted copies (the second is the sort / trial target)
     ParticleSoA P[2];
@@ -80,7 +81,7 @@ struct ImplicitState {
     double scaleJ[4] = {1, 1, 1, 1};
     TileGeom tg{};
     SortWork sw{};
-    int grid = 148;
+    int deposit_grid = 148;
     long steps = 0;
     // kernel-level orbit entry points: host-array staging (grown on demand)
     long ocap = 0;
@@ -309,6 +310,7 @@ void free_particles(upic_ctx* c, ImplicitState& s) {
 int sort_active(upic_ctx* c, ImplicitState& s) {
     ParticleSoA& src = s.P[s.cur];
     ParticleSoA& dst = s.P[1 - s.cur];
+    s.tg.class_dt = c->cfg.dt;
     UPIC_CUDA(c, sort_particles_by_tile(s.tg, src, s.np, c->cfg.Lx, c->cfg.Ly, 0.0, s.sw, c->st));
     UPIC_CUDA(c, permute_particles(src, dst, s.np, s.sw, c->st));
     // vbar arrays ride along through the spare velocity slots of a temporary SoA
@@ -368,7 +370,7 @@ int record_failures(upic_ctx* c, ImplicitState& s, const ImplicitMapArgs& a) {
         if ((rc = dalloc(c, &s.dfail, (size_t)kFailRec * nf))) return rc;
         s.dfail_cap = nf;
     }
-    UPIC_CUDA(c, launch_failure_report(s.order, s.uniform, a.split != 0, s.tg, a, s.failed, nf, s.dfail, c->st));
+    UPIC_CUDA(c, launch_failure_report(s.order, s.uniform, s.tg, a, s.failed, nf, s.dfail, c->st));
     std::vector<double> rows((size_t)kFailRec * nf);
     UPIC_CUDA(c, cudaMemcpyAsync(rows.data(), s.dfail, sizeof(double) * rows.size(), cudaMemcpyDeviceToHost, c->st));
     if ((rc = sync(c))) return rc;
@@ -438,7 +440,8 @@ int eval_map(upic_ctx* c, ImplicitState& s, const double* guess, double* out, bo
     a.stats = s.dstats;
     a.qtab = s.qtab;
     a.nq = s.nq;
-    a.mnq = s.mnq;
+    a.closed = s.closed ? 1 : 0;
+    a.closed_solve = s.closed && c->ny > 1 && s.np >= kClosedSolveMin;
     if (s.layout_active) {
         a.nsub = s.nsub;
         a.refined = s.refined;
@@ -473,7 +476,7 @@ int eval_map(upic_ctx* c, ImplicitState& s, const double* guess, double* out, bo
             UPIC_CUDA(c, cudaEventCreate(&e1));
             UPIC_CUDA(c, cudaEventRecord(e0, c->st));
         }
-        UPIC_CUDA(c, launch_implicit_map(s.order, s.uniform, a.split != 0, s.tg, a, s.grid, c->st));
+        UPIC_CUDA(c, launch_implicit_map(s.order, s.uniform, s.tg, a, c->nsm, s.deposit_grid, c->st));
         if (c->profiling) {
             UPIC_CUDA(c, cudaEventRecord(e1, c->st));
             c->prof_events.emplace_back(e0, e1);
@@ -561,14 +564,14 @@ int picard_eval(upic_ctx* c, ImplicitState& s, NormSums& vel) {
         a.stats = s.dstats;
         a.qtab = s.qtab;
         a.nq = s.nq;
-        a.mnq = s.mnq;
+        a.closed = s.closed ? 1 : 0;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         if (c->profiling) {
             UPIC_CUDA(c, cudaEventCreate(&e0));
             UPIC_CUDA(c, cudaEventCreate(&e1));
             UPIC_CUDA(c, cudaEventRecord(e0, c->st));
         }
-        UPIC_CUDA(c, launch_implicit_map(s.order, s.uniform, a.split != 0, s.tg, a, s.grid, c->st, true));
+        UPIC_CUDA(c, launch_implicit_map(s.order, s.uniform, s.tg, a, c->nsm, s.deposit_grid, c->st, true));
         if (c->profiling) {
             UPIC_CUDA(c, cudaEventRecord(e1, c->st));
             c->prof_events.emplace_back(e0, e1);
@@ -601,11 +604,11 @@ int picard_eval(upic_ctx* c, ImplicitState& s, NormSums& vel) {
     q.rec = s.rec;
     q.split = cf.split_orbit_at_knots;
     q.nq = s.nq;
-    q.mnq = s.mnq;
+    q.closed = s.closed ? 1 : 0;
     q.qtab = s.qtab;
     q.partials = s.partials;
     q.err = s.perr;
-    UPIC_CUDA(c, launch_picard_push(s.order, s.uniform, q.split != 0, q, kNormGrid, s.dnorm, c->st));
+    UPIC_CUDA(c, launch_picard_push(s.order, s.uniform, q, kNormGrid, s.dnorm, c->st));
     UPIC_CUDA(c, cudaMemcpyAsync(s.hstats, s.dstats, sizeof(MapStats), cudaMemcpyDeviceToHost, c->st));
     UPIC_CUDA(c, cudaMemcpyAsync(s.hnorm, s.dnorm, sizeof(NormSums), cudaMemcpyDeviceToHost, c->st));
     UPIC_CUDA(c, cudaMemcpyAsync(s.hflag, s.perr, sizeof(int), cudaMemcpyDeviceToHost, c->st));
@@ -1430,33 +1433,30 @@ int implicit_create(upic_ctx* c) {
     s->tg.key_shift = 0.0;
     s->tg.chunk = kMaxImplicitChunk;
     const bool split = cf.split_orbit_at_knots != 0;
-    if (implicit_configure_smem(s->tg, s->order, split, s->picard) != cudaSuccess)
+    if (split && c->ny > 1) {
+        s->tg.classes = 4;  // 0, 1, 2 or more knots passed
+        s->tg.class_off = 0.5 * (double)(s->order - 1);
+    }
+    // With knot splitting, every orbit integrand within a segment -- S_a S_b,
+    // (1-s) S'_a S_b, s S'_a S_b, the time-interpolated A included -- is a
+    // polynomial of degree <= 2 order + 1 in s, which the deck's rule of nq >=
+    // order + 1 points integrates exactly: the deposit and the Picard push then
+    // take the integrals in closed form, and the sums that remain (local
+    // solves, sub-cycled orbits, step diagnostics) the (order+1)-point rule,
+    // each equal to the deck's sums up to rounding.  Without knot splitting a
+    // segment spans several spline pieces and the deck's rule is kept, as is
+    // a rule of fewer points.
+    s->closed = split && s->nq >= s->order + 1;
+    if (s->closed) s->nq = s->order + 1;
+    if (implicit_configure_smem(s->tg, s->order, split, s->closed, s->picard) != cudaSuccess)
         return fail(c, UPIC_ERR_CUDA, "cudaFuncSetAttribute (implicit map) failed");
-    const int occ = implicit_map_occupancy(s->tg, s->order, split, s->picard);
-    s->grid = c->nsm * (occ > 0 ? occ : 1);
-    // Gauss rules.  With knot splitting, every orbit integrand within a
-    // segment -- S_a S_b, (1-s) S'_a S_b, s S'_a S_b in 2D, S_a, (1-s) S'_a,
-    // s S'_a on a grid one cell high, the time-interpolated A included -- is
-    // a polynomial of degree <= 2 order + 1 in s, which an (order+1)-point
-    // Gauss rule integrates exactly, as the deck's nq-point rule does when
-    // nq >= order+1: the two then differ by rounding only.  So with knot
-    // splitting and nq > order+1 both the point-by-point orbit integrals and
-    // the segment moments use the (order+1)-point rule; without knot
-    // splitting a segment spans several spline pieces and the deck's rule is
-    // kept.
-    std::vector<double> qs, qw, ms, mw;
-    if (split && s->nq > s->order + 1) s->nq = s->order + 1;
+    s->deposit_grid = c->nsm * std::max(1, implicit_deposit_occupancy(s->tg, s->order, split, s->closed, s->picard));
+    std::vector<double> qs, qw;
     gauss_legendre_01(s->nq, qs, qw);
-    s->mnq = s->nq;
-    gauss_legendre_01(s->mnq, ms, mw);
-    std::vector<double> tab(4 * kMaxQuad, 0.0);
+    std::vector<double> tab(2 * kMaxQuad, 0.0);
     for (int i = 0; i < s->nq; ++i) {
         tab[i] = qs[i];
         tab[kMaxQuad + i] = qw[i];
-    }
-    for (int i = 0; i < s->mnq; ++i) {
-        tab[2 * kMaxQuad + i] = ms[i];
-        tab[3 * kMaxQuad + i] = mw[i];
     }
     int rc;
     if ((rc = dalloc(c, &s->qtab, tab.size()))) return rc;
@@ -1540,7 +1540,7 @@ int implicit_set_particles(upic_ctx* c, long np, const double* x, const double* 
     }
     if ((rc = ensure_tmp3(c, np))) return rc;
     s.np = np;
-    s.tg.chunk = choose_chunk(np, s.grid, kMaxImplicitChunk);
+    s.tg.chunk = choose_chunk(np, s.deposit_grid, kMaxImplicitChunk);
     s.cur = 0;
     s.uniform = uniform;
     s.q0 = np ? q[0] : 0.0;
@@ -1614,7 +1614,7 @@ int implicit_state_io(upic_ctx* c, StateIO& io) {
         if ((rc = ensure_tmp3(c, np))) return rc;
         s.cur = 0;
         s.np = np;
-        s.tg.chunk = choose_chunk(np, s.grid, kMaxImplicitChunk);
+        s.tg.chunk = choose_chunk(np, s.deposit_grid, kMaxImplicitChunk);
         s.uniform = uniform != 0;
         s.loaded = loaded != 0;
         s.ready = ready != 0;
@@ -1858,8 +1858,8 @@ int step_diagnostics(upic_ctx* c, ImplicitState& s, double W0, double K0, double
         a.stats = s.dstats;
         a.qtab = s.qtab;
         a.nq = s.nq;
-        a.mnq = s.mnq;
-        UPIC_CUDA(c, launch_implicit_map(s.order, s.uniform, a.split != 0, s.tg, a, s.grid, c->st, true));
+        a.closed = s.closed ? 1 : 0;
+        UPIC_CUDA(c, launch_implicit_map(s.order, s.uniform, s.tg, a, c->nsm, s.deposit_grid, c->st, true));
         UPIC_CUDA(c, launch_convert_acc(s.acc, N, s.scaleJ, s.trial, nullptr, 0.0, 1, c->st));
         Jgrid = s.trial;
     }
@@ -2402,7 +2402,7 @@ extern "C" int upic_push_gmhc(upic_ctx* c, long np, const double* x, const doubl
     a.loc_maxit = cf.local_max_iter;
     a.qtab = s.qtab;
     a.nq = s.nq;
-    a.mnq = s.mnq;
+    a.closed = s.closed ? 1 : 0;
     UPIC_CUDA(c, launch_gmhc_push(s.order, a, c->nx, c->ny, np, din, dg, dout, drep, c->st));
     std::vector<double> out(11 * (size_t)np);
     UPIC_CUDA(c, cudaMemcpyAsync(out.data(), dout, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, c->st));

@@ -8,12 +8,13 @@
 // damped local fixed point on the orbit velocity vbar
 // (solve_local_particle_substep :4930, evaluate_local_particle_substep :4843)
 // followed by the orbit-averaged current deposit of the accepted orbit
-// (path_average_deposit_current :2784) -- all in implicit_map_kernel, one
-// thread per particle.  The grid runs in 2D (nz = 1): the z stencil of the
+// (path_average_deposit_current :2784), one thread per particle
+// (implicit_solve_kernel, implicit_deposit_kernel).  The grid runs in 2D (nz = 1): the z stencil of the
 // reference then sums to one, so its z factors and z-knot splits only change
 // rounding and are dropped here.
 #include <climits>
 
+#include "deposit.cuh"
 #include "implicit_kernels.h"
 #include "upic_common.cuh"
 
@@ -22,43 +23,24 @@ namespace upic {
 namespace {
 
 constexpr int kMapThreads = 128;
-// Resident CTAs per SM the map kernel is compiled for (register budget
-// 65536 / (128 * kMapMinBlocks) per thread).
-#ifndef UPIC_MAP_MIN_BLOCKS
-#define UPIC_MAP_MIN_BLOCKS 3
-#endif
-constexpr int kMapMinBlocks = UPIC_MAP_MIN_BLOCKS;
-// A map evaluation runs as one fused launch (kPartFused), or as a local-solve
-// launch followed by a deposit launch (kPartSolve, kPartDeposit) that hands
-// the orbit velocities over through global memory.  The split keeps the
-// solve's code and registers free of the deposit machinery and gives the
-// deposit its own occupancy; the sums are the same bit for bit.
-#ifndef UPIC_MAP_SPLIT
-#define UPIC_MAP_SPLIT 1
-#endif
-// resident CTAs of the local-solve launch: 3 for the segment-moment
-// instances, 4 for the point-by-point ones (orders 3-4 in 2D), each the
-// faster of 2, 3 and 4 measured
+// A map evaluation is a local-solve launch followed by a deposit launch that
+// takes the orbit velocities through global memory: the solve's code and
+// registers stay free of the deposit machinery and each has its own
+// occupancy.
+// Resident CTAs per SM of the local solve.
 #ifndef UPIC_SOLVE_MIN_BLOCKS
-#define UPIC_SOLVE_MIN_BLOCKS 3
+#define UPIC_SOLVE_MIN_BLOCKS 4
 #endif
 #ifndef UPIC_SOLVE_POINTS_MIN_BLOCKS
 #define UPIC_SOLVE_POINTS_MIN_BLOCKS 4
 #endif
-// resident CTAs of the deposit launch: 8 for the segment-moment instances
-// (one item per segment), 6 for the point-by-point ones (one item per
-// quadrature point), whose 8-CTA build measured slower
-#ifndef UPIC_DEPOSIT_MIN_BLOCKS
-#define UPIC_DEPOSIT_MIN_BLOCKS 6
-#endif
-#ifndef UPIC_DEPOSIT_MOM_MIN_BLOCKS
-#define UPIC_DEPOSIT_MOM_MIN_BLOCKS 8
-#endif
-constexpr int kPartFused = 0, kPartSolve = 1, kPartDeposit = 2;
-constexpr int map_min_blocks(int part, bool mom = false) {
-    return part == kPartSolve     ? (mom ? UPIC_SOLVE_MIN_BLOCKS : UPIC_SOLVE_POINTS_MIN_BLOCKS)
-           : part == kPartDeposit ? (mom ? UPIC_DEPOSIT_MOM_MIN_BLOCKS : UPIC_DEPOSIT_MIN_BLOCKS)
-                                  : kMapMinBlocks;
+constexpr int solve_min_blocks(bool mom) { return mom ? UPIC_SOLVE_MIN_BLOCKS : UPIC_SOLVE_POINTS_MIN_BLOCKS; }
+// Resident CTAs per SM of the deposit.  With private windows shared memory
+// allows five to six CTAs of a quadratic 2D tile and four of a cubic one,
+// which leaves registers for them; with the shared window 8 for one item per
+// segment and 6 for one per quadrature point measured best.
+constexpr int deposit_min_blocks(int order, bool mom, bool picard, bool priv) {
+    return priv ? (order >= 3 ? 4 : 5) : picard ? 3 : mom ? 8 : 6;
 }
 constexpr int kMapWarps = kMapThreads / kWarp;
 constexpr int kKeyNone = -1;
@@ -155,11 +137,9 @@ UPIC_D void bspline_f(double f, double inv_h, double* w, double* dw) {
 struct Geo {
     int nx, ny;
     double Lx, Ly, inv_dx, inv_dy;
-    // orbit quadrature (map kernel only, in shared memory): the deck's
-    // Gauss rule for point-wise orbit sums, and the rule used for segment
-    // moments
-    const double *qs = nullptr, *qw = nullptr, *ms = nullptr, *mw = nullptr;
-    int nq = 0, mnq = 0;
+    // Gauss rule of the point-by-point orbit sums and of the segment moments
+    const double *qs = nullptr, *qw = nullptr;
+    int nq = 0;
 };
 
 // SY: nodes of the y stencil, ORDER + 1, or 1 on a grid one cell high
@@ -492,10 +472,10 @@ UPIC_D void segment_moments(const Geo& g, double x0, double y0, double dxx, doub
         M.m[k] = 0.0;
         if (GRAD) M.x0[k] = M.x1[k] = M.y0[k] = M.y1[k] = 0.0;
     }
-    const int nq = g.mnq;
+    const int nq = g.nq;
     for (int iq = 0; iq < nq; ++iq) {
-        const double s = sa + len * g.ms[iq];
-        const double wq = len * g.mw[iq];
+        const double s = sa + len * g.qs[iq];
+        const double wq = len * g.qw[iq];
         double wx[S], dwx[S], wy[S], dwy[S];
         bspline_f<ORDER>((ox + s * dxx) * g.inv_dx - fx0, g.inv_dx, wx, dwx);
         if constexpr (SY == 1) {
@@ -584,6 +564,405 @@ UPIC_D bool evaluate_moments(const Geo& g, const double* __restrict__ rec, doubl
     return true;
 }
 
+// ---- knot-split orbits in closed form -------------------------------------
+// Inside a knot-split segment every point of the orbit has the same stencil
+// and the shape functions are polynomials of the segment's parameter tau in
+// [-1/2, 1/2] (tau = 0 at its middle), so the integrals
+//   <S_a S_b>, <S'_a S_b>, <tau S'_a S_b>, <S_a S'_b>, <tau S_a S'_b>
+// that path_average_gather_vector_one (:2738) and
+// orbit_discrete_gradient_A_interval (:2958) form with a Gauss rule follow
+// from the Taylor coefficients at the middle and the moments of tau,
+// <tau^k> = 2^-k / (k + 1) for even k and 0 for odd.  The Gauss rule of order
+// + 1 points or more, which integrates these polynomials exactly, gives the
+// same value up to rounding.  Each node's five weights are formed as its
+// record is read, so no array of sums is kept: the solve needs neither the
+// quadrature loop (3 x 95 FP64 instructions of a quadratic segment, of about
+// 410) nor the 45 accumulators that held it at 168 registers with 344 B of
+// spills.
+UPIC_HD constexpr double tau_moment(int k) {
+    if (k & 1) return 0.0;
+    double p = 1.0;
+    for (int i = 0; i < k; ++i) p *= 0.5;
+    return p / (double)(k + 1);
+}
+
+// Centred B-splines of degree R at offset t in [0, 1) of their knot cell (the
+// stencil's first node il, t = u - (R - 1)/2 - il): w[a] = S_a, and the Taylor
+// coefficients of their derivative along a path that moves d cells per unit
+// tau, G[i][a] = d^i / i! S_a^(i+1)(t) in units of 1/h.  Cox-de Boor: the
+// k-th derivatives are k-th differences of the degree R - k splines.
+template <int R>
+UPIC_D void spline_taylor(double t, double d, double (&w)[R + 1], double (&G)[R][R + 1]) {
+    double W[R + 1][R + 1];
+    W[0][0] = 1.0;
+#pragma unroll
+    for (int p = 1; p <= R; ++p)
+#pragma unroll
+        for (int a = 0; a <= p; ++a) {
+            double v = 0.0;
+            if (a > 0) v = W[p - 1][a - 1] * (t + (double)(p - a));
+            if (a < p) v = fma(W[p - 1][a], (double)(a + 1) - t, v);
+            W[p][a] = v * (1.0 / (double)p);
+        }
+#pragma unroll
+    for (int a = 0; a <= R; ++a) w[a] = W[R][a];
+    double scale = 1.0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        double D[R + 1];
+#pragma unroll
+        for (int a = 0; a <= R; ++a) D[a] = a <= R - i - 1 ? W[R - i - 1][a] : 0.0;
+#pragma unroll
+        for (int k = 0; k <= i; ++k)
+#pragma unroll
+            for (int a = R; a >= 0; --a) D[a] = (a > 0 ? D[a - 1] : 0.0) - D[a];
+        if (i > 0) scale *= d * (1.0 / (double)i);
+#pragma unroll
+        for (int a = 0; a <= R; ++a) G[i][a] = i > 0 ? scale * D[a] : D[a];
+    }
+}
+
+// Taylor coefficient i of S_a itself along the path: w for i = 0, else
+// d / i G[i - 1].
+template <int R>
+UPIC_D double taylor(const double (&w)[R + 1], const double (&G)[R][R + 1], double d, int i, int a) {
+    return i == 0 ? w[a] : d * (1.0 / (double)i) * G[i - 1][a];
+}
+
+// The next knot (integer) that an orbit u0 + s du passes along one axis after
+// fraction s (2: none in (0, 1)); s = 0 for the first
+// (path_breakpoints_for_particle :2555).  Only s is kept between calls: the
+// knot passed at s is the integer nearest u0 + s du.
+UPIC_D double next_knot(double u0, double du, double s) {
+    const double step = du > 0.0 ? 1.0 : -1.0;
+    double m = s > 0.0 ? rint(fma(s, du, u0)) + step : du > 0.0 ? floor(u0) + 1.0 : ceil(u0) - 1.0;
+    for (;;) {
+        if (fabs(du) < 1.0e-300 || !((m - (u0 + du)) * step < 0.0)) return 2.0;
+        s = (m - u0) / du;
+        if (s > 1.0e-13) return s < 1.0 - 1.0e-13 ? s : 2.0;
+        m += step;
+    }
+}
+
+// The segments of an orbit between its knots, one after the other; knots
+// closer than 1e-12 count once, and more than kMaxBreaks end points fail.
+struct KnotWalk {
+    double sx, sy, prev;
+    int nb;  // end points so far; 0 when no segment is left, -1 when there were too many
+    UPIC_D void init(double ux, double uy, double dux, double duy) {
+        sx = next_knot(ux, dux, 0.0);
+        sy = next_knot(uy, duy, 0.0);
+        prev = 0.0;
+        nb = 2;
+    }
+    UPIC_D bool more() const { return nb > 0; }
+    UPIC_D bool next(double ux, double uy, double dux, double duy, double& sa, double& sb) {
+        while (nb > 0) {
+            double s = fmin(sx, sy);
+            if (s < 1.0) {
+                const bool ex = sx == s, ey = sy == s;
+                if (ex) sx = next_knot(ux, dux, s);
+                if (ey) sy = next_knot(uy, duy, s);
+                nb += (ex ? 1 : 0) + (ey ? 1 : 0);
+                if (nb > kMaxBreaks) {
+                    nb = -1;
+                    return false;
+                }
+            } else {
+                s = 1.0;
+                nb = 0;
+            }
+            if (s - prev > 1.0e-12) {
+                sa = prev;
+                sb = s;
+                prev = s;
+                return true;
+            }
+        }
+        return false;
+    }
+};
+
+// Grid coordinate less the stencil offset: the stencil of a point starts at
+// node floor of it, its knots are the integers.
+template <int ORDER>
+UPIC_D double knot_coord(double x, double L, double inv_h) {
+    return (x + 0.5 * L) * inv_h - 0.5 * (double)(ORDER - 1);
+}
+
+// One segment's middle on one axis: first node and offset in its knot cell.
+UPIC_D int segment_cell(double u, double& t) {
+    const double fl = floor(u);
+    t = u - fl;
+    return (int)fl;
+}
+
+// Orbit averages along the orbit from (ux, uy) by (dux, duy) (knot_coord
+// units): gp = <grad phi_mid>, D[c][d] = <dA_c/dx_d> with
+// A = (1-s) A^n + s A^{n+1}, and A1 = A^{n+1} at the orbit's end, whose
+// stencil is the last segment's.  False: too many knots.  The loop over
+// stencil rows stays rolled (its row's coefficients are rotated to the front),
+// which bounds the registers of the unrolled loop over a row's nodes.
+template <int R, int SY>
+UPIC_D bool orbit_averages(const Geo& g, const double* __restrict__ rec, double ux, double uy, double dux, double duy,
+                           double gp[2], double D[3][2], double A1[3]) {
+    KnotWalk walk;
+    walk.init(ux, uy, dux, duy);
+    gp[0] = gp[1] = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) D[c][0] = D[c][1] = A1[c] = 0.0;
+    double sa, sb;
+    int ilx = 0, ily = 0;
+    while (walk.next(ux, uy, dux, duy, sa, sb)) {
+        const double len = sb - sa, sm = sa + 0.5 * len;
+        const double dx = len * dux, dy = len * duy;
+        double tx, ty = 0.0;
+        ilx = segment_cell(ux + sm * dux, tx);
+        if constexpr (SY > 1) ily = segment_cell(uy + sm * duy, ty);
+        double wx[R + 1], Gx[R][R + 1], wy[R + 1], Gy[R][R + 1];
+        spline_taylor<R>(tx, dx, wx, Gx);
+        if constexpr (SY > 1) spline_taylor<R>(ty, dy, wy, Gy);
+        const double* row[R + 1];
+#pragma unroll
+        for (int a = 0; a <= R; ++a) row[a] = rec + (size_t)(wrap_index(ilx + a, g.nx) * g.ny) * kIRec;
+#pragma unroll 1
+        for (int b = 0; b < SY; ++b) {
+            // U[i] = len <tau^i S_b>, V[i] = len <tau^i S'_b>
+            double U[R + 2], V[R + 2];
+#pragma unroll
+            for (int i = 0; i <= R + 1; ++i) {
+                if constexpr (SY > 1) {
+                    double u = 0.0, v = 0.0;
+#pragma unroll
+                    for (int j = 0; j <= R; ++j) {
+                        if (i <= R && !((i + j) & 1)) u = fma(tau_moment(i + j), taylor<R>(wy, Gy, dy, j, 0), u);
+                        if (j < R && !((i + j) & 1)) v = fma(tau_moment(i + j), Gy[j][0], v);
+                    }
+                    U[i] = len * u;
+                    V[i] = len * v;
+                } else {
+                    U[i] = len * tau_moment(i);
+                    V[i] = 0.0;
+                }
+            }
+            if constexpr (SY > 1) {
+                // the next row's coefficients to the front
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    wy[k] = wy[k + 1];
+#pragma unroll
+                    for (int i = 0; i < R; ++i) Gy[i][k] = Gy[i][k + 1];
+                }
+            }
+            const int off = SY == 1 ? 0 : wrap_index(ily + b, g.ny) * kIRec;
+#pragma unroll
+            for (int a = 0; a <= R; ++a) {
+                const double* r = row[a] + off;
+                const double2 r01 = __ldg(reinterpret_cast<const double2*>(r));
+                const double2 r23 = __ldg(reinterpret_cast<const double2*>(r + 2));
+                const double2 r45 = __ldg(reinterpret_cast<const double2*>(r + 4));
+                const double2 r67 = __ldg(reinterpret_cast<const double2*>(r + 6));
+                double m = 0.0, x0 = 0.0, x1 = 0.0, y0 = 0.0, y1 = 0.0;
+#pragma unroll
+                for (int i = 0; i <= R; ++i) {
+                    const double A = taylor<R>(wx, Gx, dx, i, a);
+                    m = fma(A, U[i], m);
+                    if constexpr (SY > 1) {
+                        y0 = fma(A, V[i], y0);
+                        y1 = fma(A, V[i + 1], y1);
+                    }
+                    if (i < R) {
+                        x0 = fma(Gx[i][a], U[i], x0);
+                        if (SY > 1 || ((i + 1) & 1) == 0) x1 = fma(Gx[i][a], U[i + 1], x1);
+                    }
+                }
+                // weights of A^n and A^{n+1}: <(1-s) .> and <s .>, s = sm + len tau
+                x1 = fma(sm, x0, len * x1);
+                x0 -= x1;
+                gp[0] = fma(r01.x, m, gp[0]);
+                gp[1] = fma(r01.y, m, gp[1]);
+                const double An[3] = {r23.x, r23.y, r45.x}, Ae[3] = {r45.y, r67.x, r67.y};
+#pragma unroll
+                for (int c = 0; c < 3; ++c) D[c][0] = fma(An[c], x0, fma(Ae[c], x1, D[c][0]));
+                if constexpr (SY > 1) {
+                    y1 = fma(sm, y0, len * y1);
+                    y0 -= y1;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) D[c][1] = fma(An[c], y0, fma(Ae[c], y1, D[c][1]));
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        D[c][0] *= g.inv_dx;
+        D[c][1] *= g.inv_dy;
+    }
+    // the orbit's end in the last segment's stencil
+    double ex[R + 1], ey[R + 1], unused[R][R + 1];
+    spline_taylor<R>(ux + dux - (double)ilx, 0.0, ex, unused);
+    if constexpr (SY > 1) spline_taylor<R>(uy + duy - (double)ily, 0.0, ey, unused);
+    else ey[0] = 1.0;
+#pragma unroll
+    for (int a = 0; a <= R; ++a) {
+        const double* r = rec + (size_t)(wrap_index(ilx + a, g.nx) * g.ny) * kIRec;
+#pragma unroll
+        for (int b = 0; b < SY; ++b) {
+            const int off = SY == 1 ? 0 : wrap_index(ily + b, g.ny) * kIRec;
+            const double e0 = __ldg(r + off + kIRecAe);
+            const double2 e12 = __ldg(reinterpret_cast<const double2*>(r + off + 6));
+            const double e = ex[a] * ey[b];
+            A1[0] = fma(e0, e, A1[0]);
+            A1[1] = fma(e12.x, e, A1[1]);
+            A1[2] = fma(e12.y, e, A1[2]);
+        }
+    }
+    return walk.nb == 0;
+}
+
+// Shape sums len <S_a S_b> of the segment [sa, sb] to out[(a SY + b) STEP].
+template <int R, int SY, int STEP>
+UPIC_D void segment_weights(double ux, double uy, double dux, double duy, double sa, double sb, double* out) {
+    const double len = sb - sa, sm = sa + 0.5 * len;
+    const double dx = len * dux, dy = len * duy;
+    double tx, ty = 0.0;
+    segment_cell(ux + sm * dux, tx);
+    if constexpr (SY > 1) segment_cell(uy + sm * duy, ty);
+    double wx[R + 1], Gx[R][R + 1], wy[R + 1], Gy[R][R + 1];
+    spline_taylor<R>(tx, dx, wx, Gx);
+    if constexpr (SY > 1) spline_taylor<R>(ty, dy, wy, Gy);
+#pragma unroll 1
+    for (int b = 0; b < SY; ++b) {
+        double U[R + 1];
+#pragma unroll
+        for (int i = 0; i <= R; ++i) {
+            if constexpr (SY > 1) {
+                double u = 0.0;
+#pragma unroll
+                for (int j = 0; j <= R; ++j)
+                    if (!((i + j) & 1)) u = fma(tau_moment(i + j), taylor<R>(wy, Gy, dy, j, 0), u);
+                U[i] = len * u;
+            } else {
+                U[i] = len * tau_moment(i);
+            }
+        }
+        if constexpr (SY > 1) {
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                wy[k] = wy[k + 1];
+#pragma unroll
+                for (int i = 0; i < R; ++i) Gy[i][k] = Gy[i][k + 1];
+            }
+        }
+#pragma unroll
+        for (int a = 0; a <= R; ++a) {
+            double m = 0.0;
+#pragma unroll
+            for (int i = 0; i <= R; ++i)
+                if (SY > 1 || !(i & 1)) m = fma(taylor<R>(wx, Gx, dx, i, a), U[i], m);
+            out[(a * SY + b) * STEP] = m;
+        }
+    }
+}
+
+// The local map of the closed-form solve: as kick_rotate_kick, with fewer
+// square roots and divisions.
+UPIC_D double rotate_closed(const double* pm, const double* B, double q, double m, double mk, double inv_mk,
+                        double dt, double* out) {
+    double u[3] = {pm[0] * inv_mk, pm[1] * inv_mk, pm[2] * inv_mk};
+    const double gm = sqrt(1.0 + dot3(u, u));
+    const double c = q * dt / (2.0 * m);
+    const double tau[3] = {c * B[0], c * B[1], c * B[2]};
+    const double tau2 = dot3(tau, tau);
+    const double udt = dot3(u, tau);
+    const double sigma = gm * gm - tau2;
+    const double ghc2 = 0.5 * (sigma + sqrt(sigma * sigma + 4.0 * (tau2 + udt * udt)));
+    const double inv_ghc = rsqrt(fmax(ghc2, 1.0));
+    const double t[3] = {tau[0] * inv_ghc, tau[1] * inv_ghc, tau[2] * inv_ghc};
+    const double sf = 2.0 / (1.0 + dot3(t, t));
+    const double sv[3] = {sf * t[0], sf * t[1], sf * t[2]};
+    const double up[3] = {u[0] + (u[1] * t[2] - u[2] * t[1]), u[1] + (u[2] * t[0] - u[0] * t[2]),
+                          u[2] + (u[0] * t[1] - u[1] * t[0])};
+    const double upl[3] = {u[0] + (up[1] * sv[2] - up[2] * sv[1]), u[1] + (up[2] * sv[0] - up[0] * sv[2]),
+                           u[2] + (up[0] * sv[1] - up[1] * sv[0])};
+    out[0] = mk * upl[0];
+    out[1] = mk * upl[1];
+    out[2] = mk * upl[2];
+    return gm;  // gamma of pm, and of the rotated momentum
+}
+
+// One evaluation's mapped orbit velocity, and what the particle's end state
+// is formed from when the evaluation is accepted (local_end).
+struct ClosedOut {
+    double vbar_map[3];
+    double P_end[3];
+    double A1p[3];
+    double gam;  // gamma of P_end - q A1p
+};
+
+// The kick-rotate-kick of one local map evaluation over a step h
+// (evaluate_local_particle_substep :4843-4929): the orbit averages gp =
+// <grad phi_mid> and D = <dA/dx>, A' at the orbit's end (A1p) and at its
+// midpoint ((A0p + A1p) / 2) give P_end and the secant orbit velocity
+// vbar_map.  Each gamma is evaluated once: gamma(pstart) is a particle
+// constant, the rotation keeps gamma(p_minus), so that it serves both
+// secants, and gamma(p_end) serves its secant and the end velocity; the two
+// secants share a division.
+UPIC_D void kick_closed(const LocalIn& in, const double* guess, double gp0, double gp1, const double (&D)[3][2],
+                             const double* A1p, double h, ClosedOut& o) {
+    const double Aep[3] = {0.5 * (in.A0p[0] + A1p[0]), 0.5 * (in.A0p[1] + A1p[1]),
+                           0.5 * (in.A0p[2] + A1p[2])};
+    // D vbar and the skew part K = D^T - D as B_eff (:4585-4620); the z
+    // columns of D vanish in 2D.
+    const double Dv[3] = {D[0][0] * guess[0] + D[0][1] * guess[1], D[1][0] * guess[0] + D[1][1] * guess[1],
+                          D[2][0] * guess[0] + D[2][1] * guess[1]};
+    const double B[3] = {D[2][1], -D[2][0], D[1][0] - D[0][1]};
+    const double q = in.q, m = in.m, hq = 0.5 * q * h;
+    const double gpb[3] = {gp0, gp1, 0.0};
+    double pm[3], pp[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) pm[c] = ((in.P0[c] - q * Aep[c]) - hq * gpb[c]) + hq * Dv[c];
+    const double gm = rotate_closed(pm, B, q, m, in.mk, in.inv_mk, h, pp);
+    double pend[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        o.P_end[c] = ((pp[c] + q * Aep[c]) - hq * gpb[c]) + hq * Dv[c];
+        o.A1p[c] = A1p[c];
+        pend[c] = o.P_end[c] - q * A1p[c];
+    }
+    o.gam = gamma_p_inv(pend, in.inv_mk);
+    // kinetic_secant_velocity (:682) of (p_minus, pstart) and (p_end, p_plus)
+    const double dm = gm + in.gstart, dp = o.gam + gm;
+    const double r = 0.5 / (m * dm * dp);
+    const double sm = r * dp, sp = r * dm;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o.vbar_map[c] = sm * (pm[c] + in.pstart[c]) + sp * (pend[c] + pp[c]);
+}
+
+// End position of the orbit of velocity vbar over h and the end velocity of
+// its accepted evaluation.
+UPIC_D void local_end(const Geo& g, const LocalIn& in, const double* vbar, double h, const ClosedOut& o, double& x1,
+                      double& y1, double* v_end) {
+    x1 = wrap1(in.x0 + h * vbar[0], g.Lx);
+    y1 = wrap1(in.y0 + h * vbar[1], g.Ly);
+    const double inv = 1.0 / (in.m * o.gam);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v_end[c] = (o.P_end[c] - in.q * o.A1p[c]) * inv;
+}
+
+// evaluate() of a knot-split orbit in closed form.
+template <int ORDER, int SY = ORDER + 1>
+UPIC_D bool evaluate_closed(const Geo& g, const double* __restrict__ rec, double dt, const LocalIn& in,
+                            const double* guess, ClosedOut& o) {
+    double gpv[2], D[3][2], A1p[3];
+    if (!orbit_averages<ORDER, SY>(g, rec, knot_coord<ORDER>(in.x0, g.Lx, g.inv_dx),
+                                   knot_coord<ORDER>(in.y0, g.Ly, g.inv_dy), dt * guess[0] * g.inv_dx,
+                                   dt * guess[1] * g.inv_dy, gpv, D, A1p))
+        return false;
+    kick_closed(in, guess, gpv[0], gpv[1], D, A1p, dt, o);
+    return true;
+}
+
 UPIC_D bool finite3(const double* v) { return isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]); }
 
 UPIC_D int window_coord(int s, int origin, int n, int w, int span) {
@@ -591,47 +970,330 @@ UPIC_D int window_coord(int s, int origin, int n, int w, int span) {
     return d <= w - span ? d : -1;
 }
 
-// MOM: segment moments (ORDER <= 2 with knot splitting on); otherwise the
-// orbit integrals are gathered point by point.  PICARD: the deposit of the
-// non-relativistic Picard map (evaluate_picard_map_orbit,
-// Project1/ec_pic_serial_demo.cpp:1455-1474): the orbit velocity is
-// vbar = (v_guess + v^n) / 2 with no local solve, followed by the same
-// orbit-averaged deposit.
-// PART: kPartFused (solve and deposit in one launch), kPartSolve (local
-// solves only; writes each particle's orbit velocity to vbar_*) or
-// kPartDeposit (the deposit of the orbits in vbar_*).
-// ONED: a grid one cell high (ny = 1): the y stencil is one row (SY = 1).
-template <int ORDER, bool UNIFORM, bool MOM, bool PICARD, int PART = kPartFused, bool ONED = false>
-__global__ void __launch_bounds__(kMapThreads, map_min_blocks(PART, MOM))
-implicit_map_kernel(ImplicitMapArgs a, TileGeom tg) {
-    constexpr bool kSolve = PART != kPartDeposit;
-    constexpr bool kDeposit = PART != kPartSolve;
+UPIC_D Geo map_geo(const ImplicitMapArgs& a, int nx, int ny) {
+    Geo g{nx, ny, a.Lx, a.Ly, a.inv_dx, a.inv_dy};
+    g.qs = a.qtab;
+    g.qw = a.qtab + kMaxQuad;
+    g.nq = a.nq;
+    return g;
+}
+
+// The local solves of one map evaluation (solve_local_particle_substep
+// :4930): one thread per particle; each writes the particle's accepted orbit
+// velocity (NaN: none) to vbar_* for the deposit launch and, with write_state,
+// its trial end state.  MOM: segment moments (knot splitting on; order 1 or 2
+// in 2D, any order on a grid one cell high); otherwise point by point.  SY:
+// nodes of the y stencil (1 on a grid one cell high).  The arithmetic is the
+// Gauss rule's, not the closed form: which iterate a particle stops at, and
+// with it the last reported residual, turns on single roundings of its map.
+// The particles are ordered by the number of knots their orbits pass within a
+// tile (sort.cu), so that a warp's lanes walk the same number of segments.
+// Warps take batches of 32 particles from a queue: a tile's batches differ in
+// segments and so in time, and a fixed stride gave the same CTAs the long
+// ones (SMs active 63% of the launch).
+template <int ORDER, bool UNIFORM, bool MOM, int SY>
+__global__ void __launch_bounds__(kMapThreads, solve_min_blocks(MOM))
+implicit_solve_kernel(ImplicitMapArgs a, int nx, int ny) {
+    const Geo g = map_geo(a, nx, ny);
+    unsigned long long it_total = 0;
+    int it_max = 0, nfail = 0;
+    unsigned long long first_fail = ~0ull;
+    double worst = 0.0;
+    const int lane = threadIdx.x & 31;
+    const unsigned nbatches = (unsigned)((a.np + 31) / 32), warps = gridDim.x * kMapWarps;
+    for (unsigned batch = blockIdx.x * kMapWarps + (threadIdx.x >> 5), next; batch < nbatches; batch = next) {
+        if (lane == 0) next = warps + atomicAdd(&a.stats->next_batch, 1u);
+        const long p = (long)batch * 32 + lane;
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        double guess[3] = {nan, nan, nan};
+        if (p < a.np && !(a.nsub && a.nsub[p] > 1)) {
+            LocalIn in;
+            in.x0 = a.x[p];
+            in.y0 = a.y[p];
+            in.P0[0] = a.Px[p];
+            in.P0[1] = a.Py[p];
+            in.P0[2] = a.Pz[p];
+            in.q = UNIFORM ? a.q0 : a.q[p];
+            in.m = UNIFORM ? a.m0 : a.m[p];
+            gather_rec3<ORDER, kIRec, SY>(g, a.rec, kIRecAn, in.x0, in.y0, in.A0p);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) in.pstart[c] = in.P0[c] - in.q * in.A0p[c];
+            set_local_constants(in, a.kappa);
+            guess[0] = a.warm_x ? a.warm_x[p] : a.vx[p];
+            guess[1] = a.warm_x ? a.warm_y[p] : a.vy[p];
+            guess[2] = a.warm_x ? a.warm_z[p] : a.vz[p];
+            double bk[kMaxBreaks];
+            int nb = 0;
+            // solve_local_particle_substep (:4930)
+            int reason = kLocalMaxIter;
+            int iters = 0;
+            double scaled = INFINITY;
+            LocalOut o;
+            for (int it = 0; it < a.loc_maxit; ++it) {
+                bool okev;
+                if constexpr (MOM)
+                    okev = evaluate_moments<ORDER, SY>(g, a.rec, a.dt, a.kappa, a.split, in, guess, o, bk, nb);
+                else
+                    okev = evaluate<ORDER, SY>(g, a.rec, a.dt, a.kappa, a.split, in, guess, o, bk, nb);
+                if (!okev) {
+                    reason = kLocalTooManyCrossings;
+                    break;
+                }
+                ++iters;
+                if (!finite3(o.vbar_map)) {
+                    reason = kLocalNonfiniteMap;
+                    break;
+                }
+                if (norm3(o.vbar_map) >= a.kappa) {
+                    reason = kLocalSuperluminalMap;
+                    break;
+                }
+                const double res[3] = {o.vbar_map[0] - guess[0], o.vbar_map[1] - guess[1],
+                                       o.vbar_map[2] - guess[2]};
+                const double sc = 0.5 * (norm3(o.vbar_map) + norm3(guess));
+                scaled = norm3(res) / (a.loc_atol + a.loc_rtol * sc);
+                if (scaled <= 1.0) {
+                    reason = kLocalOk;
+                    break;
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) guess[c] += a.loc_damp * res[c];
+                if (!finite3(guess)) {
+                    reason = kLocalNonfiniteIterate;
+                    break;
+                }
+                if (norm3(guess) >= a.kappa) {
+                    reason = kLocalSuperluminalIterate;
+                    break;
+                }
+            }
+            it_total += (unsigned long long)iters;
+            it_max = max(it_max, iters);
+            worst = fmax(worst, isfinite(scaled) ? scaled : 1.0e300);
+            const bool ok = reason == kLocalOk;
+            if (!ok) {
+                ++nfail;
+                const unsigned long long key = ((unsigned long long)(unsigned)a.id[p] << 8) | (unsigned)reason;
+                first_fail = key < first_fail ? key : first_fail;
+                if (a.failed) a.failed[atomicAdd(a.nfailed, 1)] = (int)p;
+                guess[0] = guess[1] = guess[2] = nan;
+            } else {
+                if (a.keep_x) {
+                    a.keep_x[p] = guess[0];
+                    a.keep_y[p] = guess[1];
+                    a.keep_z[p] = guess[2];
+                }
+                if (a.write_state) {
+                    a.ox[p] = o.x1;
+                    a.oy[p] = o.y1;
+                    a.oPx[p] = o.P_end[0];
+                    a.oPy[p] = o.P_end[1];
+                    a.oPz[p] = o.P_end[2];
+                    a.ovx[p] = o.v_end[0];
+                    a.ovy[p] = o.v_end[1];
+                    a.ovz[p] = o.v_end[2];
+                    a.obx[p] = guess[0];
+                    a.oby[p] = guess[1];
+                    a.obz[p] = guess[2];
+                }
+            }
+        }
+        if (p < a.np) {
+            a.vbar_x[p] = guess[0];
+            a.vbar_y[p] = guess[1];
+            a.vbar_z[p] = guess[2];
+        }
+        next = __shfl_sync(0xffffffffu, next, 0);
+    }
+    // statistics (integer atomics and max over bit patterns: order independent)
+    MapStats* st = a.stats;
+    for (int o = 16; o > 0; o >>= 1) {
+        it_total += __shfl_xor_sync(0xffffffffu, it_total, o);
+        it_max = max(it_max, __shfl_xor_sync(0xffffffffu, it_max, o));
+        nfail += __shfl_xor_sync(0xffffffffu, nfail, o);
+        const unsigned long long ff = __shfl_xor_sync(0xffffffffu, first_fail, o);
+        first_fail = ff < first_fail ? ff : first_fail;
+        worst = fmax(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (it_total) atomicAdd(&st->iter_total, it_total);
+        atomicMax(&st->iter_max, it_max);
+        if (nfail) {
+            atomicAdd(&st->failures, nfail);
+            atomicMin(&st->first_fail_key, first_fail);
+        }
+        atomicMax(&st->worst_scaled_bits, (unsigned long long)__double_as_longlong(worst));
+    }
+}
+
+// implicit_solve_kernel for large 2D sets (ImplicitMapArgs::closed_solve) with
+// the orbit integrals in closed form.  512 x 512 x 16 quadratic: 2.33 -> 1.38
+// ms a launch, 256 x 256 x 16 cubic 1.22 -> 0.53 ms (FP64 work per segment 410
+// -> 340 instructions quadratic, 64 record loads for 256 cubic; registers 168
+// with 344 B of spills -> 128).
+template <int ORDER, bool UNIFORM>
+__global__ void __launch_bounds__(kMapThreads, ORDER >= 3 ? 3 : 4)
+implicit_solve_closed_kernel(ImplicitMapArgs a, int nx, int ny) {
+    const Geo g = map_geo(a, nx, ny);
+    const double kappa2 = a.kappa * a.kappa;
+    unsigned long long it_total = 0;
+    int it_max = 0, nfail = 0;
+    unsigned long long first_fail = ~0ull;
+    double worst = 0.0;
+    const int lane = threadIdx.x & 31;
+    const unsigned nbatches = (unsigned)((a.np + 31) / 32), warps = gridDim.x * kMapWarps;
+    for (unsigned batch = blockIdx.x * kMapWarps + (threadIdx.x >> 5), next; batch < nbatches; batch = next) {
+        if (lane == 0) next = warps + atomicAdd(&a.stats->next_batch, 1u);
+        const long p = (long)batch * 32 + lane;
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        double guess[3] = {nan, nan, nan};
+        if (p < a.np && !(a.nsub && a.nsub[p] > 1)) {
+            LocalIn in;
+            in.x0 = a.x[p];
+            in.y0 = a.y[p];
+            in.P0[0] = a.Px[p];
+            in.P0[1] = a.Py[p];
+            in.P0[2] = a.Pz[p];
+            in.q = UNIFORM ? a.q0 : a.q[p];
+            in.m = UNIFORM ? a.m0 : a.m[p];
+            gather_rec3<ORDER>(g, a.rec, kIRecAn, in.x0, in.y0, in.A0p);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) in.pstart[c] = in.P0[c] - in.q * in.A0p[c];
+            set_local_constants(in, a.kappa);
+            const double* const* start = a.warm_x ? &a.warm_x : &a.vx;
+            guess[0] = start[0][p];
+            guess[1] = start[1][p];
+            guess[2] = start[2][p];
+            int reason = kLocalMaxIter, iters = 0;
+            double g2 = dot3(guess, guess), r2 = INFINITY, tol = 1.0;
+            ClosedOut o;
+            for (int it = 0; it < a.loc_maxit; ++it) {
+                const bool okev = evaluate_closed<ORDER>(g, a.rec, a.dt, in, guess, o);
+                if (!okev) {
+                    reason = kLocalTooManyCrossings;
+                    break;
+                }
+                ++iters;
+                // |vbar_map| >= kappa, a non-finite map included
+                const double m2 = dot3(o.vbar_map, o.vbar_map);
+                if (!(m2 < kappa2)) {
+                    reason = finite3(o.vbar_map) ? kLocalSuperluminalMap : kLocalNonfiniteMap;
+                    break;
+                }
+                const double res[3] = {o.vbar_map[0] - guess[0], o.vbar_map[1] - guess[1],
+                                       o.vbar_map[2] - guess[2]};
+                r2 = dot3(res, res);
+                tol = a.loc_atol + a.loc_rtol * (0.5 * (sqrt(m2) + sqrt(g2)));
+                if (r2 <= tol * tol) {
+                    reason = kLocalOk;
+                    break;
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) guess[c] += a.loc_damp * res[c];
+                g2 = dot3(guess, guess);
+                if (!(g2 < kappa2)) {
+                    reason = finite3(guess) ? kLocalSuperluminalIterate : kLocalNonfiniteIterate;
+                    break;
+                }
+            }
+            it_total += (unsigned long long)iters;
+            it_max = max(it_max, iters);
+            const bool ok = reason == kLocalOk;
+            const double scaled = sqrt(r2) / tol;
+            worst = fmax(worst, ok ? fmin(scaled, 1.0) : isfinite(scaled) ? scaled : 1.0e300);
+            if (!ok) {
+                ++nfail;
+                const unsigned long long key = ((unsigned long long)(unsigned)a.id[p] << 8) | (unsigned)reason;
+                first_fail = key < first_fail ? key : first_fail;
+                if (a.failed) a.failed[atomicAdd(a.nfailed, 1)] = (int)p;
+                guess[0] = guess[1] = guess[2] = nan;
+            } else {
+                if (a.keep_x) {
+                    a.keep_x[p] = guess[0];
+                    a.keep_y[p] = guess[1];
+                    a.keep_z[p] = guess[2];
+                }
+                if (a.write_state) {
+                    double x1, y1, v_end[3];
+                    local_end(g, in, guess, a.dt, o, x1, y1, v_end);
+                    a.ox[p] = x1;
+                    a.oy[p] = y1;
+                    a.oPx[p] = o.P_end[0];
+                    a.oPy[p] = o.P_end[1];
+                    a.oPz[p] = o.P_end[2];
+                    a.ovx[p] = v_end[0];
+                    a.ovy[p] = v_end[1];
+                    a.ovz[p] = v_end[2];
+                    a.obx[p] = guess[0];
+                    a.oby[p] = guess[1];
+                    a.obz[p] = guess[2];
+                }
+            }
+        }
+        if (p < a.np) {
+            a.vbar_x[p] = guess[0];
+            a.vbar_y[p] = guess[1];
+            a.vbar_z[p] = guess[2];
+        }
+        next = __shfl_sync(0xffffffffu, next, 0);
+    }
+    // statistics (integer atomics and max over bit patterns: order independent)
+    MapStats* st = a.stats;
+    for (int o = 16; o > 0; o >>= 1) {
+        it_total += __shfl_xor_sync(0xffffffffu, it_total, o);
+        it_max = max(it_max, __shfl_xor_sync(0xffffffffu, it_max, o));
+        nfail += __shfl_xor_sync(0xffffffffu, nfail, o);
+        const unsigned long long ff = __shfl_xor_sync(0xffffffffu, first_fail, o);
+        first_fail = ff < first_fail ? ff : first_fail;
+        worst = fmax(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (it_total) atomicAdd(&st->iter_total, it_total);
+        atomicMax(&st->iter_max, it_max);
+        if (nfail) {
+            atomicAdd(&st->failures, nfail);
+            atomicMin(&st->first_fail_key, first_fail);
+        }
+        atomicMax(&st->worst_scaled_bits, (unsigned long long)__double_as_longlong(worst));
+    }
+}
+
+// The orbit-averaged deposit (path_average_deposit_current :2784) of the
+// orbits in vbar_* (the local solves' result), over tile chunks of the sorted
+// particles, a persistent CTA walking consecutive chunks with one window of
+// fixed-point sums.  PICARD: the deposit of the non-relativistic Picard map
+// (evaluate_picard_map_orbit, Project1/ec_pic_serial_demo.cpp:1455-1474),
+// whose orbit velocity is vbar = (v_guess + v^n) / 2 with no local solve.
+// PRIV: closed-form shape sums into warp-private FP64 windows (deposit.cuh);
+// otherwise segment moments (MOM) or quadrature points, and the CTA shares
+// one window of fixed-point words, to which each group of equal cells of a
+// warp adds its sums.  512 x 512 x 16 quadratic 0.70 -> 0.37 ms a launch, 256
+// x 256 x 16 cubic 0.74 -> 0.10 ms (one item per segment instead of four).
+template <int ORDER, bool UNIFORM, bool MOM, bool PICARD, int SY, bool PRIV>
+__global__ void __launch_bounds__(kMapThreads, deposit_min_blocks(ORDER, MOM, PICARD, PRIV))
+implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
     constexpr int S = ORDER + 1;
-    constexpr int SY = ONED ? 1 : S;
     constexpr int SS = S * SY;
     constexpr int NV = 3 * SS;
     constexpr int RW = SS + 3;
+    constexpr int STAGE = PRIV ? RW * kColStride : 32 * RW;  // doubles staged per warp
     constexpr int NPER = (NV + 31) / 32;
     extern __shared__ unsigned long long smem_u64[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int WN = tg.wx * tg.wy;
+    const PrivateWindow pw = private_window(tg, S, SY);
+    const int psize = pw.ex * pw.ey * 3;
     unsigned long long* whi = smem_u64;
     unsigned long long* wlo = whi + 3 * WN;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* srow = reinterpret_cast<double*>(wlo + 3 * WN) + warp * 32 * RW;
-    int* sgk = reinterpret_cast<int*>(reinterpret_cast<double*>(wlo + 3 * WN) + kMapWarps * 32 * RW) + warp * 32;
-    double* squad = reinterpret_cast<double*>(reinterpret_cast<int*>(reinterpret_cast<double*>(wlo + 3 * WN) +
-                                                                       kMapWarps * 32 * RW) + kMapWarps * 32);
-    for (int i = threadIdx.x; i < 4 * kMaxQuad; i += blockDim.x) squad[i] = a.qtab[i];
-    __syncthreads();
+    double* wins = reinterpret_cast<double*>(smem_u64);
+    const int window_words = PRIV ? kMapWarps * psize : 6 * WN;
+    double* srow = reinterpret_cast<double*>(smem_u64 + ((window_words + 1) & ~1)) + warp * STAGE;
+    int* sgk = reinterpret_cast<int*>(reinterpret_cast<double*>(smem_u64 + ((window_words + 1) & ~1)) +
+                                      kMapWarps * STAGE) +
+               warp * 32;
 
-    Geo g{tg.nx, tg.ny, a.Lx, a.Ly, a.inv_dx, a.inv_dy};
-    g.qs = squad;
-    g.qw = squad + kMaxQuad;
-    g.ms = squad + 2 * kMaxQuad;
-    g.mw = squad + 3 * kMaxQuad;
-    g.nq = a.nq;
-    g.mnq = a.mnq;
     const int nx = tg.nx, ny = tg.ny, N = nx * ny;
+    const Geo g = map_geo(a, nx, ny);
     const int nch = *a.nchunks;
     const int c_begin = (int)(((long long)blockIdx.x * nch) / gridDim.x);
     const int c_end = (int)(((long long)(blockIdx.x + 1) * nch) / gridDim.x);
@@ -646,33 +1308,42 @@ implicit_map_kernel(ImplicitMapArgs a, TileGeom tg) {
         t_a[r] = ab / SY;
         t_b[r] = ab % SY;
         t_c[r] = t < NV ? t - 3 * ab : 0;
-        t_off[r] = t_a[r] * tg.wy + t_b[r];
+        t_off[r] = PRIV ? (t_a[r] * pw.ey + t_b[r]) * 3 + t_c[r] : t_a[r] * tg.wy + t_b[r];
     }
-
-    unsigned long long it_total = 0;
-    int it_max = 0, nfail = 0;
+    if (PRIV) {
+        for (int idx = threadIdx.x; idx < window_words; idx += blockDim.x) wins[idx] = 0.0;
+        __syncthreads();
+    }
+    int nfail = 0;
     unsigned long long first_fail = ~0ull;
-    double worst = 0.0;
 
     int cur_tile = -1, ox = 0, oy = 0;
+    auto fold = [&]() {
+        if constexpr (PRIV) {
+            fold_private<3, kMapWarps>(wins, psize, pw, tg, ox, oy, a.acc, a.scale, [](int c) { return c; });
+        } else {
+            for (int idx = threadIdx.x; idx < 3 * WN; idx += blockDim.x) {
+                const unsigned long long hi = whi[idx], lo = wlo[idx];
+                if ((hi | lo) == 0ull) continue;
+                const int cc = idx / WN, widx = idx - cc * WN;
+                const int lx = widx / tg.wy, ly = widx - lx * tg.wy;
+                const int gx = tg.full_x ? lx : wrap_index(ox + lx, nx);
+                const int gy = tg.full_y ? ly : wrap_index(oy + ly, ny);
+                atomicAdd(&a.acc[(size_t)(2 * cc) * N + gx * ny + gy], hi);
+                atomicAdd(&a.acc[(size_t)(2 * cc + 1) * N + gx * ny + gy], lo);
+            }
+        }
+    };
     for (int ci = c_begin; ci < c_end; ++ci) {
         const Chunk ch = a.chunks[ci];
-        if (kDeposit && ch.tile != cur_tile) {
+        if (ch.tile != cur_tile) {
             __syncthreads();
             if (cur_tile >= 0) {
-                for (int idx = threadIdx.x; idx < 3 * WN; idx += blockDim.x) {
-                    const unsigned long long hi = whi[idx], lo = wlo[idx];
-                    if ((hi | lo) == 0ull) continue;
-                    const int cc = idx / WN, widx = idx - cc * WN;
-                    const int lx = widx / tg.wy, ly = widx - lx * tg.wy;
-                    const int gx = tg.full_x ? lx : wrap_index(ox + lx, nx);
-                    const int gy = tg.full_y ? ly : wrap_index(oy + ly, ny);
-                    atomicAdd(&a.acc[(size_t)(2 * cc) * N + gx * ny + gy], hi);
-                    atomicAdd(&a.acc[(size_t)(2 * cc + 1) * N + gx * ny + gy], lo);
-                }
+                fold();
                 __syncthreads();
             }
-            for (int idx = threadIdx.x; idx < 6 * WN; idx += blockDim.x) whi[idx] = 0ull;
+            if (!PRIV)
+                for (int idx = threadIdx.x; idx < 6 * WN; idx += blockDim.x) whi[idx] = 0ull;
             cur_tile = ch.tile;
             const int tx = cur_tile / tg.nty, ty = cur_tile - tx * tg.nty;
             ox = tg.full_x ? 0 : tx * tg.tile_x - tg.guard - tg.lo;
@@ -683,182 +1354,98 @@ implicit_map_kernel(ImplicitMapArgs a, TileGeom tg) {
             const int p = base + threadIdx.x;
             const bool active = p < ch.end;
             bool ok = false;
-            double vb[3] = {0.0, 0.0, 0.0};
-            double bk[kMaxBreaks];
-            int nb = 0;
-            LocalIn in;
-            if (PART == kPartDeposit) {
-                // the orbit velocity the solve launch accepted (NaN: none)
-                if (active) {
+            double vb[3] = {0.0, 0.0, 0.0}, x0 = 0.0, y0 = 0.0, q = 0.0;
+            if (active) {
+                if (PICARD) {
+                    vb[0] = 0.5 * (a.gx[p] + a.vx[p]);
+                    vb[1] = 0.5 * (a.gy[p] + a.vy[p]);
+                    vb[2] = 0.5 * (a.gz[p] + a.vz[p]);
+                    ok = fabs(vb[0]) <= a.vb_limit && fabs(vb[1]) <= a.vb_limit && fabs(vb[2]) <= a.vb_limit;
+                } else {
                     vb[0] = a.vbar_x[p];
                     vb[1] = a.vbar_y[p];
                     vb[2] = a.vbar_z[p];
                     ok = finite3(vb);
-                    if (ok) {
-                        in.x0 = a.x[p];
-                        in.y0 = a.y[p];
-                        in.q = UNIFORM ? a.q0 : a.q[p];
-                        nb = breakpoints<ORDER>(g, in.x0, in.y0, a.dt * vb[0], a.dt * vb[1], a.split, bk);
-                        ok = nb >= 0;
-                    }
-                    if (!ok) nb = 0;
                 }
-            } else if (PICARD && active) {
-                in.x0 = a.x[p];
-                in.y0 = a.y[p];
-                in.q = UNIFORM ? a.q0 : a.q[p];
-                vb[0] = 0.5 * (a.gx[p] + a.vx[p]);
-                vb[1] = 0.5 * (a.gy[p] + a.vy[p]);
-                vb[2] = 0.5 * (a.gz[p] + a.vz[p]);
-                int reason = kLocalOk;
-                if (!(fabs(vb[0]) <= a.vb_limit && fabs(vb[1]) <= a.vb_limit && fabs(vb[2]) <= a.vb_limit)) {
-                    reason = kLocalNonfiniteIterate;
-                } else {
-                    nb = breakpoints<ORDER>(g, in.x0, in.y0, a.dt * vb[0], a.dt * vb[1], a.split, bk);
-                    if (nb < 0) reason = kLocalTooManyCrossings;
-                }
-                ok = reason == kLocalOk;
-                if (!ok) {
-                    nb = 0;
-                    ++nfail;
-                    const unsigned long long key = ((unsigned long long)(unsigned)a.id[p] << 8) | (unsigned)reason;
-                    first_fail = key < first_fail ? key : first_fail;
-                }
-            } else if (active && !(a.nsub && a.nsub[p] > 1)) {
-                in.x0 = a.x[p];
-                in.y0 = a.y[p];
-                in.P0[0] = a.Px[p];
-                in.P0[1] = a.Py[p];
-                in.P0[2] = a.Pz[p];
-                in.q = UNIFORM ? a.q0 : a.q[p];
-                in.m = UNIFORM ? a.m0 : a.m[p];
-                gather_rec3<ORDER, kIRec, SY>(g, a.rec, kIRecAn, in.x0, in.y0, in.A0p);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) in.pstart[c] = in.P0[c] - in.q * in.A0p[c];
-                set_local_constants(in, a.kappa);
-                double guess[3] = {a.vx[p], a.vy[p], a.vz[p]};
-                if (a.warm_x) {
-                    guess[0] = a.warm_x[p];
-                    guess[1] = a.warm_y[p];
-                    guess[2] = a.warm_z[p];
-                }
-                // solve_local_particle_substep (:4930)
-                int reason = kLocalMaxIter;
-                int iters = 0;
-                double scaled = INFINITY;
-                LocalOut o;
-                for (int it = 0; it < a.loc_maxit; ++it) {
-                    bool okev;
-                    if constexpr (MOM)
-                        okev = evaluate_moments<ORDER, SY>(g, a.rec, a.dt, a.kappa, a.split, in, guess, o, bk, nb);
-                    else
-                        okev = evaluate<ORDER, SY>(g, a.rec, a.dt, a.kappa, a.split, in, guess, o, bk, nb);
-                    if (!okev) {
-                        reason = kLocalTooManyCrossings;
-                        break;
-                    }
-                    ++iters;
-                    if (!finite3(o.vbar_map)) {
-                        reason = kLocalNonfiniteMap;
-                        break;
-                    }
-                    if (norm3(o.vbar_map) >= a.kappa) {
-                        reason = kLocalSuperluminalMap;
-                        break;
-                    }
-                    const double res[3] = {o.vbar_map[0] - guess[0], o.vbar_map[1] - guess[1],
-                                           o.vbar_map[2] - guess[2]};
-                    const double sc = 0.5 * (norm3(o.vbar_map) + norm3(guess));
-                    scaled = norm3(res) / (a.loc_atol + a.loc_rtol * sc);
-                    if (scaled <= 1.0) {
-                        reason = kLocalOk;
-                        break;
-                    }
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) guess[c] += a.loc_damp * res[c];
-                    if (!finite3(guess)) {
-                        reason = kLocalNonfiniteIterate;
-                        break;
-                    }
-                    if (norm3(guess) >= a.kappa) {
-                        reason = kLocalSuperluminalIterate;
-                        break;
-                    }
-                }
-                it_total += (unsigned long long)iters;
-                it_max = max(it_max, iters);
-                worst = fmax(worst, isfinite(scaled) ? scaled : 1.0e300);
-                ok = reason == kLocalOk;
-                if (!ok) {
-                    ++nfail;
-                    const unsigned long long key = ((unsigned long long)(unsigned)a.id[p] << 8) | (unsigned)reason;
-                    first_fail = key < first_fail ? key : first_fail;
-                    if (a.failed) a.failed[atomicAdd(a.nfailed, 1)] = p;
-                } else {
-                    vb[0] = guess[0];
-                    vb[1] = guess[1];
-                    vb[2] = guess[2];
-                    if (a.keep_x) {
-                        a.keep_x[p] = guess[0];
-                        a.keep_y[p] = guess[1];
-                        a.keep_z[p] = guess[2];
-                    }
-                    if (a.write_state) {
-                        a.ox[p] = o.x1;
-                        a.oy[p] = o.y1;
-                        a.oPx[p] = o.P_end[0];
-                        a.oPy[p] = o.P_end[1];
-                        a.oPz[p] = o.P_end[2];
-                        a.ovx[p] = o.v_end[0];
-                        a.ovy[p] = o.v_end[1];
-                        a.ovz[p] = o.v_end[2];
-                        a.obx[p] = guess[0];
-                        a.oby[p] = guess[1];
-                        a.obz[p] = guess[2];
-                    }
+                if (ok) {
+                    x0 = a.x[p];
+                    y0 = a.y[p];
+                    q = UNIFORM ? a.q0 : a.q[p];
                 }
             }
-            if constexpr (PART == kPartSolve) {
-                if (active) {
-                    const double nan = __longlong_as_double(0x7ff8000000000000ll);
-                    a.vbar_x[p] = ok ? vb[0] : nan;
-                    a.vbar_y[p] = ok ? vb[1] : nan;
-                    a.vbar_z[p] = ok ? vb[2] : nan;
-                }
-                continue;
-            }
-            // Orbit-averaged deposit of the accepted orbit (:2784).  Item k of
-            // a particle is its k-th segment (MOM: the segment's shape sums,
-            // one stencil per segment) or its k-th (segment, quadrature point)
-            // pair; the warp works through the items in rounds and reduces
-            // equal window keys.
+            int reason = active && PICARD && !ok ? kLocalNonfiniteIterate : kLocalOk;
+            // Items: the orbit's segments (MOM: the segment's shape sums) or its
+            // (segment, quadrature point) pairs; the warp works through them in
+            // rounds and reduces equal window keys.
             const double dxx = a.dt * vb[0], dxy = a.dt * vb[1];
-            const double qa = ok ? in.q * a.inv_dV : 0.0;
+            double bk[PRIV ? 1 : kMaxBreaks];
+            int nb = 0;
+            KnotWalk walk;
+            walk.nb = 0;
+            const double ux = knot_coord<ORDER>(x0, g.Lx, g.inv_dx), uy = knot_coord<ORDER>(y0, g.Ly, g.inv_dy);
+            const double dux = dxx * g.inv_dx, duy = dxy * g.inv_dy;
+            if constexpr (PRIV) {
+                if (ok) walk.init(ux, uy, dux, duy);
+                // an orbit with more knots than the walk holds deposits nothing
+                if (ok && fabs(dux) + fabs(duy) > (double)(kMaxBreaks - 6)) {
+                    KnotWalk all = walk;
+                    double sa, sb;
+                    while (all.next(ux, uy, dux, duy, sa, sb)) {
+                    }
+                    if (all.nb < 0) {
+                        walk.nb = 0;
+                        ok = false;
+                        reason = kLocalTooManyCrossings;
+                    }
+                }
+            } else if (ok) {
+                nb = breakpoints<ORDER>(g, x0, y0, dxx, dxy, a.split, bk);
+                if (nb < 0) {
+                    ok = false;
+                    reason = kLocalTooManyCrossings;
+                    nb = 0;
+                }
+            }
+            if (PICARD && reason != kLocalOk) {
+                ++nfail;
+                const unsigned long long key = ((unsigned long long)(unsigned)a.id[p] << 8) | (unsigned)reason;
+                first_fail = key < first_fail ? key : first_fail;
+            }
+            const double qa = ok ? q * a.inv_dV : 0.0;
             const double val[3] = {qa * vb[0], qa * vb[1], qa * vb[2]};
             const int nq = MOM ? 1 : g.nq;
-            const int nitems = ok ? (nb - 1) * nq : 0;
-            const int rounds = __reduce_max_sync(0xffffffffu, nitems);
-            for (int rd = 0; rd < rounds; ++rd) {
+            const int nitems = !PRIV && ok ? (nb - 1) * nq : 0;
+            for (int rd = 0; __any_sync(0xffffffffu, PRIV ? walk.more() : rd < nitems); ++rd) {
                 int key = kKeyNone, gx0 = 0, gy0 = 0;
-                double wgt[SS];
-                if (rd < nitems) {
+                int ilx = 0, ily = 0;
+                double sa = 0.0, sb = 0.0;   // PRIV: the segment
+                double wgt[PRIV ? 1 : SS];
+                bool have = false;
+                if constexpr (PRIV) {
+                    have = walk.next(ux, uy, dux, duy, sa, sb);
+                    if (have) {
+                        const double sm = sa + 0.5 * (sb - sa);
+                        ilx = (int)floor(ux + sm * dux);
+                        ily = (int)floor(uy + sm * duy);
+                    }
+                } else if (rd < nitems) {
                     const int k = rd / nq, iq = rd - k * nq;
-                    const double sa = bk[k], len = bk[k + 1] - bk[k];
-                    if (len > 0.0) {
-                        int ilx, ily;
+                    const double sk = bk[k], len = bk[k + 1] - bk[k];
+                    have = len > 0.0;
+                    if (have) {
                         if constexpr (MOM) {
                             (void)iq;
                             SegMoments<ORDER, SY> M;
-                            segment_moments<ORDER, false, SY>(g, in.x0, in.y0, dxx, dxy, sa, len, M);
+                            segment_moments<ORDER, false, SY>(g, x0, y0, dxx, dxy, sk, len, M);
                             ilx = M.ilx;
                             ily = M.ily;
 #pragma unroll
                             for (int j = 0; j < SS; ++j) wgt[j] = M.m[j];
                         } else {
-                            const double s = sa + len * g.qs[iq];
+                            const double s = sk + len * g.qs[iq];
                             const double wq = len * g.qw[iq];
-                            const double xs = wrap1(in.x0 + s * dxx, g.Lx);
-                            const double ys = wrap1(in.y0 + s * dxy, g.Ly);
+                            const double xs = wrap1(x0 + s * dxx, g.Lx);
+                            const double ys = wrap1(y0 + s * dxy, g.Ly);
                             Stencil<ORDER> sx, sy;
                             stencil_xy<ORDER, SY>(g, xs, ys, sx, sy);
                             ilx = sx.il;
@@ -868,39 +1455,56 @@ implicit_map_kernel(ImplicitMapArgs a, TileGeom tg) {
 #pragma unroll
                                 for (int ib = 0; ib < SY; ++ib) wgt[ia * SY + ib] = wq * sx.w[ia] * sy.w[ib];
                         }
-                        gx0 = wrap_index(ilx, nx);
-                        gy0 = wrap_index(ily, ny);
-                        const int lx = tg.full_x ? gx0 : window_coord(ilx, ox, nx, tg.wx, S);
-                        const int ly = tg.full_y ? gy0 : window_coord(ily, oy, ny, tg.wy, SY);
-                        key = (lx < 0 || ly < 0) ? kKeyEscape : lx * tg.wy + ly;
                     }
+                }
+                if (have) {
+                    gx0 = wrap_index(ilx, nx);
+                    gy0 = wrap_index(ily, ny);
+                    const int lx = tg.full_x ? gx0 : window_coord(ilx, ox, nx, tg.wx, S);
+                    const int ly = tg.full_y ? gy0 : window_coord(ily, oy, ny, tg.wy, SY);
+                    key = (lx < 0 || ly < 0) ? kKeyEscape : PRIV ? (lx * pw.ey + ly) * 3 : lx * tg.wy + ly;
                 }
                 const unsigned full = 0xffffffffu;
                 const unsigned lt = (1u << lane) - 1u;
                 const unsigned valid = __ballot_sync(full, key >= 0);
                 const unsigned esc = __ballot_sync(full, key == kKeyEscape);
-                const unsigned peers = __match_any_sync(full, key);
-                int row = -1, nvalid = 0, ngroups = 0;
+                int row = -1, nvalid = 0;
                 unsigned heads = 0u;
-                for (unsigned rem = valid; rem;) {
-                    const int l = __ffs(rem) - 1;
-                    const unsigned gm = __shfl_sync(full, peers, l);
-                    const int gk = __shfl_sync(full, key, l);
-                    if ((gm >> lane) & 1u) row = nvalid + __popc(gm & lt);
-                    if (lane == 0) sgk[ngroups] = gk;
-                    heads |= 1u << nvalid;
-                    nvalid += __popc(gm);
-                    rem &= ~gm;
-                    ++ngroups;
+                if constexpr (PRIV) {
+                    heads = run_heads(key, valid);
+                } else {
+                    const unsigned peers = __match_any_sync(full, key);
+                    int ngroups = 0;
+                    for (unsigned rem = valid; rem;) {
+                        const int l = __ffs(rem) - 1;
+                        const unsigned gm = __shfl_sync(full, peers, l);
+                        const int gk = __shfl_sync(full, key, l);
+                        if ((gm >> lane) & 1u) row = nvalid + __popc(gm & lt);
+                        if (lane == 0) sgk[ngroups] = gk;
+                        heads |= 1u << nvalid;
+                        nvalid += __popc(gm);
+                        rem &= ~gm;
+                        ++ngroups;
+                    }
                 }
-                if (key == kKeyEscape) row = nvalid + __popc(esc & lt);
-                if (row >= 0) {
-                    double* mine = srow + row * RW;
+                if (!PRIV && key == kKeyEscape) row = nvalid + __popc(esc & lt);
+                // value k of this lane's particle goes to mine[k * step]
+                double* mine = PRIV ? srow + lane : srow + row * RW;
+                constexpr int step = PRIV ? kColStride : 1;
+                if (PRIV && key == kKeyNone) {
 #pragma unroll
-                    for (int j = 0; j < SS; ++j) mine[j] = wgt[j];
-                    mine[SS + 0] = val[0];
-                    mine[SS + 1] = val[1];
-                    mine[SS + 2] = val[2];
+                    for (int k = 0; k < RW; ++k) mine[k * step] = 0.0;
+                }
+                if (PRIV ? key != kKeyNone : row >= 0) {
+                    if constexpr (PRIV) {
+                        segment_weights<ORDER, SY, step>(ux, uy, dux, duy, sa, sb, mine);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < SS; ++j) mine[j] = wgt[j];
+                    }
+                    mine[(SS + 0) * step] = val[0];
+                    mine[(SS + 1) * step] = val[1];
+                    mine[(SS + 2) * step] = val[2];
                 }
                 __syncwarp();
                 {
@@ -915,7 +1519,8 @@ implicit_map_kernel(ImplicitMapArgs a, TileGeom tg) {
                         for (int r = 0; r < NPER; ++r) {
                             const int t = lane + 32 * r;
                             if (t < NV) {
-                                const double v = srow[erow * RW + SS + t_c[r]] * srow[erow * RW + t_ab[r]];
+                                const double v = PRIV ? srow[(SS + t_c[r]) * step + j] * srow[t_ab[r] * step + j]
+                                                      : srow[erow * RW + SS + t_c[r]] * srow[erow * RW + t_ab[r]];
                                 if (v != 0.0) {
                                     const int gi = wrap_index(gxj + t_a[r], nx) * ny + wrap_index(gyj + t_b[r], ny);
                                     const Fixed2 f = to_fixed(v, a.scale[t_c[r]]);
@@ -927,7 +1532,16 @@ implicit_map_kernel(ImplicitMapArgs a, TileGeom tg) {
                         ++erow;
                     }
                 }
-                {
+                if (PRIV && esc) {
+                    // escaped particles are done: their columns add nothing
+                    __syncwarp();
+                    if (key == kKeyEscape)
+                        for (int k = 0; k < 3; ++k) mine[(SS + k) * step] = 0.0;
+                    __syncwarp();
+                }
+                if constexpr (PRIV) {
+                    if (valid) add_columns<NV, SS>(srow, key, valid, heads, wins + warp * psize, t_ab, t_c, t_off);
+                } else {
                     unsigned h = heads;
                     int gi = 0;
                     while (h) {
@@ -965,40 +1579,20 @@ implicit_map_kernel(ImplicitMapArgs a, TileGeom tg) {
             }
         }
     }
-    if (kDeposit) {
-        __syncthreads();
-        if (cur_tile >= 0) {
-            for (int idx = threadIdx.x; idx < 3 * WN; idx += blockDim.x) {
-                const unsigned long long hi = whi[idx], lo = wlo[idx];
-                if ((hi | lo) == 0ull) continue;
-                const int cc = idx / WN, widx = idx - cc * WN;
-                const int lx = widx / tg.wy, ly = widx - lx * tg.wy;
-                const int gx = tg.full_x ? lx : wrap_index(ox + lx, nx);
-                const int gy = tg.full_y ? ly : wrap_index(oy + ly, ny);
-                atomicAdd(&a.acc[(size_t)(2 * cc) * N + gx * ny + gy], hi);
-                atomicAdd(&a.acc[(size_t)(2 * cc + 1) * N + gx * ny + gy], lo);
-            }
-        }
+    __syncthreads();
+    if (cur_tile >= 0) {
+        fold();
     }
-    if (!kSolve) return;
-    // statistics (integer atomics and max over bit patterns: order independent)
+    if (!PICARD) return;
     MapStats* st = a.stats;
     for (int o = 16; o > 0; o >>= 1) {
-        it_total += __shfl_xor_sync(0xffffffffu, it_total, o);
-        it_max = max(it_max, __shfl_xor_sync(0xffffffffu, it_max, o));
         nfail += __shfl_xor_sync(0xffffffffu, nfail, o);
         const unsigned long long ff = __shfl_xor_sync(0xffffffffu, first_fail, o);
         first_fail = ff < first_fail ? ff : first_fail;
-        worst = fmax(worst, __shfl_xor_sync(0xffffffffu, worst, o));
     }
-    if (lane == 0) {
-        if (it_total) atomicAdd(&st->iter_total, it_total);
-        atomicMax(&st->iter_max, it_max);
-        if (nfail) {
-            atomicAdd(&st->failures, nfail);
-            atomicMin(&st->first_fail_key, first_fail);
-        }
-        atomicMax(&st->worst_scaled_bits, (unsigned long long)__double_as_longlong(worst));
+    if (lane == 0 && nfail) {
+        atomicAdd(&st->failures, nfail);
+        atomicMin(&st->first_fail_key, first_fail);
     }
 }
 
@@ -1016,10 +1610,7 @@ __global__ void __launch_bounds__(128) refined_map_kernel(ImplicitMapArgs a, int
     Geo g{nx, ny, a.Lx, a.Ly, a.inv_dx, a.inv_dy};
     g.qs = a.qtab;
     g.qw = a.qtab + kMaxQuad;
-    g.ms = a.qtab + 2 * kMaxQuad;
-    g.mw = a.qtab + 3 * kMaxQuad;
     g.nq = a.nq;
-    g.mnq = a.mnq;
     const int N = nx * ny;
     unsigned long long it_total = 0;
     int it_max = 0, nfail = 0;
@@ -1255,7 +1846,7 @@ UPIC_D bool traced_solve(const ImplicitMapArgs& a, const double* start, Eval eva
 // failed substep, theta0, theta1, h, iterations, reason, first / final
 // scaled residual, final absolute residual, q, m, x0 (3), P0 (3), initial
 // guess (3), last guess (3), last map (3).
-template <int ORDER, bool UNIFORM, bool MOM, int SY>
+template <int ORDER, bool UNIFORM, bool MOM, int SY, bool CLOSED = false>
 __global__ void __launch_bounds__(128) failure_report_kernel(ImplicitMapArgs a, int nx, int ny, const int* failed,
                                                              int nf, double* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1263,10 +1854,7 @@ __global__ void __launch_bounds__(128) failure_report_kernel(ImplicitMapArgs a, 
     Geo g{nx, ny, a.Lx, a.Ly, a.inv_dx, a.inv_dy};
     g.qs = a.qtab;
     g.qw = a.qtab + kMaxQuad;
-    g.ms = a.qtab + 2 * kMaxQuad;
-    g.mw = a.qtab + 3 * kMaxQuad;
     g.nq = a.nq;
-    g.mnq = a.mnq;
     const int p = failed[i];
     const int n = a.nsub ? a.nsub[p] : 1;
     const double q = UNIFORM ? a.q0 : a.q[p];
@@ -1295,10 +1883,16 @@ __global__ void __launch_bounds__(128) failure_report_kernel(ImplicitMapArgs a, 
         start[1] = a.warm_x ? a.warm_y[p] : v[1];
         start[2] = a.warm_x ? a.warm_z[p] : v[2];
         traced_solve(a, start, [&](const double* gs, LocalOut& o) {
-            if constexpr (MOM)
+            if constexpr (CLOSED) {
+                ClosedOut c;
+                const bool ok = evaluate_closed<ORDER>(g, a.rec, a.dt, in, gs, c);
+                for (int k = 0; k < 3; ++k) o.vbar_map[k] = c.vbar_map[k];
+                return ok;
+            } else if constexpr (MOM) {
                 return evaluate_moments<ORDER, SY>(g, a.rec, a.dt, a.kappa, a.split, in, gs, o, bk, nb);
-            else
+            } else {
                 return evaluate<ORDER, SY>(g, a.rec, a.dt, a.kappa, a.split, in, gs, o, bk, nb);
+            }
         }, t);
     } else {
         h = a.dt / (double)n;
@@ -1540,10 +2134,7 @@ __global__ void gmhc_push_kernel(ImplicitMapArgs a, int nx, int ny, long np, con
     Geo g{nx, ny, a.Lx, a.Ly, a.inv_dx, a.inv_dy};
     g.qs = a.qtab;
     g.qw = a.qtab + kMaxQuad;
-    g.ms = a.qtab + 2 * kMaxQuad;
-    g.mw = a.qtab + 3 * kMaxQuad;
     g.nq = a.nq;
-    g.mnq = a.mnq;
     for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < np; p += (long)gridDim.x * blockDim.x) {
         LocalIn in;
         in.x0 = in7[p];
@@ -2309,18 +2900,19 @@ __global__ void __launch_bounds__(kRed) grid_work_kernel(int N, const double* J,
 // P_end = P + dt (-q <grad phi> + q D_A^T vbar), v_next = (P_end - q A)/m.
 // Writes the trial state (sorted order) and per-CTA double-double partials of
 // |v_next - v_guess|^2, |v_next|^2, |v_guess|^2 in the residual-norm layout.
-template <int ORDER, bool UNIFORM, bool MOM>
-__global__ void __launch_bounds__(kRed) picard_push_kernel(PicardPushArgs a) {
+template <int ORDER, bool UNIFORM, bool MOM, int SY>
+__global__ void __launch_bounds__(kRed, 2) picard_push_kernel(PicardPushArgs a) {
     Geo g{a.nx, a.ny, a.Lx, a.Ly, a.inv_dx, a.inv_dy};
     g.qs = a.qtab;
     g.qw = a.qtab + kMaxQuad;
-    g.ms = a.qtab + 2 * kMaxQuad;
-    g.mw = a.qtab + 3 * kMaxQuad;
     g.nq = a.nq;
-    g.mnq = a.mnq;
     DD d2{0, 0}, n2{0, 0}, g2{0, 0};
     int nfail = 0;
-    for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < a.np; p += (long)gridDim.x * blockDim.x) {
+    // block i takes batch i + r of round r: a fixed stride would keep a block
+    // at one place of the tiles, whose batches differ in segments per orbit
+    for (long round = 0; round * gridDim.x * blockDim.x < a.np; ++round) {
+        const long p = (round * gridDim.x + (blockIdx.x + round) % gridDim.x) * blockDim.x + threadIdx.x;
+        if (p >= a.np) continue;
         const double x0 = a.x[p], y0 = a.y[p];
         const double vg[3] = {a.gx[p], a.gy[p], a.gz[p]};
         const double vb[3] = {0.5 * (vg[0] + a.vx[p]), 0.5 * (vg[1] + a.vy[p]), 0.5 * (vg[2] + a.vz[p])};
@@ -2328,18 +2920,19 @@ __global__ void __launch_bounds__(kRed) picard_push_kernel(PicardPushArgs a) {
         const double m = UNIFORM ? a.m0 : a.m[p];
         const double dxx = a.dt * vb[0], dxy = a.dt * vb[1];
         const double x1 = wrap1(x0 + dxx, g.Lx), y1 = wrap1(y0 + dxy, g.Ly);
-        double b[kMaxBreaks];
-        const int nb = breakpoints<ORDER>(g, x0, y0, dxx, dxy, a.split, b);
-        double gp[2] = {0.0, 0.0}, D[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-        if (nb < 0) {
-            ++nfail;
-        } else if constexpr (MOM) {
-            orbit_integrals_moments<ORDER>(g, a.rec, x0, y0, dxx, dxy, b, nb, gp, D);
+        double gp[2] = {0.0, 0.0}, D[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}}, A1p[3];
+        if constexpr (MOM) {
+            if (!orbit_averages<ORDER, SY>(g, a.rec, knot_coord<ORDER>(x0, g.Lx, g.inv_dx),
+                                           knot_coord<ORDER>(y0, g.Ly, g.inv_dy), dxx * g.inv_dx, dxy * g.inv_dy, gp,
+                                           D, A1p))
+                ++nfail;
         } else {
-            orbit_integrals_points<ORDER>(g, a.rec, x0, y0, dxx, dxy, b, nb, gp, D);
+            double b[kMaxBreaks];
+            const int nb = breakpoints<ORDER>(g, x0, y0, dxx, dxy, a.split, b);
+            if (nb < 0) ++nfail;
+            else orbit_integrals_points<ORDER, SY>(g, a.rec, x0, y0, dxx, dxy, b, nb, gp, D);
+            gather_rec3<ORDER, kIRec, SY>(g, a.rec, kIRecAe, x1, y1, A1p);
         }
-        double A1p[3];
-        gather_rec3<ORDER>(g, a.rec, kIRecAe, x1, y1, A1p);
         // D_A^T vbar (the z derivatives vanish in 2D)
         const double DATv[3] = {D[0][0] * vb[0] + D[1][0] * vb[1] + D[2][0] * vb[2],
                                 D[0][1] * vb[0] + D[1][1] * vb[1] + D[2][1] * vb[2], 0.0};
@@ -2590,113 +3183,137 @@ int gsize(long n, int threads = 256) {
     return g < 1 ? 1 : (int)g;
 }
 
-using MapKernel = void (*)(ImplicitMapArgs, TileGeom);
+// The instance of a kernel template <ORDER, UNIFORM, MOM, SY> (or with PICARD
+// before SY) for the order, uniform q/m, the closed form and a grid one cell
+// high (SY = 1; without the closed form the full stencil, which wraps).
+using SolveKernel = void (*)(ImplicitMapArgs, int, int);
+using DepositKernel = void (*)(ImplicitMapArgs, TileGeom);
+using PicardPushKernel = void (*)(PicardPushArgs);
 
-// The map kernel instance of (order, uniform q/m, knot splitting, Picard
-// deposit, part).
-template <bool PICARD, int PART>
-MapKernel map_kernel_of(int order, bool uniform, bool split) {
-    const bool mom = split && order <= 2;
-#define UPIC_K(O, U, M) &implicit_map_kernel<O, U, M, PICARD, PART>
-    switch (order) {
-        case 1:
-            return mom ? (uniform ? UPIC_K(1, true, true) : UPIC_K(1, false, true))
-                       : (uniform ? UPIC_K(1, true, false) : UPIC_K(1, false, false));
-        case 2:
-            return mom ? (uniform ? UPIC_K(2, true, true) : UPIC_K(2, false, true))
-                       : (uniform ? UPIC_K(2, true, false) : UPIC_K(2, false, false));
-        case 3: return uniform ? UPIC_K(3, true, false) : UPIC_K(3, false, false);
-        case 4: return uniform ? UPIC_K(4, true, false) : UPIC_K(4, false, false);
+template <int O, bool U>
+SolveKernel solve_kernel_of(bool split, bool oned) {
+    if (split && oned) return implicit_solve_kernel<O, U, true, 1>;
+    if constexpr (O <= 2) {
+        if (split) return implicit_solve_kernel<O, U, true, O + 1>;
     }
-#undef UPIC_K
+    return implicit_solve_kernel<O, U, false, O + 1>;
+}
+template <int O, bool U, bool P>
+DepositKernel deposit_kernel_of(bool split, bool oned, bool priv) {
+    if (priv) return implicit_deposit_kernel<O, U, true, P, O + 1, true>;
+    if constexpr (!P) {
+        if (split && oned) return implicit_deposit_kernel<O, U, true, P, 1, false>;
+    }
+    if constexpr (O <= 2) {
+        if (split) return implicit_deposit_kernel<O, U, true, P, O + 1, false>;
+    }
+    return implicit_deposit_kernel<O, U, false, P, O + 1, false>;
+}
+template <int O, bool U>
+PicardPushKernel picard_push_of(bool closed, bool oned) {
+    if (!closed) return picard_push_kernel<O, U, false, O + 1>;
+    return oned ? picard_push_kernel<O, U, true, 1> : picard_push_kernel<O, U, true, O + 1>;
+}
+
+#define UPIC_BY_ORDER(F)            \
+    switch (order) {                \
+        case 1: return F(1);        \
+        case 2: return F(2);        \
+        case 3: return F(3);        \
+        case 4: return F(4);        \
+    }                               \
     return nullptr;
+
+SolveKernel solve_kernel(int order, bool uniform, bool split, bool oned) {
+#define UPIC_F(O) (uniform ? solve_kernel_of<O, true>(split, oned) : solve_kernel_of<O, false>(split, oned))
+    UPIC_BY_ORDER(UPIC_F)
+#undef UPIC_F
+}
+template <bool U, bool P>
+DepositKernel deposit_kernel_up(int order, bool split, bool oned, bool priv) {
+#define UPIC_F(O) (deposit_kernel_of<O, U, P>(split, oned, priv))
+    UPIC_BY_ORDER(UPIC_F)
+#undef UPIC_F
+}
+DepositKernel deposit_kernel(int order, bool uniform, bool split, bool picard, bool oned, bool priv) {
+    if (uniform)
+        return picard ? deposit_kernel_up<true, true>(order, split, oned, priv)
+                      : deposit_kernel_up<true, false>(order, split, oned, priv);
+    return picard ? deposit_kernel_up<false, true>(order, split, oned, priv)
+                  : deposit_kernel_up<false, false>(order, split, oned, priv);
+}
+SolveKernel solve_closed_kernel(int order, bool uniform) {
+#define UPIC_F(O) (uniform ? implicit_solve_closed_kernel<O, true> : implicit_solve_closed_kernel<O, false>)
+    UPIC_BY_ORDER(UPIC_F)
+#undef UPIC_F
+}
+PicardPushKernel picard_push(int order, bool uniform, bool closed, bool oned) {
+#define UPIC_F(O) (uniform ? picard_push_of<O, true>(closed, oned) : picard_push_of<O, false>(closed, oned))
+    UPIC_BY_ORDER(UPIC_F)
+#undef UPIC_F
+}
+#undef UPIC_BY_ORDER
+
+}  // namespace
+
+namespace {
+
+// Shared memory of the deposit launch with private or shared windows.
+int deposit_smem(const TileGeom& tg, int order, bool priv) {
+    const int S = order + 1, row = S * S + 3;
+    if (priv) return kMapWarps * (private_window_doubles(tg, S, S, 3) + row * kColStride) * 8 + 8;
+    return 2 * 3 * tg.wx * tg.wy * 8 + kMapWarps * (32 * row * 8 + 32 * 4);
 }
 
-// The one-row (ny = 1) instances of the split launches: segment moments for
-// every order (knot splitting on; one y node leaves (ORDER + 1) moments per
-// segment).
-template <int PART>
-MapKernel map_kernel_oned(int order, bool uniform) {
-#define UPIC_K1(O) (uniform ? &implicit_map_kernel<O, true, true, false, PART, true> \
-                            : &implicit_map_kernel<O, false, true, false, PART, true>)
-    switch (order) {
-        case 1: return UPIC_K1(1);
-        case 2: return UPIC_K1(2);
-        case 3: return UPIC_K1(3);
-        case 4: return UPIC_K1(4);
-    }
-#undef UPIC_K1
-    return nullptr;
-}
-
-// oned: the grid is one cell high; its split launches (relativistic map,
-// knot splitting on) use the one-row instances.
-MapKernel map_kernel(int order, bool uniform, bool split, bool picard, int part = kPartFused, bool oned = false) {
-    if (picard) return map_kernel_of<true, kPartFused>(order, uniform, split);
-    if (oned && split && part == kPartSolve) return map_kernel_oned<kPartSolve>(order, uniform);
-    if (oned && split && part == kPartDeposit) return map_kernel_oned<kPartDeposit>(order, uniform);
-    switch (part) {
-        case kPartSolve: return map_kernel_of<false, kPartSolve>(order, uniform, split);
-        case kPartDeposit: return map_kernel_of<false, kPartDeposit>(order, uniform, split);
-        default: return map_kernel_of<false, kPartFused>(order, uniform, split);
-    }
-}
-
-// Split launches for the relativistic map when the caller supplied the
-// hand-over buffers.
-bool use_split(const ImplicitMapArgs& a, bool picard) {
-    return UPIC_MAP_SPLIT && !picard && a.vbar_x && a.vbar_y && a.vbar_z;
+// Private windows where the closed form holds and four CTAs fit an SM (the
+// default tile of 8 cells takes 30-52 KB); a larger tile, a user's choice,
+// keeps the shared window, which needs a quarter to a half of the memory.  So
+// does a grid one cell high: its few nodes hold many particles each, so that
+// the deposit is small beside the solve (37 and 103 us at 150,000 particles)
+// and the order of its sums shows in the last residual.
+bool deposit_private(const TileGeom& tg, int order, bool closed) {
+    return closed && tg.ny > 1 && deposit_smem(tg, order, true) <= 55 * 1024;
 }
 
 }  // namespace
 
-int implicit_map_smem_bytes(const TileGeom& tg, int order) {
-    const int S = order + 1;
-    const int RW = S * S + 3;
-    return 2 * 3 * tg.wx * tg.wy * 8 + kMapWarps * (32 * RW * 8 + 32 * 4) + 4 * kMaxQuad * 8;
-}
-
-cudaError_t implicit_configure_smem(const TileGeom& tg, int order, bool split, bool picard) {
-    const int b = implicit_map_smem_bytes(tg, order);
+cudaError_t implicit_configure_smem(const TileGeom& tg, int order, bool split, bool closed, bool picard) {
+    const bool priv = deposit_private(tg, order, closed);
+    const int b = deposit_smem(tg, order, priv);
     for (int u = 0; u < 2; ++u) {
-        for (int part = kPartFused; part <= (picard ? kPartFused : kPartDeposit); ++part) {
-            MapKernel k = map_kernel(order, u != 0, split, picard, part, tg.ny == 1);
-            if (!k) return cudaErrorInvalidValue;
-            const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), b);
-            if (e != cudaSuccess) return e;
-        }
+        const DepositKernel k = deposit_kernel(order, u != 0, split, picard, tg.ny == 1, priv);
+        if (!k) return cudaErrorInvalidValue;
+        const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), b);
+        if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
-int implicit_map_occupancy(const TileGeom& tg, int order, bool split, bool picard) {
+int implicit_deposit_occupancy(const TileGeom& tg, int order, bool split, bool closed, bool picard) {
     int n = 0;
-    MapKernel k = map_kernel(order, true, split, picard);
+    const bool priv = deposit_private(tg, order, closed);
+    const DepositKernel k = deposit_kernel(order, true, split, picard, tg.ny == 1, priv);
     if (!k) return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kMapThreads, implicit_map_smem_bytes(tg, order));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kMapThreads, deposit_smem(tg, order, priv));
     return n;
 }
 
-cudaError_t launch_implicit_map(int order, bool uniform, bool split, const TileGeom& tg,
-                                const ImplicitMapArgs& a, int grid, cudaStream_t st, bool picard) {
-    const int smem = implicit_map_smem_bytes(tg, order);
-    if (use_split(a, picard)) {
-        MapKernel ks = map_kernel(order, uniform, split, picard, kPartSolve, tg.ny == 1);
-        MapKernel kd = map_kernel(order, uniform, split, picard, kPartDeposit, tg.ny == 1);
-        if (!ks || !kd) return cudaErrorInvalidValue;
-        // grid is sized for the fused kernel's resident CTAs; each part is
-        // given as many CTAs as it keeps resident
-        const bool mom = (tg.ny == 1 && split) || (split && order <= 2);
-        const int gs = grid / kMapMinBlocks * map_min_blocks(kPartSolve, mom);
-        const int gd = grid / kMapMinBlocks * map_min_blocks(kPartDeposit, mom);
-        ks<<<gs > 0 ? gs : grid, kMapThreads, smem, st>>>(a, tg);
-        kd<<<gd > 0 ? gd : grid, kMapThreads, smem, st>>>(a, tg);
-        count_launches(2);
-        return cudaGetLastError();
+cudaError_t launch_implicit_map(int order, bool uniform, const TileGeom& tg, const ImplicitMapArgs& a, int nsm,
+                                int deposit_grid, cudaStream_t st, bool picard) {
+    const bool priv = deposit_private(tg, order, a.closed != 0);
+    const DepositKernel kd = deposit_kernel(order, uniform, a.split != 0, picard, tg.ny == 1, priv);
+    if (!kd) return cudaErrorInvalidValue;
+    if (!picard) {
+        const SolveKernel ks = a.closed_solve ? solve_closed_kernel(order, uniform)
+                                              : solve_kernel(order, uniform, a.split != 0, tg.ny == 1);
+        if (!ks) return cudaErrorInvalidValue;
+        const long blocks = (a.np + kMapThreads - 1) / kMapThreads;
+        const bool mom = a.split && (order <= 2 || tg.ny == 1);
+        const int resident = nsm * (a.closed_solve ? (order >= 3 ? 3 : 4) : solve_min_blocks(mom));
+        ks<<<(int)(blocks < resident ? blocks : resident), kMapThreads, 0, st>>>(a, tg.nx, tg.ny);
+        count_launches(1);
     }
-    MapKernel k = map_kernel(order, uniform, split, picard);
-    if (!k) return cudaErrorInvalidValue;
-    k<<<grid, kMapThreads, smem, st>>>(a, tg);
+    kd<<<deposit_grid, kMapThreads, deposit_smem(tg, order, priv), st>>>(a, tg);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -2720,18 +3337,19 @@ cudaError_t launch_refined_map(int order, bool uniform, const ImplicitMapArgs& a
     return cudaGetLastError();
 }
 
-cudaError_t launch_failure_report(int order, bool uniform, bool split, const TileGeom& tg, const ImplicitMapArgs& a,
+cudaError_t launch_failure_report(int order, bool uniform, const TileGeom& tg, const ImplicitMapArgs& a,
                                   const int* failed, int nf, double* out, cudaStream_t st) {
     if (nf <= 0) return cudaSuccess;
     const int g = (nf + 127) / 128;
-    // the evaluation form of the map launch (map_kernel): one-row instances for
-    // split launches on a grid one cell high, segment moments for split
-    // orbits of order <= 2
-    const bool oned = tg.ny == 1 && split && use_split(a, false);
-    const bool mom = oned || (split && order <= 2);
+    // the evaluation form of the map launch (solve_kernel)
+    const bool oned = tg.ny == 1 && a.split;
+    const bool mom = oned || (a.split && order <= 2);
 #define UPIC_FR(O, U, M, SY) failure_report_kernel<O, U, M, SY><<<g, 128, 0, st>>>(a, tg.nx, tg.ny, failed, nf, out)
 #define UPIC_FR_ORDER(O)                                                    \
-    if (oned) {                                                             \
+    if (a.closed_solve) {                                                   \
+        if (uniform) failure_report_kernel<O, true, false, O + 1, true><<<g, 128, 0, st>>>(a, tg.nx, tg.ny, failed, nf, out); \
+        else failure_report_kernel<O, false, false, O + 1, true><<<g, 128, 0, st>>>(a, tg.nx, tg.ny, failed, nf, out); \
+    } else if (oned) {                                                             \
         if (uniform) UPIC_FR(O, true, true, 1); else UPIC_FR(O, false, true, 1); \
     } else if (mom && O <= 2) {                                             \
         if (uniform) UPIC_FR(O, true, (O <= 2), O + 1); else UPIC_FR(O, false, (O <= 2), O + 1); \
@@ -2826,24 +3444,11 @@ cudaError_t launch_grid_work(int N, const double* J, const double* rec12, double
     return cudaGetLastError();
 }
 
-cudaError_t launch_picard_push(int order, bool uniform, bool split, const PicardPushArgs& a, int grid,
-                              NormSums* out, cudaStream_t st) {
-    const bool mom = split && order <= 2;
-#define UPIC_PP(O, U, M) picard_push_kernel<O, U, M><<<grid, kRed, 0, st>>>(a)
-    switch (order) {
-        case 1:
-            if (mom) { if (uniform) UPIC_PP(1, true, true); else UPIC_PP(1, false, true); }
-            else { if (uniform) UPIC_PP(1, true, false); else UPIC_PP(1, false, false); }
-            break;
-        case 2:
-            if (mom) { if (uniform) UPIC_PP(2, true, true); else UPIC_PP(2, false, true); }
-            else { if (uniform) UPIC_PP(2, true, false); else UPIC_PP(2, false, false); }
-            break;
-        case 3: if (uniform) UPIC_PP(3, true, false); else UPIC_PP(3, false, false); break;
-        case 4: if (uniform) UPIC_PP(4, true, false); else UPIC_PP(4, false, false); break;
-        default: return cudaErrorInvalidValue;
-    }
-#undef UPIC_PP
+cudaError_t launch_picard_push(int order, bool uniform, const PicardPushArgs& a, int grid, NormSums* out,
+                               cudaStream_t st) {
+    const PicardPushKernel k = picard_push(order, uniform, a.closed != 0, a.ny == 1);
+    if (!k) return cudaErrorInvalidValue;
+    k<<<grid, kRed, 0, st>>>(a);
     residual_final_kernel<<<1, 32, 0, st>>>(a.partials, grid, out);
     count_launches(2);
     return cudaGetLastError();

@@ -39,6 +39,7 @@ struct MapStats {
     // particles, ~0 when none failed
     unsigned long long first_fail_key;
     unsigned long long worst_scaled_bits;  // max final scaled residual (bit pattern)
+    unsigned next_batch;                   // work queue of the solve launch: 32-particle batches handed out
 };
 
 struct ImplicitMapArgs {
@@ -64,11 +65,14 @@ struct ImplicitMapArgs {
     unsigned long long* acc;  // [comp][hi,lo][N]
     double scale[3];
     MapStats* stats;
-    // Gauss rules on [0, 1] (device, 4 x kMaxQuad doubles: nodes and
-    // weights of the deck's nq-point rule, then of the mnq-point rule used
-    // for segment moments)
+    // Gauss rule on [0, 1] of the orbit sums (device, nodes, then weights at
+    // + kMaxQuad)
     const double* qtab;
-    int nq, mnq;
+    int nq;
+    // knot splitting on and a deck rule that integrates the segments' polynomials
+    // exactly: the deposit's shape sums in closed form, and with closed_solve the
+    // local solves' orbit integrals
+    int closed, closed_solve;
     // Picard deposit (picard = true): guess velocities, orbit vbar = (guess + v) / 2;
     // a particle with a component of vbar above vb_limit (or not finite) is
     // counted as a failure, since its deposit could leave the fixed-point range
@@ -94,8 +98,7 @@ struct ImplicitMapArgs {
     int* failed;
     int* nfailed;
     // orbit velocities handed from the local-solve launch to the deposit
-    // launch of a split map evaluation (NaN for a particle that deposits
-    // nothing), or null: one fused launch
+    // launch (NaN for a particle that deposits nothing)
     double *vbar_x, *vbar_y, *vbar_z;
 };
 // The refined particles of a sub-cycled map evaluation: chained local
@@ -106,19 +109,27 @@ cudaError_t launch_refined_map(int order, bool uniform, const ImplicitMapArgs& a
 // arguments are a (kFailRec doubles each, in failed order), for a grid of
 // tg's size: each particle's failing local solve run again with its report.
 constexpr int kFailRec = 28;
-cudaError_t launch_failure_report(int order, bool uniform, bool split, const TileGeom& tg, const ImplicitMapArgs& a,
+cudaError_t launch_failure_report(int order, bool uniform, const TileGeom& tg, const ImplicitMapArgs& a,
                                   const int* failed, int nf, double* out, cudaStream_t st);
 // nsub[p] = 1 for p < n
 cudaError_t launch_fill_int(int n, int value, int* out, cudaStream_t st);
 
-// split: knot splitting of the orbit (ImplicitMapArgs::split); picard: the
-// non-relativistic Picard deposit instead of the local GM-HC solve.  Both
-// select the kernel instance.
-cudaError_t launch_implicit_map(int order, bool uniform, bool split, const TileGeom& tg,
-                                const ImplicitMapArgs& a, int grid, cudaStream_t st, bool picard = false);
-int implicit_map_smem_bytes(const TileGeom& tg, int order);
-cudaError_t implicit_configure_smem(const TileGeom& tg, int order, bool split, bool picard = false);
-int implicit_map_occupancy(const TileGeom& tg, int order, bool split, bool picard = false);
+// The local solves and the deposit (deposit_grid CTAs) of a map evaluation on
+// nsm SMs; picard: the non-relativistic Picard deposit alone.
+cudaError_t launch_implicit_map(int order, bool uniform, const TileGeom& tg, const ImplicitMapArgs& a, int nsm,
+                                int deposit_grid, cudaStream_t st, bool picard = false);
+cudaError_t implicit_configure_smem(const TileGeom& tg, int order, bool split, bool closed, bool picard);
+// Resident CTAs per SM of the deposit.
+int implicit_deposit_occupancy(const TileGeom& tg, int order, bool split, bool closed, bool picard);
+// The local solves take their orbit integrals in closed form from this many
+// particles on (2D).  Which iterate a particle's fixed point stops at turns on
+// single roundings, and each particle that stops elsewhere than with the Gauss
+// rule's roundings moves the mean iteration count by 1 / np and the last
+// residual, with the convergence rate reported from it, by about 1e-12 / np
+// of the current: from half a million particles on both stay below 1e-9 of
+// the report's values, below it a step is latency (64 x 64 x 16: 71 us of 430
+// per map evaluation).
+constexpr long kClosedSolveMin = 1L << 19;
 
 // Point deposit of rho (q S / dV, slot 3) and J (q v S / dV, slots 0..2) at
 // the particle positions (deposit_scalar_to_mesh :2117, deposit_current_to_mesh
@@ -310,13 +321,13 @@ struct PicardPushArgs {
     int nx, ny;
     double Lx, Ly, inv_dx, inv_dy, dt;
     const double* rec;
-    int split, nq, mnq;
+    int split, closed, nq;
     const double* qtab;
     double* partials;  // grid x 8
     int* err;          // += particles whose orbit crosses too many knots
 };
-cudaError_t launch_picard_push(int order, bool uniform, bool split, const PicardPushArgs& a, int grid,
-                              NormSums* out, cudaStream_t st);
+cudaError_t launch_picard_push(int order, bool uniform, const PicardPushArgs& a, int grid, NormSums* out,
+                               cudaStream_t st);
 // P = m v, v_prev = v - dt (q/m) E(x) (Project1 start-up).
 cudaError_t launch_picard_startup(int order, int nx, int ny, double Lx, double Ly, const double* E3, long np,
                                   const double* x, const double* y, const double* vx, const double* vy,

@@ -90,6 +90,11 @@ struct TileGeom {
     // nearest node for the explicit method (origin 0, shift 1/2), the cell
     // floor((x + L/2) / dx) for the implicit method (origin L/2, shift 0)
     double key_origin_x, key_origin_y, key_shift;
+    // Sub-order of a tile's particles before their cells: with classes > 1, by
+    // the number of knots (at most classes - 1) that the orbit x + class_dt v
+    // passes, the knots of an axis lying at grid coordinate class_off + integer
+    int classes;
+    double class_dt, class_off;
 };
 
 struct Chunk {

@@ -5,7 +5,11 @@
 // particles are periodically reordered by the nearest-node cell of their next
 // gather position, in tile-major cell order, so that a warp's 32 particles
 // share a handful of cells (broadcast gathers, long runs in the segmented
-// deposit reduction) and a CTA's chunk fits one shared-memory window.
+// deposit reduction) and a CTA's chunk fits one shared-memory window.  The
+// implicit methods order a tile's particles by the number of knots their
+// orbits pass before their cells (TileGeom::classes): a warp that walks its
+// lanes' segments in rounds otherwise takes two or three rounds for a mean of
+// 1.2 segments.
 //
 // The sort is a stable LSD radix sort of (cell key, index) pairs written for
 // this purpose: block histograms, a device-wide exclusive scan, and a scatter
@@ -40,7 +44,15 @@ __global__ void make_keys_kernel(TileGeom tg, ParticleSoA p, long np, double Lx,
         const int icy = wrap_index((int)floor((y + tg.key_origin_y) * inv_dy + tg.key_shift), tg.ny);
         const int tx = icx / tg.tile_x, lx = icx - tx * tg.tile_x;
         const int ty = icy / tg.tile_y, ly = icy - ty * tg.tile_y;
-        const unsigned tile = (unsigned)(tx * tg.nty + ty);
+        unsigned tile = (unsigned)(tx * tg.nty + ty);
+        if (tg.classes > 1) {
+            const double ux = (x + tg.key_origin_x) * inv_dx - tg.class_off;
+            const double uy = (y + tg.key_origin_y) * inv_dy - tg.class_off;
+            const double n = fabs(floor(ux + tg.class_dt * p.vx[q] * inv_dx) - floor(ux)) +
+                             fabs(floor(uy + tg.class_dt * p.vy[q] * inv_dy) - floor(uy));
+            const double most = (double)(tg.classes - 1);
+            tile = tile * (unsigned)tg.classes + (unsigned)(n < most ? n : most);
+        }
         keys[q] = tile * (unsigned)(tg.tile_x * tg.tile_y) + (unsigned)(lx * tg.tile_y + ly);
     }
 }
@@ -302,7 +314,7 @@ int grid_for(long n) {
 // Digit passes of the radix sort for the grid's cell keys: ceil(bits / 8)
 // passes of equal width (at most 8 bits).
 int radix_passes(const TileGeom& tg, int* dbits) {
-    const long ncells = (long)tg.nx * tg.ny;
+    const long ncells = (long)tg.nx * tg.ny * tg.classes;
     int bits = 0;
     while ((1L << bits) < ncells) ++bits;
     if (bits == 0) bits = 1;
@@ -364,7 +376,7 @@ cudaError_t sort_keys_to_chunks(const TileGeom& tg, long np, SortWork& w, cudaSt
     }
     // chunk table
     const int ntiles = tg.ntx * tg.nty;
-    tile_bounds_kernel<<<grid_for(np + 1), 256, 0, st>>>(w.keys, np, (unsigned)(tg.tile_x * tg.tile_y),
+    tile_bounds_kernel<<<grid_for(np + 1), 256, 0, st>>>(w.keys, np, (unsigned)(tg.tile_x * tg.tile_y * tg.classes),
                                                          ntiles, w.tile_start);
     tile_counts_kernel<<<(ntiles + 255) / 256, 256, 0, st>>>(w.tile_start, ntiles, w.tile_count);
     count_launches(2);
