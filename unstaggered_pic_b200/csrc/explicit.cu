@@ -13,6 +13,7 @@
 #include <map>
 #include <mutex>
 #include <utility>
+#include "deposit.cuh"
 #include "kernels.h"
 #include "upic_common.cuh"
 
@@ -28,14 +29,11 @@ namespace {
 #ifndef UPIC_PUSH_MIN_BLOCKS
 #define UPIC_PUSH_MIN_BLOCKS 3
 #endif
-// 1: the step push stages its tile window's field records in shared memory
-// and gathers from there (the same sums in the same order as the global
-// gather, which remains for stencils outside the window)
-#ifndef UPIC_PUSH_SMEM_GATHER
-#define UPIC_PUSH_SMEM_GATHER 1
-#endif
 constexpr int kPushThreads = UPIC_PUSH_THREADS;
 constexpr int kPushWarps = kPushThreads / kWarp;
+// With private windows two CTAs fit an SM and their threads keep their values
+// in registers.
+constexpr int push_min_blocks(bool priv) { return priv ? 2 : UPIC_PUSH_MIN_BLOCKS; }
 constexpr int kKeyNone = -1;
 constexpr int kKeyEscape = -2;
 
@@ -124,8 +122,11 @@ UPIC_D void prefetch_next_batch(const PushArgs& a, const Chunk& ch, int base, in
     prefetch_l2(arr, n0, n1);
 }
 
-template <int MODE, int NCOMP, bool UNIFORM>
-__global__ void __launch_bounds__(kPushThreads, UPIC_PUSH_MIN_BLOCKS)
+// PRIV: warp-private FP64 windows (deposit.cuh); otherwise the CTA shares one
+// window of fixed-point words, to which each group of equal cells of a warp
+// adds its sums.
+template <int MODE, int NCOMP, bool UNIFORM, bool PRIV>
+__global__ void __launch_bounds__(kPushThreads, push_min_blocks(PRIV))
 push_deposit_kernel(PushArgs a, TileGeom tg) {
     constexpr int NV = StageLayout<NCOMP>::kNV;
     constexpr int RW = StageLayout<NCOMP>::kRow;
@@ -135,21 +136,20 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
     unsigned long long* whi = smem_u64;
     unsigned long long* wlo = whi + NCOMP * WN;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* sprod = reinterpret_cast<double*>(wlo + NCOMP * WN) + warp * StageLayout<NCOMP>::kDoubles;
-    int* sgk = reinterpret_cast<int*>(reinterpret_cast<double*>(wlo + NCOMP * WN) +
-                                      kPushWarps * StageLayout<NCOMP>::kDoubles) + warp * 32;
-#if UPIC_PUSH_SMEM_GATHER
+    const PrivateWindow pw = private_window(tg, 3, 3);
+    const int psize = pw.ex * pw.ey * NCOMP;
+    double* wins = reinterpret_cast<double*>(smem_u64);
+    constexpr int STAGE = PRIV ? RW * kColStride : StageLayout<NCOMP>::kDoubles;  // doubles staged per warp
+    const int window_words = PRIV ? (kPushWarps * psize + 1) & ~1 : 2 * NCOMP * WN;
+    double* sprod = reinterpret_cast<double*>(smem_u64 + window_words) + warp * STAGE;
+    int* sgk = reinterpret_cast<int*>(smem_u64 + window_words + kPushWarps * STAGE) + warp * 32;
     // field records of the tile's window (kModePush): the gathers of
     // particles whose stencil lies in the window read them from here
-    // (16-byte aligned; the offset is taken from the shared base so that the
-    // pointer keeps the shared state space and the gathers are LDS, not
-    // generic loads)
-    unsigned char* const sbytes = reinterpret_cast<unsigned char*>(smem_u64);
-    const unsigned char* const sgk_end = reinterpret_cast<const unsigned char*>(
-        reinterpret_cast<int*>(reinterpret_cast<double*>(wlo + NCOMP * WN) +
-                               kPushWarps * StageLayout<NCOMP>::kDoubles) + kPushWarps * 32);
-    double2* srec = reinterpret_cast<double2*>(sbytes + (((sgk_end - sbytes) + 15) & ~ptrdiff_t(15)));
-#endif
+    // (16-byte aligned; an offset from the shared base, so that the pointer
+    // keeps the shared state space and the gathers are LDS, not generic
+    // loads)
+    double2* srec = reinterpret_cast<double2*>(
+        smem_u64 + ((window_words + kPushWarps * STAGE + (PRIV ? 0 : kPushWarps * 16) + 1) & ~1));
 
     const int nx = tg.nx, ny = tg.ny;
     const int N = nx * ny;
@@ -161,7 +161,6 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
     // stencil node ab = t / NCOMP (a = ab/3 along x, b = ab%3 along y) and
     // deposit component c = t % NCOMP
     int t_off[NPER], t_a[NPER], t_b[NPER], t_c[NPER], t_ab[NPER];
-    double t_scale[NPER];
 #pragma unroll
     for (int r = 0; r < NPER; ++r) {
         const int t = lane + 32 * r;
@@ -170,8 +169,11 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
         t_a[r] = ab / 3;
         t_b[r] = ab % 3;
         t_c[r] = t < NV ? t - ab * NCOMP : 0;
-        t_off[r] = t_a[r] * tg.wy + t_b[r];
-        t_scale[r] = a.scale[acc_slot(NCOMP, t_c[r])];
+        t_off[r] = PRIV ? (t_a[r] * pw.ey + t_b[r]) * NCOMP + t_c[r] : t_a[r] * tg.wy + t_b[r];
+    }
+    if (PRIV) {
+        for (int idx = threadIdx.x; idx < window_words; idx += blockDim.x) wins[idx] = 0.0;
+        __syncthreads();
     }
 
     DD kin{0.0, 0.0}, gsum{0.0, 0.0};
@@ -179,20 +181,27 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
     const double c2 = a.c * a.c;
 
     int cur_tile = -1, ox = 0, oy = 0;
+    auto fold = [&]() {
+        if constexpr (PRIV)
+            fold_private<NCOMP, kPushWarps>(wins, psize, pw, tg, ox, oy, a.acc, a.scale,
+                                            [](int c) { return acc_slot(NCOMP, c); });
+        else
+            fold_window<NCOMP>(whi, wlo, WN, tg, ox, oy, a.acc);
+    };
     for (int ci = c_begin; ci < c_end; ++ci) {
         const Chunk ch = a.chunks[ci];
         if (ch.tile != cur_tile) {
             __syncthreads();
             if (cur_tile >= 0) {
-                fold_window<NCOMP>(whi, wlo, WN, tg, ox, oy, a.acc);
+                fold();
                 __syncthreads();
             }
-            for (int idx = threadIdx.x; idx < 2 * NCOMP * WN; idx += blockDim.x) whi[idx] = 0ull;
+            if (!PRIV)
+                for (int idx = threadIdx.x; idx < 2 * NCOMP * WN; idx += blockDim.x) whi[idx] = 0ull;
             cur_tile = ch.tile;
             const int tx = cur_tile / tg.nty, ty = cur_tile - tx * tg.nty;
             ox = tg.full_x ? 0 : tx * tg.tile_x - tg.guard - 1;
             oy = tg.full_y ? 0 : ty * tg.tile_y - tg.guard - 1;
-#if UPIC_PUSH_SMEM_GATHER
             if (MODE == kModePush) {
                 const double2* g2 = reinterpret_cast<const double2*>(a.gfields);
                 for (int idx = threadIdx.x; idx < WN * (kGFStride / 2); idx += blockDim.x) {
@@ -203,7 +212,6 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                     srec[idx] = __ldg(g2 + (size_t)(gx * ny + gy) * (kGFStride / 2) + f);
                 }
             }
-#endif
             __syncthreads();
         }
         for (int base = ch.start; base < ch.end; base += kPushThreads) {
@@ -228,7 +236,6 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                     double G[12];
 #pragma unroll
                     for (int f = 0; f < 12; ++f) G[f] = 0.0;
-#if UPIC_PUSH_SMEM_GATHER
                     const int lx0 = tg.full_x ? 0 : window_coord(qx.ic - 1, ox, nx, tg.wx);
                     const int ly0 = tg.full_y ? 0 : window_coord(qy.ic - 1, oy, ny, tg.wy);
                     if (lx0 >= 0 && ly0 >= 0) {
@@ -249,7 +256,6 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                             }
                         }
                     } else
-#endif
 #pragma unroll
                     for (int ia = 0; ia < 3; ++ia) {
                         const int gx = wrap_index(qx.ic - 1 + ia, nx);
@@ -329,12 +335,58 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                 gy0 = wrap_index(dy_.ic - 1, ny);
                 const int lx = tg.full_x ? gx0 : window_coord(dx_.ic - 1, ox, nx, tg.wx);
                 const int ly = tg.full_y ? gy0 : window_coord(dy_.ic - 1, oy, ny, tg.wy);
-                key = (lx < 0 || ly < 0) ? kKeyEscape : lx * tg.wy + ly;
+                key = (lx < 0 || ly < 0) ? kKeyEscape : PRIV ? (lx * pw.ey + ly) * NCOMP : lx * tg.wy + ly;
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     dwx[k] = wxs[k];
                     dwy[k] = wys[k];
                 }
+            }
+            if constexpr (PRIV) {
+                // stage S_ab and q v_c / dA column by column
+                const unsigned full = 0xffffffffu;
+                const unsigned valid = __ballot_sync(full, key >= 0);
+                const unsigned esc = __ballot_sync(full, key == kKeyEscape);
+                const unsigned heads = run_heads(key, valid);
+                double* mine = sprod + lane;
+#pragma unroll
+                for (int ia = 0; ia < 3; ++ia)
+#pragma unroll
+                    for (int ib = 0; ib < 3; ++ib)
+                        mine[(ia * 3 + ib) * kColStride] = key == kKeyNone ? 0.0 : dwx[ia] * dwy[ib];
+#pragma unroll
+                for (int cc = 0; cc < NCOMP; ++cc) mine[(9 + cc) * kColStride] = key == kKeyNone ? 0.0 : dval[cc];
+                __syncwarp();
+                if (esc) {
+                    // stencils that leave the window (rare): exact fixed-point
+                    // adds straight to the grid, then nothing for the window
+                    for (unsigned e = esc; e; e &= e - 1) {
+                        const int j = __ffs(e) - 1;
+                        const int gxj = __shfl_sync(full, gx0, j);
+                        const int gyj = __shfl_sync(full, gy0, j);
+#pragma unroll
+                        for (int r = 0; r < NPER; ++r) {
+                            if (lane + 32 * r < NV) {
+                                const double v = sprod[(9 + t_c[r]) * kColStride + j] * sprod[t_ab[r] * kColStride + j];
+                                if (v != 0.0) {
+                                    const int g = wrap_index(gxj + t_a[r], nx) * ny + wrap_index(gyj + t_b[r], ny);
+                                    const int sl = acc_slot(NCOMP, t_c[r]);
+                                    const Fixed2 f = to_fixed(v, a.scale[sl]);
+                                    atomicAdd(&a.acc[(size_t)(2 * sl) * N + g], f.hi);
+                                    atomicAdd(&a.acc[(size_t)(2 * sl + 1) * N + g], f.lo);
+                                }
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (key == kKeyEscape)
+#pragma unroll
+                        for (int cc = 0; cc < NCOMP; ++cc) mine[(9 + cc) * kColStride] = 0.0;
+                    __syncwarp();
+                }
+                if (valid)
+                    add_columns<NV, 9, NPER>(sprod, key, valid, heads, wins + warp * psize, t_ab, t_c, t_off);
+                continue;
             }
             // Group the warp's particles by window key: groups in the order of
             // their first particle, particles in index order inside a group
@@ -387,7 +439,7 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                             if (v != 0.0) {
                                 const int g = wrap_index(gxj + t_a[r], nx) * ny + wrap_index(gyj + t_b[r], ny);
                                 const int sl = acc_slot(NCOMP, t_c[r]);
-                                const Fixed2 f = to_fixed(v, t_scale[r]);
+                                const Fixed2 f = to_fixed(v, a.scale[sl]);
                                 atomicAdd(&a.acc[(size_t)(2 * sl) * N + g], f.hi);
                                 atomicAdd(&a.acc[(size_t)(2 * sl + 1) * N + g], f.lo);
                             }
@@ -433,7 +485,7 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                                 } else {
                                     widx = k + t_off[r];
                                 }
-                                const Fixed2 f = to_fixed(sum, t_scale[r]);
+                                const Fixed2 f = to_fixed(sum, a.scale[acc_slot(NCOMP, t_c[r])]);
                                 atomicAdd(&whi[t_c[r] * WN + widx], f.hi);
                                 atomicAdd(&wlo[t_c[r] * WN + widx], f.lo);
                             }
@@ -445,7 +497,7 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
         }
     }
     __syncthreads();
-    if (cur_tile >= 0) fold_window<NCOMP>(whi, wlo, WN, tg, ox, oy, a.acc);
+    if (cur_tile >= 0) fold();
     // particle reductions: fixed order (lanes, then warps in index order)
     if (a.diag_part) {
         kin = warp_sum_dd(kin);
@@ -875,17 +927,37 @@ int grid_for(long n, int threads) {
     return (int)g;
 }
 
-template <int MODE, int NCOMP, bool UNIFORM>
-cudaError_t launch_one(const TileGeom& tg, const PushArgs& a, int grid, cudaStream_t st) {
-    const int smem = push_deposit_smem_bytes(tg, NCOMP);
-    push_deposit_kernel<MODE, NCOMP, UNIFORM><<<grid, kPushThreads, smem, st>>>(a, tg);
-    count_launches(1);
-    return cudaGetLastError();
+// Shared memory of the push kernels with private or shared windows.
+int push_smem(const TileGeom& tg, int ncomp, bool priv) {
+    const int records = 16 + tg.wx * tg.wy * kGFStride * 8;
+    const int windows = priv ? kPushWarps * private_window_doubles(tg, 3, 3, ncomp) * 8 + 8
+                             : 2 * ncomp * tg.wx * tg.wy * 8;
+    const int stage = priv ? kPushWarps * (9 + ncomp) * kColStride * 8
+                           : kPushWarps * (32 * (9 + ncomp) * 8 + 32 * 4);
+    const int bytes = windows + stage + records;
+    const int red = kPushWarps * 5 * 8;
+    return bytes > red ? bytes : red;
 }
 
-template <int MODE, int NCOMP, bool UNIFORM>
-cudaError_t set_smem_one(int bytes) {
-    return raise_smem_limit(reinterpret_cast<const void*>(push_deposit_kernel<MODE, NCOMP, UNIFORM>), bytes);
+// Private windows while two CTAs fit an SM, as with the default tile of 8
+// cells (83 KB, 98 KB with the charge); larger windows stay shared.
+bool push_private(const TileGeom& tg, int ncomp) { return push_smem(tg, ncomp, true) <= 113 * 1024; }
+
+using PushKernel = void (*)(PushArgs, TileGeom);
+PushKernel push_kernel(int mode, int ncomp, bool uniform, bool priv) {
+#define UPIC_CASE(MODE, NC)                                                                                        \
+    if (mode == MODE && ncomp == NC)                                                                               \
+        return uniform ? (priv ? push_deposit_kernel<MODE, NC, true, true> : push_deposit_kernel<MODE, NC, true, false>) \
+                       : (priv ? push_deposit_kernel<MODE, NC, false, true> : push_deposit_kernel<MODE, NC, false, false>);
+    UPIC_CASE(kModeDeposit, 1)
+    UPIC_CASE(kModeDeposit, 3)
+    UPIC_CASE(kModeDeposit, 4)
+    UPIC_CASE(kModeAdvanceDeposit, 3)
+    UPIC_CASE(kModeAdvanceDeposit, 4)
+    UPIC_CASE(kModePush, 3)
+    UPIC_CASE(kModePush, 4)
+#undef UPIC_CASE
+    return nullptr;
 }
 
 }  // namespace
@@ -908,42 +980,24 @@ static long g_launches = 0;
 void count_launches(long n) { __atomic_fetch_add(&g_launches, n, __ATOMIC_RELAXED); }
 long launches_total() { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED); }
 
-int push_deposit_smem_bytes(const TileGeom& tg, int ncomp) {
-    const int WN = tg.wx * tg.wy;
-    const int window = 2 * ncomp * WN * 8;
-    const int stage = kPushWarps * (32 * (9 + ncomp) * 8 + 32 * 4);
-    int bytes = window + stage;
-#if UPIC_PUSH_SMEM_GATHER
-    bytes += 16 + WN * kGFStride * 8;
-#endif
-    const int red = kPushWarps * 5 * 8;
-    return bytes > red ? bytes : red;
-}
-
 cudaError_t push_configure_smem(const TileGeom& tg) {
-    cudaError_t e = cudaSuccess;
-#define UPIC_SET(MODE, NC, U)                                                   \
-    e = set_smem_one<MODE, NC, U>(push_deposit_smem_bytes(tg, NC));              \
-    if (e != cudaSuccess) return e;
-    UPIC_SET(kModeDeposit, 1, true) UPIC_SET(kModeDeposit, 1, false)
-    UPIC_SET(kModeDeposit, 3, true) UPIC_SET(kModeDeposit, 3, false)
-    UPIC_SET(kModeDeposit, 4, true) UPIC_SET(kModeDeposit, 4, false)
-    UPIC_SET(kModeAdvanceDeposit, 3, true) UPIC_SET(kModeAdvanceDeposit, 3, false)
-    UPIC_SET(kModeAdvanceDeposit, 4, true) UPIC_SET(kModeAdvanceDeposit, 4, false)
-    UPIC_SET(kModePush, 3, true) UPIC_SET(kModePush, 3, false)
-    UPIC_SET(kModePush, 4, true) UPIC_SET(kModePush, 4, false)
-#undef UPIC_SET
-    return e;
+    for (int mode : {kModeDeposit, kModeAdvanceDeposit, kModePush})
+        for (int nc : {1, 3, 4})
+            for (bool uniform : {true, false}) {
+                const bool priv = push_private(tg, nc);
+                const PushKernel k = push_kernel(mode, nc, uniform, priv);
+                if (!k) continue;
+                const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), push_smem(tg, nc, priv));
+                if (e != cudaSuccess) return e;
+            }
+    return cudaSuccess;
 }
 
 int push_occupancy(const TileGeom& tg, int ncomp) {
     int n = 0;
-    if (ncomp == 4)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, push_deposit_kernel<kModePush, 4, true>, kPushThreads,
-                                                      push_deposit_smem_bytes(tg, 4));
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, push_deposit_kernel<kModePush, 3, true>, kPushThreads,
-                                                      push_deposit_smem_bytes(tg, 3));
+    const bool priv = push_private(tg, ncomp);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, push_kernel(kModePush, ncomp, true, priv), kPushThreads,
+                                                  push_smem(tg, ncomp, priv));
     return n;
 }
 
@@ -1007,19 +1061,12 @@ cudaError_t launch_iaem_push(long np, const double* x, const double* y, double* 
 
 cudaError_t launch_push_deposit(int mode, int ncomp, bool uniform, const TileGeom& tg,
                                 const PushArgs& a, int grid, cudaStream_t st) {
-#define UPIC_CASE(MODE, NC)                                                     \
-    if (mode == MODE && ncomp == NC)                                            \
-        return uniform ? launch_one<MODE, NC, true>(tg, a, grid, st)            \
-                       : launch_one<MODE, NC, false>(tg, a, grid, st);
-    UPIC_CASE(kModeDeposit, 1)
-    UPIC_CASE(kModeDeposit, 3)
-    UPIC_CASE(kModeDeposit, 4)
-    UPIC_CASE(kModeAdvanceDeposit, 3)
-    UPIC_CASE(kModeAdvanceDeposit, 4)
-    UPIC_CASE(kModePush, 3)
-    UPIC_CASE(kModePush, 4)
-#undef UPIC_CASE
-    return cudaErrorInvalidValue;
+    const bool priv = push_private(tg, ncomp);
+    const PushKernel k = push_kernel(mode, ncomp, uniform, priv);
+    if (!k) return cudaErrorInvalidValue;
+    k<<<grid, kPushThreads, push_smem(tg, ncomp, priv), st>>>(a, tg);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_convert_acc(unsigned long long* acc, int N, const double* scale, double* J,

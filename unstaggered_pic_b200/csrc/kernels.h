@@ -200,7 +200,6 @@ cudaError_t launch_push_deposit(int mode, int ncomp, bool uniform_qm, const Tile
 cudaError_t launch_iaem_push(long np, const double* x, const double* y, double* P, double* v, double* vp,
                              const double* q, const double* m, const double* F, int nx, int ny, double inv_dx,
                              double inv_dy, double dt, double c, cudaStream_t st);
-int push_deposit_smem_bytes(const TileGeom& tg, int ncomp);
 cudaError_t push_configure_smem(const TileGeom& tg);
 // Resident CTAs per SM of the step's push kernel (ncomp 3 or 4).
 int push_occupancy(const TileGeom& tg, int ncomp);
