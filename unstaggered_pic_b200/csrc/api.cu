@@ -117,13 +117,18 @@ TileGeom make_tiles(int nx, int ny, int tile, int guard, int lo, int hi) {
 
 int iota(upic_ctx* c, int* id, long n);
 
-int choose_chunk(long np, int grid, int max_chunk) {
+int choose_chunk(long np, int grid, int max_chunk, int unit) {
     long t = (np + grid - 1) / (grid > 0 ? grid : 1);
-    t = (t + kMinChunk - 1) / kMinChunk * kMinChunk;
-    if (t < kMinChunk) t = kMinChunk;
+    t = (t + unit - 1) / unit * unit;
+    if (t < unit) t = unit;
     if (t > max_chunk) t = max_chunk;
     return (int)t;
 }
+
+// Particles per push chunk: the launch's resident CTAs each get one while a
+// 2048-particle chunk would leave some without (16,384 particles: 64 CTAs of
+// one 256-particle round instead of 16 of four).
+int push_chunk(const upic_ctx* c) { return choose_chunk(c->np, c->push_grid, 2048, 256); }
 
 int alloc_soa(upic_ctx* c, ParticleSoA& s, long cap, bool with_state, bool with_qm) {
     int rc = 0;
@@ -185,8 +190,8 @@ int alloc_sortwork(upic_ctx* c, SortWork& w, long cap, const TileGeom& tg) {
     if ((rc = dalloc(c, &w.keys_alt, cap))) return rc;
     if ((rc = dalloc(c, &w.vals, cap))) return rc;
     if ((rc = dalloc(c, &w.vals_alt, cap))) return rc;
-    const long nblocks = (cap + 4095) / 4096;
-    const long hist = 256 * nblocks;
+    // digit histograms of 4096-key blocks, or of 1024-key ones for a small set
+    const long hist = 256 * std::max((cap + 4095) / 4096, (std::min(cap, 148L * 4096) + 1023) / 1024);
     if ((rc = dalloc(c, &w.hist, hist))) return rc;
     const long scan_blocks = (hist + 1023) / 1024 + 16;
     if ((rc = dalloc(c, &w.scan_tmp, scan_blocks))) return rc;
@@ -234,14 +239,6 @@ __global__ void split3_kernel(const double* t, long n, double* a, double* b, dou
     }
 }
 
-__global__ void join3_kernel(double* t, long n, const double* a, const double* b, const double* c) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        t[3 * i] = a[i];
-        t[3 * i + 1] = b[i];
-        t[3 * i + 2] = c[i];
-    }
-}
-
 __global__ void iota_kernel(int* id, long n) {
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
         id[i] = (int)i;
@@ -281,12 +278,26 @@ int upload3(upic_ctx* c, const double* host, long n, double* a, double* b, doubl
     return 0;
 }
 
-int download3(upic_ctx* c, double* host, long n, const double* a, const double* b, const double* d) {
-    join3_kernel<<<gridn(n), 256, 0, c->st>>>(c->d_tmp3, n, a, b, d);
-    count_launches(1);
-    UPIC_CUDA(c, cudaGetLastError());
-    UPIC_CUDA(c, cudaMemcpyAsync(host, c->d_tmp3, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->st));
-    return 0;
+int download_particles(upic_ctx* c, const ParticleSoA& s, long np, int* inv, double* x, double* y, double* P,
+                       double* v, double* v_prev) {
+    if (np == 0) return 0;
+    // the staging buffer is reused in stream order: each gather waits for the
+    // previous copy out of it
+    double* t = c->d_tmp3;
+    UPIC_CUDA(c, invert_order(s.id, np, inv, c->st));
+    if (x || y) {
+        UPIC_CUDA(c, gather_pair(s.x, s.y, inv, np, t, t + np, c->st));
+        if (x) UPIC_CUDA(c, cudaMemcpyAsync(x, t, sizeof(double) * np, cudaMemcpyDeviceToHost, c->st));
+        if (y) UPIC_CUDA(c, cudaMemcpyAsync(y, t + np, sizeof(double) * np, cudaMemcpyDeviceToHost, c->st));
+    }
+    double* const out[3] = {P, v, v_prev};
+    const double* const src[3][3] = {{s.Px, s.Py, s.Pz}, {s.vx, s.vy, s.vz}, {s.wx, s.wy, s.wz}};
+    for (int k = 0; k < 3; ++k) {
+        if (!out[k]) continue;
+        UPIC_CUDA(c, gather_triple(src[k][0], src[k][1], src[k][2], inv, np, t, c->st));
+        UPIC_CUDA(c, cudaMemcpyAsync(out[k], t, sizeof(double) * 3 * np, cudaMemcpyDeviceToHost, c->st));
+    }
+    return sync(c);
 }
 
 #ifndef UPIC_DEVICE_SCAN
@@ -478,7 +489,7 @@ const double2* charge_spectrum(const upic_ctx* c) {
 }
 
 // Diagnostics row of the current spectra (hist slot_new with derivatives
-// against slot_prev0) into c->h_row.
+// against slot_prev0) into `row` (page-locked).
 DiagArgs diag_args(upic_ctx* c, int slot_new, int slot_prev0, int na, const double* acoef) {
     DiagArgs d{};
     d.g = kgrid(c);
@@ -496,7 +507,7 @@ DiagArgs diag_args(upic_ctx* c, int slot_new, int slot_prev0, int na, const doub
     d.dA = c->dA;
     return d;
 }
-int run_diag(upic_ctx* c, int slot_new, int slot_prev0, int na, const double* acoef) {
+int run_diag(upic_ctx* c, int slot_new, int slot_prev0, int na, const double* acoef, double* row) {
     DiagArgs d = diag_args(c, slot_new, slot_prev0, na, acoef);
     d.partials = c->d_partials;
     d.max_blocks = kRedGrid;
@@ -504,7 +515,7 @@ int run_diag(upic_ctx* c, int slot_new, int slot_prev0, int na, const double* ac
     d.pdiag = c->d_pdiag;
     d.pcount = c->push_grid;
     d.np = c->np;
-    d.row = c->h_row;
+    d.row = row;
     UPIC_CUDA(c, launch_diag_reduce(d, c->st));
     return 0;
 }
@@ -790,7 +801,7 @@ int upic_create(const upic_config* cfg, upic_ctx** out) {
         (rc = dalloc(c, &c->d_done, 1)) || (rc = dalloc(c, &c->d_scan, 3)) ||
         (c->mixed && (rc = dalloc(c, &c->d_gf32, (size_t)kGFStride * N))))
         return bail(rc);
-    if (cudaMallocHost(&c->h_row, sizeof(double) * UPIC_DIAG_COUNT) != cudaSuccess ||
+    if (cudaMallocHost(&c->h_row, sizeof(double) * UPIC_DIAG_COUNT * kRowRing) != cudaSuccess ||
         cudaMallocHost(&c->h_scan, 3 * sizeof(unsigned long long)) != cudaSuccess)
         return bail(fail(c, UPIC_ERR_NOMEM, "cudaMallocHost failed"));
     std::vector<double> kx(N), ky(N), k2(N);
@@ -923,6 +934,7 @@ int explicit_state_io(upic_ctx* c, StateIO& io) {
         if (has_bg && !c->d_bg && (rc = dalloc(c, &c->d_bg, c->N))) return rc;
         c->cur = 0;
         c->np = np;
+        c->tg.chunk = push_chunk(c);
         c->uniform_qm = uniform != 0;
         c->fields_ready = ready != 0;
     }
@@ -1096,6 +1108,7 @@ static int set_particles_mixed(upic_ctx* c, long np, const double* x, const doub
             if ((rc = dalloc(c, &c->M[k].q, c->cap + 2)) || (rc = dalloc(c, &c->M[k].m, c->cap + 2))) return rc;
     }
     c->np = np;
+    c->tg.chunk = push_chunk(c);
     c->cur = 0;
     c->uniform_qm = uniform;
     c->q0 = np ? q[0] : 0.0;
@@ -1118,11 +1131,11 @@ static int set_particles_mixed(upic_ctx* c, long np, const double* x, const doub
 
 static int get_particles_mixed(upic_ctx* c, long np, double* x, double* y, double* P, double* v, double* v_prev) {
     if (np == 0) return UPIC_OK;
-    MixedSoA& s = c->M[c->cur];
-    MixedSoA& d = c->M[1 - c->cur];
-    UPIC_CUDA(c, unpermute_mixed(s, d, np, c->st));
+    MixedSoA& d = c->M[c->cur];
+    int* inv = c->sw.vals_alt;  // free between sorts
+    UPIC_CUDA(c, invert_order(d.id, np, inv, c->st));
     double* t = c->d_tmp3;
-    UPIC_CUDA(c, mixed_to_positions(np, d.cell, d.rx, d.ry, c->dx, c->dy, c->cfg.Lx, c->cfg.Ly, c->lny, c->ny, t,
+    UPIC_CUDA(c, mixed_to_positions(np, inv, d.cell, d.rx, d.ry, c->dx, c->dy, c->cfg.Lx, c->cfg.Ly, c->lny, c->ny, t,
                                     t + np, c->st));
     if (x) UPIC_CUDA(c, cudaMemcpyAsync(x, t, sizeof(double) * np, cudaMemcpyDeviceToHost, c->st));
     if (y) UPIC_CUDA(c, cudaMemcpyAsync(y, t + np, sizeof(double) * np, cudaMemcpyDeviceToHost, c->st));
@@ -1131,7 +1144,7 @@ static int get_particles_mixed(upic_ctx* c, long np, double* x, double* y, doubl
     for (int k = 0; k < 3; ++k) {
         if (!out[k]) continue;
         // the staging buffer is reused in stream order
-        UPIC_CUDA(c, mixed_join3(np, src[k][0], src[k][1], src[k][2], t, c->st));
+        UPIC_CUDA(c, mixed_join3(np, inv, src[k][0], src[k][1], src[k][2], t, c->st));
         UPIC_CUDA(c, cudaMemcpyAsync(out[k], t, sizeof(double) * 3 * np, cudaMemcpyDeviceToHost, c->st));
     }
     return sync(c);
@@ -1207,6 +1220,7 @@ int upic_set_particles(upic_ctx* c, long np, const double* x, const double* y, c
             if ((rc = dalloc(c, &c->P[k].q, c->cap + 2)) || (rc = dalloc(c, &c->P[k].m, c->cap + 2))) return rc;
     }
     c->np = np;
+    c->tg.chunk = push_chunk(c);
     c->cur = 0;
     c->uniform_qm = uniform;
     c->q0 = np ? q[0] : 0.0;
@@ -1233,19 +1247,7 @@ int upic_get_particles(upic_ctx* c, long np, double* x, double* y, double* P, do
     if (np != c->np) return fail(c, UPIC_ERR_ARGUMENT, "particle count does not match the context");
     if (c->imp) return implicit_get_particles(c, np, x, y, P, v, v_prev);
     if (c->mixed) return get_particles_mixed(c, np, x, y, P, v, v_prev);
-    if (np == 0) return UPIC_OK;
-    ParticleSoA& s = c->P[c->cur];
-    ParticleSoA& d = c->P[1 - c->cur];
-    UPIC_CUDA(c, unpermute_particles(s, d, np, c->st));
-    int rc;
-    if (x) UPIC_CUDA(c, cudaMemcpyAsync(x, d.x, sizeof(double) * np, cudaMemcpyDeviceToHost, c->st));
-    if (y) UPIC_CUDA(c, cudaMemcpyAsync(y, d.y, sizeof(double) * np, cudaMemcpyDeviceToHost, c->st));
-    // the staging buffer is reused in stream order: each join waits for the
-    // previous copy out of it
-    if (P && (rc = download3(c, P, np, d.Px, d.Py, d.Pz))) return rc;
-    if (v && (rc = download3(c, v, np, d.vx, d.vy, d.vz))) return rc;
-    if (v_prev && (rc = download3(c, v_prev, np, d.wx, d.wy, d.wz))) return rc;
-    return sync(c);
+    return download_particles(c, c->P[c->cur], np, c->sw.vals_alt, x, y, P, v, v_prev);
 }
 
 int upic_init_fields(upic_ctx* c, double* diag_row) {
@@ -1286,7 +1288,7 @@ int upic_init_fields(upic_ctx* c, double* diag_row) {
     UPIC_CUDA(c, fft2d_mapped(c->plan, sp, jn, jmap, 0, c->st, c->d_J, 0, nullptr, 0, 0));
     if (diag_row) {
         const double a1[3] = {1.0, -1.0, 0.0};
-        if ((rc = run_diag(c, c->head, c->head, 2, a1))) return rc;
+        if ((rc = run_diag(c, c->head, c->head, 2, a1, c->h_row))) return rc;
     }
     // first step's current, deposited one step ahead (:1137-1141)
     if (c->np > 0) {
@@ -1325,6 +1327,19 @@ int explicit_advance(upic_ctx* c, int nsteps, int diag_stride, double* diag, boo
     const bool naive = c->cfg.charge_update == UPIC_CHARGE_NAIVE;
     double2* sp = c->d_spec;
     int rc;
+    // Rows collect in the page-locked ring and are handed over when it is full
+    // and at the end: waiting for each row left the GPU idle for 35 of a 120 us
+    // step (32 x 32, a row every step).
+    int pending = 0, row_step[kRowRing];
+    auto hand_over = [&]() -> int {
+        if (pending == 0) return 0;
+        const int r = sync(c);
+        for (int i = 0; i < pending && r == 0; ++i)
+            std::memcpy(diag + (size_t)row_step[i] * UPIC_DIAG_COUNT, c->h_row + (size_t)i * UPIC_DIAG_COUNT,
+                        sizeof(double) * UPIC_DIAG_COUNT);
+        pending = 0;
+        return r;
+    };
     for (int s = 0; s < nsteps; ++s) {
         const long step = c->steps + 1;
         const bool want_diag = diag && diag_stride > 0 && (step % diag_stride == 0 || s == nsteps - 1);
@@ -1363,9 +1378,9 @@ int explicit_advance(upic_ctx* c, int nsteps, int diag_stride, double* diag, boo
         }
         const int snew = (c->head + kHistSlots - 1) % kHistSlots;
         if (want_diag) {
-            if ((rc = run_diag(c, snew, c->head, na, a))) return rc;
-            if ((rc = sync(c))) return rc;
-            std::memcpy(diag + (size_t)s * UPIC_DIAG_COUNT, c->h_row, sizeof(double) * UPIC_DIAG_COUNT);
+            if ((rc = run_diag(c, snew, c->head, na, a, c->h_row + (size_t)pending * UPIC_DIAG_COUNT))) return rc;
+            row_step[pending++] = s;
+            if (pending == kRowRing && (rc = hand_over())) return rc;
         } else if (diag) {
             for (int i = 0; i < UPIC_DIAG_COUNT; ++i) diag[(size_t)s * UPIC_DIAG_COUNT + i] = NAN;
         }
@@ -1373,6 +1388,7 @@ int explicit_advance(upic_ctx* c, int nsteps, int diag_stride, double* diag, boo
         c->steps = step;
         c->steps_since_sort++;
     }
+    if ((rc = hand_over())) return rc;
     return final_sync ? sync(c) : 0;
 }
 

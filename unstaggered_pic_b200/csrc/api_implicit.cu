@@ -1665,19 +1665,7 @@ int implicit_state_io(upic_ctx* c, StateIO& io) {
 int implicit_get_particles(upic_ctx* c, long np, double* x, double* y, double* P, double* v, double* v_prev) {
     ImplicitState& s = *c->imp;
     if (np != s.np) return fail(c, UPIC_ERR_ARGUMENT, "particle count does not match the context");
-    if (np == 0) return UPIC_OK;
-    ParticleSoA src = s.P[s.cur];
-    ParticleSoA dst = s.P[1 - s.cur];
-    UPIC_CUDA(c, unpermute_particles(src, dst, np, c->st));
-    int rc;
-    if (x) UPIC_CUDA(c, cudaMemcpyAsync(x, dst.x, sizeof(double) * np, cudaMemcpyDeviceToHost, c->st));
-    if (y) UPIC_CUDA(c, cudaMemcpyAsync(y, dst.y, sizeof(double) * np, cudaMemcpyDeviceToHost, c->st));
-    if (P && (rc = download3(c, P, np, dst.Px, dst.Py, dst.Pz))) return rc;
-    if ((rc = sync(c))) return rc;
-    if (v && (rc = download3(c, v, np, dst.vx, dst.vy, dst.vz))) return rc;
-    if ((rc = sync(c))) return rc;
-    if (v_prev && (rc = download3(c, v_prev, np, dst.wx, dst.wy, dst.wz))) return rc;
-    return sync(c);
+    return download_particles(c, s.P[s.cur], np, s.sw.vals_alt, x, y, P, v, v_prev);
 }
 
 int implicit_init_fields(upic_ctx* c, double* diag_row) {

@@ -18,6 +18,7 @@ namespace upic_host {
 constexpr int kHistSlots = 5;
 constexpr int kDiagFields = 10;
 constexpr int kRedGrid = 148 * 2;
+constexpr int kRowRing = 64;  // diagnostics rows a step call keeps before it hands them over
 
 struct ImplicitState;  // api_implicit.cu
 
@@ -76,7 +77,7 @@ struct upic_ctx {
     double* d_pdiag = nullptr;
     unsigned* d_done = nullptr;  // finished blocks of the diagnostics reduction (zero between launches)
     double* d_bg = nullptr;   // fixed background charge (upic_set_background) or null: uniform n0
-    double* h_row = nullptr;  // pinned; the diagnostics reduction writes it
+    double* h_row = nullptr;  // pinned, kRowRing rows; the diagnostics reduction writes them
     // particle-state scan of upic_set_particles (non-finite count, largest
     // speed and velocity component bits): device words and their pinned copy
     unsigned long long* d_scan = nullptr;
@@ -135,7 +136,10 @@ void dfree(upic_ctx* c, void* p);
 int sync(upic_ctx* c);
 int gridn(long n);
 int upload3(upic_ctx* c, const double* host, long n, double* a, double* b, double* d);
-int download3(upic_ctx* c, double* host, long n, const double* a, const double* b, const double* d);
+// The particle set in the caller's order to host arrays (any may be null);
+// inv: np ints of scratch (a sort's spare buffer).
+int download_particles(upic_ctx* c, const ParticleSoA& s, long np, int* inv, double* x, double* y, double* P,
+                       double* v, double* v_prev);
 int ensure_tmp3(upic_ctx* c, long n);
 // Validation scan of a host particle set (positions x, y; velocities v as
 // xyz triples; q, m): finiteness, uniform q/m, sum |q|, largest speed and
@@ -168,15 +172,12 @@ HostScan scan_particles(long np, const double* x, const double* y, const double*
                         const double* m);
 double fixed_scale(double bound);
 TileGeom make_tiles(int nx, int ny, int tile, int guard, int lo, int hi);
-// Particles per deposit chunk of the implicit map kernel: enough chunks for
-// every resident CTA of a `grid`-CTA launch (a small particle set would
-// otherwise keep most SMs idle behind a few long per-particle solves), a
-// multiple of kMinChunk in [kMinChunk, max_chunk].  The explicit push keeps
-// 2048-particle chunks: its per-particle work is short, and many small
-// explicit runs are better served by an ensemble.  Chunk tables are
-// allocated for kMinChunk.
+// Particles per deposit chunk: enough chunks for every resident CTA of a
+// `grid`-CTA launch (a small particle set would otherwise keep most SMs idle
+// behind a few long chunks), a multiple of `unit` up to max_chunk.  Chunk
+// tables are allocated for kMinChunk.
 constexpr int kMinChunk = 128;
-int choose_chunk(long np, int grid, int max_chunk);
+int choose_chunk(long np, int grid, int max_chunk, int unit = kMinChunk);
 int alloc_soa(upic_ctx* c, ParticleSoA& s, long cap, bool with_state, bool with_qm);
 void free_soa(upic_ctx* c, ParticleSoA& s);
 int alloc_sortwork(upic_ctx* c, SortWork& w, long cap, const TileGeom& tg);

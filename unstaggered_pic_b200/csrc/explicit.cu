@@ -248,11 +248,15 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                                 const double w = wxs[ia] * wys[ib];
                                 const double2* rec = srec + (wxi * tg.wy + wyi) * (kGFStride / 2);
 #pragma unroll
-                                for (int f2 = 0; f2 < kGFStride / 2; ++f2) {
+                                for (int f2 = 0; f2 < kGF / 2; ++f2) {
                                     const double2 r = rec[f2];
                                     G[2 * f2] = fma(r.x, w, G[2 * f2]);
                                     G[2 * f2 + 1] = fma(r.y, w, G[2 * f2 + 1]);
                                 }
+                                // the last field alone: the record's padding would
+                                // take its share of the shared-memory return path,
+                                // which bounds this kernel (75% busy)
+                                G[kGF - 1] = fma(reinterpret_cast<const double*>(rec)[kGF - 1], w, G[kGF - 1]);
                             }
                         }
                     } else

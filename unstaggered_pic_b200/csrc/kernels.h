@@ -127,9 +127,13 @@ cudaError_t sort_particles_by_tile(const TileGeom& tg, const ParticleSoA& p, lon
 // Gather every non-null array of src by w.vals (the sorted order) into dst.
 cudaError_t permute_particles(const ParticleSoA& src, const ParticleSoA& dst, long np,
                               const SortWork& w, cudaStream_t st);
-// dst[id[k]] = src[k] for the arrays x..wz (restores the caller's order).
-cudaError_t unpermute_particles(const ParticleSoA& src, const ParticleSoA& dst, long np,
-                                cudaStream_t st);
+// The caller's order: inv[id[k]] = k, and arrays gathered through it, two side
+// by side or three as triples.
+cudaError_t invert_order(const int* id, long np, int* inv, cudaStream_t st);
+cudaError_t gather_pair(const double* a, const double* b, const int* inv, long np, double* oa, double* ob,
+                        cudaStream_t st);
+cudaError_t gather_triple(const double* a, const double* b, const double* c, const int* inv, long np, double* out,
+                          cudaStream_t st);
 // The buffer a key kernel writes the unsorted cell keys into (the radix
 // passes alternate between two buffers and end in w.keys).
 unsigned* sort_key_input(const TileGeom& tg, SortWork& w);
@@ -165,11 +169,11 @@ cudaError_t mixed_from_positions(long np, const double* x, const double* y, doub
                                  int ny, int lny, int* cell, float* rx, float* ry, cudaStream_t st);
 cudaError_t mixed_split3(long np, const double* aos, float* a, float* b, float* c, cudaStream_t st);
 cudaError_t mixed_from_doubles(long np, const double* src, float* dst, cudaStream_t st);
-// Mixed (sorted order) -> caller order in dst, then positions / triples as doubles.
-cudaError_t unpermute_mixed(const MixedSoA& src, const MixedSoA& dst, long np, cudaStream_t st);
-cudaError_t mixed_to_positions(long np, const int* cell, const float* rx, const float* ry, double dx, double dy,
-                               double Lx, double Ly, int lny, int ny, double* x, double* y, cudaStream_t st);
-cudaError_t mixed_join3(long np, const float* a, const float* b, const float* c, double* aos, cudaStream_t st);
+// Mixed (sorted order) -> positions / triples as doubles in the caller's order (inv: invert_order).
+cudaError_t mixed_to_positions(long np, const int* inv, const int* cell, const float* rx, const float* ry, double dx,
+                               double dy, double Lx, double Ly, int lny, int ny, double* x, double* y, cudaStream_t st);
+cudaError_t mixed_join3(long np, const int* inv, const float* a, const float* b, const float* c, double* aos,
+                        cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // Explicit BDF/IAEM step (explicit.cu)

@@ -420,27 +420,6 @@ __global__ void mgather_kernel(const T* __restrict__ src, T* __restrict__ dst, c
         dst[q] = src[idx[q]];
 }
 
-__global__ void unpermute_mixed_kernel(MixedSoA s, MixedSoA d, long n) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-        const int o = s.id[k];
-        const int cell = s.cell[k];
-        const float v[11] = {s.rx[k], s.ry[k], s.Px[k], s.Py[k], s.Pz[k], s.vx[k],
-                             s.vy[k], s.vz[k], s.wx[k], s.wy[k], s.wz[k]};
-        d.cell[o] = cell;
-        d.rx[o] = v[0];
-        d.ry[o] = v[1];
-        d.Px[o] = v[2];
-        d.Py[o] = v[3];
-        d.Pz[o] = v[4];
-        d.vx[o] = v[5];
-        d.vy[o] = v[6];
-        d.vz[o] = v[7];
-        d.wx[o] = v[8];
-        d.wy[o] = v[9];
-        d.wz[o] = v[10];
-    }
-}
-
 // Nearest node and offset of x in [0, L) (quadratic_weights' s = x/dx,
 // ic = floor(s + 1/2), r = s - ic), the offset rounded once to FP32.
 __global__ void from_positions_kernel(long np, const double* x, const double* y, double inv_dx, double inv_dy,
@@ -456,12 +435,14 @@ __global__ void from_positions_kernel(long np, const double* x, const double* y,
 }
 
 // Position in [0, L) of node ix plus offset r.
-__global__ void to_positions_kernel(long np, const int* cell, const float* rx, const float* ry, double dx,
-                                    double dy, double Lx, double Ly, int lny, int ny, double* x, double* y) {
+__global__ void to_positions_kernel(long np, const int* inv, const int* cell, const float* rx, const float* ry,
+                                    double dx, double dy, double Lx, double Ly, int lny, int ny, double* x,
+                                    double* y) {
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < np; q += (long)gridDim.x * blockDim.x) {
-        const int c = cell[q];
-        double xv = ((double)(c >> lny) + (double)rx[q]) * dx;
-        double yv = ((double)(c & (ny - 1)) + (double)ry[q]) * dy;
+        const int k = inv[q];
+        const int c = cell[k];
+        double xv = ((double)(c >> lny) + (double)rx[k]) * dx;
+        double yv = ((double)(c & (ny - 1)) + (double)ry[k]) * dy;
         if (xv < 0.0) xv += Lx;
         if (xv >= Lx) xv -= Lx;
         if (yv < 0.0) yv += Ly;
@@ -479,11 +460,12 @@ __global__ void split3f_kernel(long n, const double* aos, float* a, float* b, fl
     }
 }
 
-__global__ void join3f_kernel(long n, const float* a, const float* b, const float* c, double* aos) {
+__global__ void join3f_kernel(long n, const int* inv, const float* a, const float* b, const float* c, double* aos) {
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-        aos[3 * q] = a[q];
-        aos[3 * q + 1] = b[q];
-        aos[3 * q + 2] = c[q];
+        const int k = inv[q];
+        aos[3 * q] = a[k];
+        aos[3 * q + 1] = b[k];
+        aos[3 * q + 2] = c[k];
     }
 }
 
@@ -648,12 +630,6 @@ cudaError_t permute_mixed(const MixedSoA& s, const MixedSoA& d, long np, const S
     return cudaGetLastError();
 }
 
-cudaError_t unpermute_mixed(const MixedSoA& s, const MixedSoA& d, long np, cudaStream_t st) {
-    unpermute_mixed_kernel<<<mgrid(np), 256, 0, st>>>(s, d, np);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
 cudaError_t mixed_from_positions(long np, const double* x, const double* y, double inv_dx, double inv_dy, int nx,
                                  int ny, int lny, int* cell, float* rx, float* ry, cudaStream_t st) {
     from_positions_kernel<<<mgrid(np), 256, 0, st>>>(np, x, y, inv_dx, inv_dy, nx, ny, lny, cell, rx, ry);
@@ -661,9 +637,10 @@ cudaError_t mixed_from_positions(long np, const double* x, const double* y, doub
     return cudaGetLastError();
 }
 
-cudaError_t mixed_to_positions(long np, const int* cell, const float* rx, const float* ry, double dx, double dy,
-                               double Lx, double Ly, int lny, int ny, double* x, double* y, cudaStream_t st) {
-    to_positions_kernel<<<mgrid(np), 256, 0, st>>>(np, cell, rx, ry, dx, dy, Lx, Ly, lny, ny, x, y);
+cudaError_t mixed_to_positions(long np, const int* inv, const int* cell, const float* rx, const float* ry, double dx,
+                               double dy, double Lx, double Ly, int lny, int ny, double* x, double* y,
+                               cudaStream_t st) {
+    to_positions_kernel<<<mgrid(np), 256, 0, st>>>(np, inv, cell, rx, ry, dx, dy, Lx, Ly, lny, ny, x, y);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -674,8 +651,9 @@ cudaError_t mixed_split3(long np, const double* aos, float* a, float* b, float* 
     return cudaGetLastError();
 }
 
-cudaError_t mixed_join3(long np, const float* a, const float* b, const float* c, double* aos, cudaStream_t st) {
-    join3f_kernel<<<mgrid(np), 256, 0, st>>>(np, a, b, c, aos);
+cudaError_t mixed_join3(long np, const int* inv, const float* a, const float* b, const float* c, double* aos,
+                        cudaStream_t st) {
+    join3f_kernel<<<mgrid(np), 256, 0, st>>>(np, inv, a, b, c, aos);
     count_launches(1);
     return cudaGetLastError();
 }

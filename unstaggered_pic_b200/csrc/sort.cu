@@ -24,14 +24,19 @@ namespace upic {
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // elements per block
+// Keys per thread of a radix pass: 16 (4096-key blocks) for sets that fill the
+// GPU with such blocks, 4 below: a 16,384-particle pass then runs 16 blocks of
+// four rounds instead of four blocks of sixteen (scatter 16.3 -> 5.6 us).
+constexpr int kSortItems = 16, kSortItemsSmall = 4;
+constexpr long kSortSmall = 148L * kSortThreads * kSortItems;
+constexpr int sort_tile(int items) { return kSortThreads * items; }  // elements per block
 constexpr int kSortWarps = kSortThreads / kWarp;
 constexpr int kMaxDigits = 256;                       // 8-bit digits at most
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
+template <bool CLASSES>
 __global__ void make_keys_kernel(TileGeom tg, ParticleSoA p, long np, double Lx, double Ly,
                                  double inv_dx, double inv_dy, double shift, unsigned* keys) {
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < np; q += (long)gridDim.x * blockDim.x) {
@@ -45,7 +50,7 @@ __global__ void make_keys_kernel(TileGeom tg, ParticleSoA p, long np, double Lx,
         const int tx = icx / tg.tile_x, lx = icx - tx * tg.tile_x;
         const int ty = icy / tg.tile_y, ly = icy - ty * tg.tile_y;
         unsigned tile = (unsigned)(tx * tg.nty + ty);
-        if (tg.classes > 1) {
+        if (CLASSES) {
             const double ux = (x + tg.key_origin_x) * inv_dx - tg.class_off;
             const double uy = (y + tg.key_origin_y) * inv_dy - tg.class_off;
             const double n = fabs(floor(ux + tg.class_dt * p.vx[q] * inv_dx) - floor(ux)) +
@@ -57,10 +62,11 @@ __global__ void make_keys_kernel(TileGeom tg, ParticleSoA p, long np, double Lx,
     }
 }
 
-// Digit histogram of one block's kSortTile keys.  Each warp reads its
-// kSortItems * 32 keys ahead of counting and adds one shared atomic per
+// Digit histogram of one block's keys.  Each warp reads its
+// ITEMS * 32 keys ahead of counting and adds one shared atomic per
 // distinct digit of each 32 (match/popc): the keys of a re-sort are nearly
 // sorted already, so most rounds cost one atomic instead of 32 on one word.
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads)
 radix_hist_kernel(const unsigned* __restrict__ keys, long n, int shift, int digits, int nblocks,
                   int* hist) {
@@ -70,15 +76,15 @@ radix_hist_kernel(const unsigned* __restrict__ keys, long n, int shift, int digi
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const unsigned mask = (unsigned)digits - 1u;
-    const long wbase = (long)blockIdx.x * kSortTile + (long)warp * (kSortItems * kWarp) + lane;
-    unsigned key[kSortItems];
+    const long wbase = (long)blockIdx.x * sort_tile(ITEMS) + (long)warp * (ITEMS * kWarp) + lane;
+    unsigned key[ITEMS];
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const long e = wbase + r * kWarp;
         key[r] = e < n ? keys[e] : 0u;
     }
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const bool valid = wbase + r * kWarp < n;
         const int d = valid ? (int)((key[r] >> shift) & mask) : digits;
         const unsigned peers = __match_any_sync(0xffffffffu, d);
@@ -94,7 +100,7 @@ radix_hist_kernel(const unsigned* __restrict__ keys, long n, int shift, int digi
 // (match/popc); offs holds the scanned histograms (digit-major).  IDENT: the
 // values are the source indices (the first pass of a sort, so the key kernel
 // writes no values).
-template <bool IDENT>
+template <int ITEMS, bool IDENT>
 __global__ void __launch_bounds__(kSortThreads)
 radix_scatter_kernel(const unsigned* __restrict__ keys, const int* __restrict__ vals, long n, int shift,
                      int digits, int nblocks, const int* __restrict__ offs, unsigned* __restrict__ okeys,
@@ -109,8 +115,8 @@ radix_scatter_kernel(const unsigned* __restrict__ keys, const int* __restrict__ 
     }
     const unsigned mask = (unsigned)digits - 1u;
     const unsigned lt = (1u << lane) - 1u;
-    const long base = (long)blockIdx.x * kSortTile;
-    for (int r = 0; r < kSortItems; ++r) {
+    const long base = (long)blockIdx.x * sort_tile(ITEMS);
+    for (int r = 0; r < ITEMS; ++r) {
         for (int k = threadIdx.x; k < kSortWarps * kMaxDigits; k += blockDim.x) (&wcnt[0][0])[k] = 0;
         __syncthreads();
         const long e = base + r * kSortThreads + threadIdx.x;
@@ -204,7 +210,62 @@ __global__ void scan_add_kernel(int* out, long n, const int* sums) {
     if (i < n) out[i] += sums[i / kScanTile];
 }
 
+// Exclusive scan by one block, kScanOneItems values per thread at a time.
+constexpr int kScanOneThreads = 1024, kScanOneItems = 8;
+constexpr long kScanOne = 4096;
+__device__ int scan_one_block(const int* in, int* out, int n) {
+    __shared__ int ws[kScanOneThreads / kWarp];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < n; base += kScanOneThreads * kScanOneItems) {
+        const int at = base + threadIdx.x * kScanOneItems;
+        int v[kScanOneItems], s = 0;
+#pragma unroll
+        for (int k = 0; k < kScanOneItems; ++k) {
+            v[k] = at + k < n ? in[at + k] : 0;
+            s += v[k];
+        }
+        int x = s;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            int t = ws[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, t, o);
+                if (lane >= o) t += y;
+            }
+            ws[lane] = t;
+        }
+        __syncthreads();
+        int ex = carry + x - s + (warp > 0 ? ws[warp - 1] : 0);
+#pragma unroll
+        for (int k = 0; k < kScanOneItems; ++k) {
+            if (at + k < n) out[at + k] = ex;
+            ex += v[k];
+        }
+        carry += ws[kScanOneThreads / kWarp - 1];
+        __syncthreads();
+    }
+    return carry;
+}
+
+__global__ void __launch_bounds__(kScanOneThreads) scan_one_kernel(const int* in, int* out, int n) {
+    scan_one_block(in, out, n);
+}
+
+// Up to kScanOne values one block scans them in one launch (2.3 us at 512
+// values, 12.8 us at 16,384); more take the three launches of blocks, block
+// sums and their addition (5.4 us).
 cudaError_t exclusive_scan(const int* in, int* out, long n, int* tmp, int* grand, cudaStream_t st) {
+    if (n <= kScanOne && !grand) {
+        scan_one_kernel<<<1, kScanOneThreads, 0, st>>>(in, out, (int)n);
+        count_launches(1);
+        return cudaGetLastError();
+    }
     const int nb = (int)((n + kScanTile - 1) / kScanTile);
     scan_blocks_kernel<<<nb, kScanThreads, 0, st>>>(in, out, n, tmp);
     scan_sums_kernel<<<1, kScanThreads, 0, st>>>(tmp, nb, grand);
@@ -251,11 +312,23 @@ __global__ void fill_chunks_kernel(const int* cnt, const int* tstart, const int*
     }
 }
 
-template <typename T>
-__global__ void gather_array_kernel(const T* __restrict__ src, T* __restrict__ dst, const int* idx,
-                                    long n) {
-    for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x)
-        dst[q] = src[idx[q]];
+// The chunk table of up to kTilesOne tiles in one launch of one block (counts,
+// chunks per tile, their scan and the table): six launches of 9 us otherwise,
+// against 3.3 us at 16 tiles and 37 us at 4096.
+constexpr int kTilesOne = 512;
+__global__ void __launch_bounds__(kScanOneThreads)
+chunk_table_kernel(const int* tstart, int ntiles, int chunk, int* nch, int* nchunks, Chunk* chunks) {
+    for (int t = threadIdx.x; t < ntiles; t += blockDim.x) nch[t] = (tstart[t + 1] - tstart[t] + chunk - 1) / chunk;
+    __syncthreads();
+    const int total = scan_one_block(nch, nch, ntiles);
+    if (threadIdx.x == 0) *nchunks = total;
+    // warps take the tiles, lanes a tile's chunks
+    const int lane = threadIdx.x & 31;
+    for (int t = threadIdx.x >> 5; t < ntiles; t += kScanOneThreads / kWarp) {
+        const int s = tstart[t], c = tstart[t + 1] - s, o = nch[t];
+        for (int k = lane; k * chunk < c; k += kWarp)
+            chunks[o + k] = Chunk{s + k * chunk, s + min((k + 1) * chunk, c), t};
+    }
 }
 
 // All payload arrays of the particle set gathered by one pass over the
@@ -283,25 +356,67 @@ __global__ void gather_set_kernel(GatherSet g, const int* __restrict__ idx, long
     }
 }
 
-// All of a particle's values are loaded before the scattered stores (the
-// arrays may alias as far as the compiler knows, so a load placed after a
-// store stays after it).
-__global__ void unpermute_kernel(ParticleSoA s, ParticleSoA d, long n) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-        const int o = s.id[k];
-        const double v[11] = {s.x[k],  s.y[k],  s.Px[k], s.Py[k], s.Pz[k], s.vx[k],
-                              s.vy[k], s.vz[k], s.wx[k], s.wy[k], s.wz[k]};
-        d.x[o] = v[0];
-        d.y[o] = v[1];
-        d.Px[o] = v[2];
-        d.Py[o] = v[3];
-        d.Pz[o] = v[4];
-        d.vx[o] = v[5];
-        d.vy[o] = v[6];
-        d.vz[o] = v[7];
-        d.wx[o] = v[8];
-        d.wy[o] = v[9];
-        d.wz[o] = v[10];
+// ---- caller's order ---------------------------------------------------------
+// The read-back gathers each array through the inverse order, so its writes
+// are whole lines and its reads, within a few cells of each other, share
+// sectors in L2.  Scattering eleven arrays of 16.8M particles by id took 7.3
+// ms and the joins into triples 0.7 ms more; the inverse and the gathers
+// straight into triples take 1.5 ms together.
+__global__ void invert_kernel(const int* __restrict__ id, long n, int* __restrict__ inv) {
+    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
+        inv[id[k]] = (int)k;
+}
+
+// Four particles per thread and round, their loads ahead of the stores.
+constexpr int kBackItems = 4;
+
+__global__ void gather_pair_kernel(const double* __restrict__ a, const double* __restrict__ b,
+                                   const int* __restrict__ inv, long n, double* __restrict__ oa,
+                                   double* __restrict__ ob) {
+    const long step = (long)gridDim.x * blockDim.x;
+    for (long o0 = blockIdx.x * (long)blockDim.x + threadIdx.x; o0 < n; o0 += kBackItems * step) {
+        int k[kBackItems];
+        double v[kBackItems][2];
+#pragma unroll
+        for (int i = 0; i < kBackItems; ++i) k[i] = o0 + i * step < n ? inv[o0 + i * step] : 0;
+#pragma unroll
+        for (int i = 0; i < kBackItems; ++i) {
+            v[i][0] = a[k[i]];
+            v[i][1] = b[k[i]];
+        }
+#pragma unroll
+        for (int i = 0; i < kBackItems; ++i) {
+            const long o = o0 + i * step;
+            if (o >= n) break;
+            oa[o] = v[i][0];
+            ob[o] = v[i][1];
+        }
+    }
+}
+
+__global__ void gather_triple_kernel(const double* __restrict__ a, const double* __restrict__ b,
+                                     const double* __restrict__ c, const int* __restrict__ inv, long n,
+                                     double* __restrict__ out) {
+    const long step = (long)gridDim.x * blockDim.x;
+    for (long o0 = blockIdx.x * (long)blockDim.x + threadIdx.x; o0 < n; o0 += kBackItems * step) {
+        int k[kBackItems];
+        double v[kBackItems][3];
+#pragma unroll
+        for (int i = 0; i < kBackItems; ++i) k[i] = o0 + i * step < n ? inv[o0 + i * step] : 0;
+#pragma unroll
+        for (int i = 0; i < kBackItems; ++i) {
+            v[i][0] = a[k[i]];
+            v[i][1] = b[k[i]];
+            v[i][2] = c[k[i]];
+        }
+#pragma unroll
+        for (int i = 0; i < kBackItems; ++i) {
+            const long o = o0 + i * step;
+            if (o >= n) break;
+            out[3 * o] = v[i][0];
+            out[3 * o + 1] = v[i][1];
+            out[3 * o + 2] = v[i][2];
+        }
     }
 }
 
@@ -337,8 +452,8 @@ cudaError_t sort_particles_by_tile(const TileGeom& tg, const ParticleSoA& p, lon
         return cudaGetLastError();
     }
     const double inv_dx = (double)tg.nx / Lx, inv_dy = (double)tg.ny / Ly;
-    make_keys_kernel<<<grid_for(np), 256, 0, st>>>(tg, p, np, Lx, Ly, inv_dx, inv_dy, shift,
-                                                   sort_key_input(tg, w));
+    auto make_keys = tg.classes > 1 ? make_keys_kernel<true> : make_keys_kernel<false>;
+    make_keys<<<grid_for(np), 256, 0, st>>>(tg, p, np, Lx, Ly, inv_dx, inv_dy, shift, sort_key_input(tg, w));
     count_launches(1);
     return sort_keys_to_chunks(tg, np, w, st);
 }
@@ -351,7 +466,9 @@ cudaError_t sort_keys_to_chunks(const TileGeom& tg, long np, SortWork& w, cudaSt
     int dbits;
     const int passes = radix_passes(tg, &dbits);
     const int digits = 1 << dbits;
-    const int nblocks = (int)((np + kSortTile - 1) / kSortTile);
+    const bool small = np < kSortSmall;
+    const int tile = sort_tile(small ? kSortItemsSmall : kSortItems);
+    const int nblocks = (int)((np + tile - 1) / tile);
     // The passes alternate between the two buffers and end in w.keys / w.vals;
     // the key kernel wrote the first pass's input (sort_key_input).
     const bool odd = passes & 1;
@@ -361,14 +478,13 @@ cudaError_t sort_keys_to_chunks(const TileGeom& tg, long np, SortWork& w, cudaSt
     int* vout = odd ? w.vals : w.vals_alt;
     for (int ps = 0; ps < passes; ++ps) {
         const int shift_bits = ps * dbits;
-        radix_hist_kernel<<<nblocks, kSortThreads, 0, st>>>(kin, np, shift_bits, digits, nblocks, w.hist);
+        auto hist = small ? radix_hist_kernel<kSortItemsSmall> : radix_hist_kernel<kSortItems>;
+        auto scatter = small ? (ps == 0 ? radix_scatter_kernel<kSortItemsSmall, true>
+                                        : radix_scatter_kernel<kSortItemsSmall, false>)
+                             : (ps == 0 ? radix_scatter_kernel<kSortItems, true> : radix_scatter_kernel<kSortItems, false>);
+        hist<<<nblocks, kSortThreads, 0, st>>>(kin, np, shift_bits, digits, nblocks, w.hist);
         exclusive_scan(w.hist, w.hist, (long)digits * nblocks, w.scan_tmp, nullptr, st);
-        if (ps == 0)
-            radix_scatter_kernel<true><<<nblocks, kSortThreads, 0, st>>>(kin, nullptr, np, shift_bits, digits,
-                                                                         nblocks, w.hist, kout, vout);
-        else
-            radix_scatter_kernel<false><<<nblocks, kSortThreads, 0, st>>>(kin, vin, np, shift_bits, digits,
-                                                                          nblocks, w.hist, kout, vout);
+        scatter<<<nblocks, kSortThreads, 0, st>>>(kin, vin, np, shift_bits, digits, nblocks, w.hist, kout, vout);
         count_launches(2);
         unsigned* tk = kin; kin = kout; kout = tk;
         vin = vout;
@@ -378,6 +494,12 @@ cudaError_t sort_keys_to_chunks(const TileGeom& tg, long np, SortWork& w, cudaSt
     const int ntiles = tg.ntx * tg.nty;
     tile_bounds_kernel<<<grid_for(np + 1), 256, 0, st>>>(w.keys, np, (unsigned)(tg.tile_x * tg.tile_y * tg.classes),
                                                          ntiles, w.tile_start);
+    if (ntiles <= kTilesOne) {
+        chunk_table_kernel<<<1, kScanOneThreads, 0, st>>>(w.tile_start, ntiles, tg.chunk, w.tile_chunks, w.nchunks,
+                                                          w.chunks);
+        count_launches(2);
+        return cudaGetLastError();
+    }
     tile_counts_kernel<<<(ntiles + 255) / 256, 256, 0, st>>>(w.tile_start, ntiles, w.tile_count);
     count_launches(2);
     tile_chunks_kernel<<<(ntiles + 255) / 256, 256, 0, st>>>(w.tile_count, ntiles, tg.chunk, w.tile_chunks);
@@ -411,8 +533,22 @@ cudaError_t permute_particles(const ParticleSoA& s, const ParticleSoA& d, long n
     return cudaGetLastError();
 }
 
-cudaError_t unpermute_particles(const ParticleSoA& s, const ParticleSoA& d, long np, cudaStream_t st) {
-    unpermute_kernel<<<grid_for(np), 256, 0, st>>>(s, d, np);
+cudaError_t invert_order(const int* id, long np, int* inv, cudaStream_t st) {
+    invert_kernel<<<grid_for(np), 256, 0, st>>>(id, np, inv);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t gather_pair(const double* a, const double* b, const int* inv, long np, double* oa, double* ob,
+                        cudaStream_t st) {
+    gather_pair_kernel<<<grid_for(np), 256, 0, st>>>(a, b, inv, np, oa, ob);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t gather_triple(const double* a, const double* b, const double* c, const int* inv, long np, double* out,
+                          cudaStream_t st) {
+    gather_triple_kernel<<<grid_for(np), 256, 0, st>>>(a, b, c, inv, np, out);
     count_launches(1);
     return cudaGetLastError();
 }
