@@ -125,10 +125,16 @@ int choose_chunk(long np, int grid, int max_chunk, int unit) {
     return (int)t;
 }
 
-// Particles per push chunk: the launch's resident CTAs each get one while a
-// 2048-particle chunk would leave some without (16,384 particles: 64 CTAs of
-// one 256-particle round instead of 16 of four).
-int push_chunk(const upic_ctx* c) { return choose_chunk(c->np, c->push_grid, 2048, 256); }
+// Particles per push chunk: 2048, or 1024 while that leaves resident CTAs
+// without a chunk.  Each chunk clears and folds its windows once, which many
+// small runs side by side pay in SM time and one small run alone gains back
+// in latency.  A smallest chunk of 256 / 512 / 1024 / 2048 takes
+//   32 x 32 x 16, 50 steps alone             3.71 / 3.78 / 4.33 / 4.56 ms
+//   64 x 64 x 64, 50 steps alone             5.37 / 5.25 / 5.24 / 6.26 ms
+//   32 runs of 1e4..1e5, 120 steps, a graph  34.2 / 31.7 / 30.5 / 30.2 ms
+// A run of an ensemble sums in the same order as the run alone, so both take
+// one rule.
+int push_chunk(const upic_ctx* c) { return choose_chunk(c->np, c->push_grid, 2048, 1024); }
 
 int alloc_soa(upic_ctx* c, ParticleSoA& s, long cap, bool with_state, bool with_qm) {
     int rc = 0;

@@ -756,7 +756,7 @@ constexpr int kNSums = 8;  // gauge, gauss, cont, Bz, B, E, rho, J
 // sum_x f^2 = (1/N) sum_k |f_hat|^2 (Parseval; double-double, fixed order), so
 // that no field is transformed back: at 64 x 64 the ten inverse transforms,
 // the reduction over their results and its one-warp finish took 60 of a
-// step's 231 us, this launch takes about 6.  Without pairing (a one-cell
+// step's 231 us, this launch takes 14 (512 x 512: 44).  Without pairing (a one-cell
 // axis) a field is the real part of its transform, whose spectrum is
 // (f(k) + conj f(-k)) / 2.  The last block to finish adds the blocks'
 // partials and the push kernel's particle partials in index order and writes

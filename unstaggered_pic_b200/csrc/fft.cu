@@ -157,7 +157,7 @@ enum YPass { kForward = 0, kInverse = 1, kForwardAcc = 2, kForwardAcc1 = 3 };
 
 // Values of component c at E nodes from the accumulators, which are cleared.
 // All words are read before the first store, so that the loads overlap (6.4
-// -> 3.1 us a launch at 32 x 32, 23 -> 14 us at 512 x 512).
+// -> 3.6 us a launch at 32 x 32, 23 -> 9.6 us at 512 x 512).
 template <bool SINGLE, int E>
 UPIC_D void take_acc(const FftAccIn& a, int c, size_t N, size_t node, int step, double (&v)[E]) {
     unsigned long long* h = a.acc + (size_t)(2 * c) * N + node;

@@ -9,9 +9,9 @@
 // (solve_local_particle_substep :4930, evaluate_local_particle_substep :4843)
 // followed by the orbit-averaged current deposit of the accepted orbit
 // (path_average_deposit_current :2784), one thread per particle
-// (implicit_solve_kernel, implicit_deposit_kernel).  The grid runs in 2D (nz = 1): the z stencil of the
-// reference then sums to one, so its z factors and z-knot splits only change
-// rounding and are dropped here.
+// (implicit_solve_kernel, implicit_deposit_kernel).  The grid runs in 2D
+// (nz = 1): the z stencil of the reference then sums to one, so its z factors
+// and z-knot splits only change rounding and are dropped here.
 #include <climits>
 
 #include "deposit.cuh"

@@ -26,7 +26,7 @@ namespace {
 constexpr int kSortThreads = 256;
 // Keys per thread of a radix pass: 16 (4096-key blocks) for sets that fill the
 // GPU with such blocks, 4 below: a 16,384-particle pass then runs 16 blocks of
-// four rounds instead of four blocks of sixteen (scatter 16.3 -> 5.6 us).
+// four rounds instead of four blocks of sixteen (scatter 16.3 -> 5.7 us).
 constexpr int kSortItems = 16, kSortItemsSmall = 4;
 constexpr long kSortSmall = 148L * kSortThreads * kSortItems;
 constexpr int sort_tile(int items) { return kSortThreads * items; }  // elements per block
@@ -361,7 +361,7 @@ __global__ void gather_set_kernel(GatherSet g, const int* __restrict__ idx, long
 // are whole lines and its reads, within a few cells of each other, share
 // sectors in L2.  Scattering eleven arrays of 16.8M particles by id took 7.3
 // ms and the joins into triples 0.7 ms more; the inverse and the gathers
-// straight into triples take 1.5 ms together.
+// straight into triples take 2.9 ms together.
 __global__ void invert_kernel(const int* __restrict__ id, long n, int* __restrict__ inv) {
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
         inv[id[k]] = (int)k;
