@@ -36,6 +36,12 @@ constexpr int kHist = 5;         // Anderson memory + 1 (memory <= 4)
 constexpr int kNormGrid = 296;
 constexpr int kMaxImplicitChunk = 1024;
 
+struct MapReport {
+    MapStats stats;
+    NormSums norms;
+    int flag, perr;
+};
+
 struct ImplicitState {
     int order = 2, nq = 8;
     bool closed = false;     // orbit integrals in closed form (ImplicitMapArgs::closed)
@@ -70,12 +76,15 @@ struct ImplicitState {
     double* hr[kHist] = {};
     int hcount = 0;
     double* partials = nullptr;
-    NormSums* dnorm = nullptr;
-    NormSums* hnorm = nullptr;    // pinned
-    MapStats* dstats = nullptr;
-    MapStats* hstats = nullptr;   // pinned
-    int* dflag = nullptr;
-    int* hflag = nullptr;         // pinned
+    unsigned* ticket = nullptr;   // of the reductions over partials
+    // what an evaluation reports, read back in one copy; the pointers lead into it
+    MapReport* dreport = nullptr;
+    MapReport* hreport = nullptr;  // pinned
+    NormSums *dnorm = nullptr, *hnorm = nullptr;
+    MapStats *dstats = nullptr, *hstats = nullptr;
+    int *dflag = nullptr, *hflag = nullptr;
+    int* perr = nullptr;
+    MapReset reset() const { return {acc, dstats, dflag, perr, nfailed}; }
     double* ddots = nullptr;
     double* hdots = nullptr;      // pinned (32)
     double scaleJ[4] = {1, 1, 1, 1};
@@ -140,7 +149,6 @@ struct ImplicitState {
     NormSums* hnorm3 = nullptr;  // pinned (3)
     double* hloss = nullptr;     // pinned
     unsigned long long* pstat = nullptr;                  // path statistics counters (4)
-    int* perr = nullptr;
     double vb_limit = 0.0;  // bound on |vbar| components of the fixed-point deposit
     double dt_max = 0.0;    // dt at creation: the deposit window guard covers kappa * dt_max
     bool loaded = false;  // upic_set_particles has succeeded
@@ -391,9 +399,8 @@ int eval_map(upic_ctx* c, ImplicitState& s, const double* guess, double* out, bo
     const upic_config& cf = c->cfg;
     const int N = c->N;
     // J_field = projected guess (:5264-5265), its spectra
-    UPIC_CUDA(c, cudaMemcpyAsync(s.Jf, guess, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, c->st));
-    if (cf.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(s.Jf, 3, c->nx, c->ny, c->st));
-    UPIC_CUDA(c, fft2d_batched(c->plan, s.Jhat, 3, 0, c->st, s.Jf));
+    if (cf.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(guess, s.Jf, 3, c->nx, c->ny, c->st));
+    UPIC_CUDA(c, fft2d_batched(c->plan, s.Jhat, 3, 0, c->st, cf.nyquist_projection ? s.Jf : guess));
     // continuity + CN update + grad phi_mid and A^{n+1} spectra
     CnArgs k{};
     k.nx = c->nx;
@@ -411,13 +418,11 @@ int eval_map(upic_ctx* c, ImplicitState& s, const double* guess, double* out, bo
     k.kappa = cf.kappa;
     k.sigma1 = cf.sigma1;
     k.sigma2 = cf.sigma2;
+    UPIC_CUDA(c, launch_map_reset(N, s.reset(), c->st));
     UPIC_CUDA(c, launch_cn_kspace(k, c->st));
     UPIC_CUDA(c, fft2d_batched(c->plan, s.gspec, 2, 1, c->st, nullptr, 2, s.rec, kIRec, kIRecGpm));
     UPIC_CUDA(c, fft2d_batched(c->plan, s.gspec + 2 * (size_t)N, 3, 1, c->st, nullptr, 2, s.rec, kIRec, kIRecAe));
     // particles: local fixed points and the orbit-averaged deposit
-    UPIC_CUDA(c, cudaMemsetAsync(s.acc, 0, sizeof(unsigned long long) * 6 * (size_t)N, c->st));
-    UPIC_CUDA(c, cudaMemsetAsync(s.dstats, 0, sizeof(MapStats), c->st));
-    UPIC_CUDA(c, cudaMemsetAsync(&s.dstats->first_fail_key, 0xff, sizeof(unsigned long long), c->st));
     const ParticleSoA& p = s.P[s.cur];
     const ParticleSoA& o = s.P[1 - s.cur];
     ImplicitMapArgs a{};
@@ -454,7 +459,6 @@ int eval_map(upic_ctx* c, ImplicitState& s, const double* guess, double* out, bo
     if (s.failed) {
         a.failed = s.failed;
         a.nfailed = s.nfailed;
-        UPIC_CUDA(c, cudaMemsetAsync(s.nfailed, 0, sizeof(int), c->st));
     }
     a.vbar_x = s.hvx;
     a.vbar_y = s.hvy;
@@ -484,17 +488,13 @@ int eval_map(upic_ctx* c, ImplicitState& s, const double* guess, double* out, bo
         if (s.layout_active && s.nref > 0) UPIC_CUDA(c, launch_refined_map(s.order, s.uniform, a, c->st));
     }
     UPIC_CUDA(c, launch_convert_acc(s.acc, N, s.scaleJ, out, nullptr, 0.0, 1, c->st));
-    if (cf.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(out, 3, c->nx, c->ny, c->st));
-    UPIC_CUDA(c, cudaMemcpyAsync(s.hstats, s.dstats, sizeof(MapStats), cudaMemcpyDeviceToHost, c->st));
-    if (map_finite) {
-        UPIC_CUDA(c, cudaMemsetAsync(s.dflag, 0, sizeof(int), c->st));
-        UPIC_CUDA(c, launch_nonfinite_flag(3 * N, out, s.dflag, c->st));
-        UPIC_CUDA(c, cudaMemcpyAsync(s.hflag, s.dflag, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-    }
+    if (cf.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(out, out, 3, c->nx, c->ny, c->st));
+    if (map_finite) UPIC_CUDA(c, launch_nonfinite_flag(3 * N, out, s.dflag, c->st));
     if (norms) {
         const int rn = launch_residual_sums(c, s, out, guess);
         if (rn) return rn;
     }
+    UPIC_CUDA(c, cudaMemcpyAsync(s.hreport, s.dreport, sizeof(MapReport), cudaMemcpyDeviceToHost, c->st));
     int rc = sync(c);
     if (rc) return rc;
     if (stats_out) *stats_out = *s.hstats;
@@ -543,10 +543,7 @@ int picard_eval(upic_ctx* c, ImplicitState& s, NormSums& vel) {
     const ParticleSoA& p = s.P[s.cur];
     const ParticleSoA& o = s.P[1 - s.cur];
     // Jbar: orbit-averaged deposit of vbar = (v_guess + v^n) / 2 (:1468-1472)
-    UPIC_CUDA(c, cudaMemsetAsync(s.acc, 0, sizeof(unsigned long long) * 6 * (size_t)N, c->st));
-    UPIC_CUDA(c, cudaMemsetAsync(s.dstats, 0, sizeof(MapStats), c->st));
-    UPIC_CUDA(c, cudaMemsetAsync(&s.dstats->first_fail_key, 0xff, sizeof(unsigned long long), c->st));
-    UPIC_CUDA(c, cudaMemsetAsync(s.perr, 0, sizeof(int), c->st));
+    UPIC_CUDA(c, launch_map_reset(N, s.reset(), c->st));
     if (s.np > 0) {
         ImplicitMapArgs a{};
         a.x = p.x; a.y = p.y; a.vx = p.vx; a.vy = p.vy; a.vz = p.vz;
@@ -609,15 +606,13 @@ int picard_eval(upic_ctx* c, ImplicitState& s, NormSums& vel) {
     q.partials = s.partials;
     q.err = s.perr;
     UPIC_CUDA(c, launch_picard_push(s.order, s.uniform, q, kNormGrid, s.dnorm, c->st));
-    UPIC_CUDA(c, cudaMemcpyAsync(s.hstats, s.dstats, sizeof(MapStats), cudaMemcpyDeviceToHost, c->st));
-    UPIC_CUDA(c, cudaMemcpyAsync(s.hnorm, s.dnorm, sizeof(NormSums), cudaMemcpyDeviceToHost, c->st));
-    UPIC_CUDA(c, cudaMemcpyAsync(s.hflag, s.perr, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    UPIC_CUDA(c, cudaMemcpyAsync(s.hreport, s.dreport, sizeof(MapReport), cudaMemcpyDeviceToHost, c->st));
     int rc = sync(c);
     if (rc) return rc;
     if (s.hstats->failures > 0 && (int)(s.hstats->first_fail_key & 0xffu) == kLocalNonfiniteIterate)
         return fail(c, UPIC_ERR_NONCONVERGED,
                     "Picard iterate velocity is not finite or exceeds 16 times the initial bound max(|v|, c)");
-    if (s.hstats->failures > 0 || *s.hflag > 0)
+    if (s.hstats->failures > 0 || s.hreport->perr > 0)
         return fail(c, UPIC_ERR_TOO_LARGE, "an orbit crosses more spline knots than the kernel holds (38)");
     vel = *s.hnorm;
     return 0;
@@ -660,7 +655,7 @@ int picard_one_step(upic_ctx* c, ImplicitState& s, double* info) {
         vel_err = relative_rms(vel, 3.0 * (double)s.np);
         cur_err = INFINITY;
         if (have_prev) {
-            UPIC_CUDA(c, launch_residual_norms(N, s.map, s.Jprev, 1.0, 0.0, 1.0, s.partials, kNormGrid, s.dnorm,
+            UPIC_CUDA(c, launch_residual_norms(N, s.map, s.Jprev, 1.0, 0.0, 1.0, s.partials, kNormGrid, s.ticket, s.dnorm,
                                                c->st));
             UPIC_CUDA(c, cudaMemcpyAsync(s.hnorm, s.dnorm, sizeof(NormSums), cudaMemcpyDeviceToHost, c->st));
             if ((rc = sync(c))) return rc;
@@ -719,14 +714,13 @@ int all_finite(upic_ctx* c, ImplicitState& s, const double* v, bool& finite) {
     return 0;
 }
 
-// nonlinear_residual_norms (:5576) on node vectors: the device sums and their
-// copy to the host, queued on the context's stream ...
+// nonlinear_residual_norms (:5576) on node vectors: the device sums, queued on
+// the context's stream; the caller copies them to the host ...
 int launch_residual_sums(upic_ctx* c, ImplicitState& s, const double* map, const double* guess) {
     const upic_config& cf = c->cfg;
     const double floor_rel = 64.0 * DBL_EPSILON * cf.kappa;
     UPIC_CUDA(c, launch_residual_norms(c->N, map, guess, floor_rel, cf.nonlinear_atol, cf.nonlinear_rtol,
-                                       s.partials, kNormGrid, s.dnorm, c->st));
-    UPIC_CUDA(c, cudaMemcpyAsync(s.hnorm, s.dnorm, sizeof(NormSums), cudaMemcpyDeviceToHost, c->st));
+                                       s.partials, kNormGrid, s.ticket, s.dnorm, c->st));
     return 0;
 }
 
@@ -762,7 +756,7 @@ int anderson_candidate(upic_ctx* c, ImplicitState& s, bool& ok) {
         x[k] = s.hx[first + k];
     }
     const int n3 = 3 * c->N;
-    UPIC_CUDA(c, launch_anderson_dots(n3, r, m, s.partials, kNormGrid, s.ddots, c->st));
+    UPIC_CUDA(c, launch_anderson_dots(n3, r, m, s.partials, kNormGrid, s.ticket, s.ddots, c->st));
     const int ndots = m * (m + 1) / 2 + m;
     UPIC_CUDA(c, cudaMemcpyAsync(s.hdots, s.ddots, sizeof(double) * ndots, cudaMemcpyDeviceToHost, c->st));
     int rc = sync(c);
@@ -791,7 +785,8 @@ int anderson_candidate(upic_ctx* c, ImplicitState& s, bool& ok) {
     return 0;
 }
 
-void push_history(upic_ctx* c, ImplicitState& s, const double* x, const double* r) {
+// The slot of the next history entry; the oldest entry makes room for it.
+int history_slot(upic_ctx* c, ImplicitState& s) {
     const int keep = c->cfg.anderson_memory + 1;
     if (s.hcount == keep) {
         double* tx = s.hx[0];
@@ -804,10 +799,14 @@ void push_history(upic_ctx* c, ImplicitState& s, const double* x, const double* 
         s.hr[s.hcount - 1] = tr;
         --s.hcount;
     }
+    return s.hcount++;
+}
+
+void push_history(upic_ctx* c, ImplicitState& s, const double* x, const double* r) {
+    const int k = history_slot(c, s);
     const size_t bytes = sizeof(double) * 3 * (size_t)c->N;
-    cudaMemcpyAsync(s.hx[s.hcount], x, bytes, cudaMemcpyDeviceToDevice, c->st);
-    cudaMemcpyAsync(s.hr[s.hcount], r, bytes, cudaMemcpyDeviceToDevice, c->st);
-    ++s.hcount;
+    cudaMemcpyAsync(s.hx[k], x, bytes, cudaMemcpyDeviceToDevice, c->st);
+    cudaMemcpyAsync(s.hr[k], r, bytes, cudaMemcpyDeviceToDevice, c->st);
 }
 
 void reset_history(upic_ctx* c, ImplicitState& s, const double* x, const double* r) {
@@ -976,15 +975,15 @@ int outer_solve(upic_ctx* c, ImplicitState& s, OuterResult& out) {
             // (:5981-5996); read back with the final evaluation
             const double* xs[2] = {s.trial, s.guess};
             const double* gs[2] = {s.trial_map, s.map};
-            UPIC_CUDA(c, launch_anderson_dots(n3, xs, 1, s.partials, kNormGrid, s.dcon + 4 * (size_t)it, c->st));
-            UPIC_CUDA(c, launch_anderson_dots(n3, gs, 1, s.partials, kNormGrid, s.dcon + 4 * (size_t)it + 2,
-                                              c->st));
+            UPIC_CUDA(c, launch_anderson_dots(n3, xs, 1, s.partials, kNormGrid, s.ticket, s.dcon + 4 * (size_t)it, c->st));
+            UPIC_CUDA(c, launch_anderson_dots(n3, gs, 1, s.partials, kNormGrid, s.ticket,
+                                              s.dcon + 4 * (size_t)it + 2, c->st));
         }
         have_prefetched = false;
-        UPIC_CUDA(c, launch_axpy(n3, s.map, s.guess, -1.0, s.resid, c->st));
         iterations = it + 1;
         if (it == 0) first_rms = norms.rms_relative;
         if (norms.rms_scaled <= 1.0 && norms.max_scaled <= 1.0) {
+            UPIC_CUDA(c, launch_axpy(n3, s.map, s.guess, -1.0, s.resid, c->st));
             converged = true;
             break;
         }
@@ -992,7 +991,8 @@ int outer_solve(upic_ctx* c, ImplicitState& s, OuterResult& out) {
             s.hcount = 0;
             ++restarts;
         }
-        push_history(c, s, s.guess, s.resid);
+        const int slot = history_slot(c, s);
+        UPIC_CUDA(c, launch_residual_push(n3, s.map, s.guess, s.resid, s.hx[slot], s.hr[slot], c->st));
         bool used_anderson = false;
         if (anderson && it >= cf.anderson_start && s.hcount >= 2) {
             if ((rc = anderson_candidate(c, s, used_anderson))) return rc;
@@ -1199,7 +1199,7 @@ int predictor_update(upic_ctx* c, ImplicitState& s, double* info) {
     const double* cand[3] = {s.J0, s.have_Jx ? s.Jx : nullptr, s.have_Jl ? s.Jl : nullptr};
     for (int k = 0; k < 3; ++k)
         if (cand[k])
-            UPIC_CUDA(c, launch_residual_norms(N, s.J, cand[k], 1.0, 0.0, 1.0, s.partials, kNormGrid, s.dnorm3 + k,
+            UPIC_CUDA(c, launch_residual_norms(N, s.J, cand[k], 1.0, 0.0, 1.0, s.partials, kNormGrid, s.ticket, s.dnorm3 + k,
                                                c->st));
     bool trained = false;
     if (learned && gnet::net_frames(s.net) >= gnet::kFrames && s.trained_steps < cf.learned_train_steps) {
@@ -1471,9 +1471,16 @@ int implicit_create(upic_ctx* c) {
         (rc = dalloc(c, &s->map, 3 * (size_t)N)) || (rc = dalloc(c, &s->trial, 3 * (size_t)N)) ||
         (rc = dalloc(c, &s->trial_map, 3 * (size_t)N)) || (rc = dalloc(c, &s->cand, 3 * (size_t)N)) ||
         (rc = dalloc(c, &s->resid, 3 * (size_t)N)) || (rc = dalloc(c, &s->partials, 64 * (size_t)kNormGrid)) ||
-        (rc = dalloc(c, &s->dnorm, 1)) || (rc = dalloc(c, &s->dstats, 1)) || (rc = dalloc(c, &s->ddots, 32)) ||
-        (rc = dalloc(c, &s->dflag, 1)) || (rc = dalloc(c, &s->pstat, 4)) || (rc = dalloc(c, &s->perr, 1)))
+        (rc = dalloc(c, &s->dreport, 1)) || (rc = dalloc(c, &s->ticket, 1)) || (rc = dalloc(c, &s->ddots, 32)) ||
+        (rc = dalloc(c, &s->pstat, 4)))
         return rc;
+    s->dnorm = &s->dreport->norms;
+    s->dstats = &s->dreport->stats;
+    s->dflag = &s->dreport->flag;
+    s->perr = &s->dreport->perr;
+    if (cudaMemset(s->ticket, 0, sizeof(unsigned)) != cudaSuccess ||
+        cudaMemset(s->dreport, 0, sizeof(MapReport)) != cudaSuccess)
+        return fail(c, UPIC_ERR_CUDA, "cudaMemset failed");
     if (s->picard && (rc = dalloc(c, &s->Jprev, 3 * (size_t)N))) return rc;
     if (c->cfg.current_predictor == UPIC_PREDICTOR_EXTRAPOLATED && (rc = dalloc(c, &s->Jold, 3 * (size_t)N)))
         return rc;
@@ -1489,14 +1496,15 @@ int implicit_create(upic_ctx* c) {
     }
     for (int k = 0; k < kHist; ++k)
         if ((rc = dalloc(c, &s->hx[k], 3 * (size_t)N)) || (rc = dalloc(c, &s->hr[k], 3 * (size_t)N))) return rc;
-    if (cudaMallocHost(&s->hnorm, sizeof(NormSums)) != cudaSuccess ||
-        cudaMallocHost(&s->hstats, sizeof(MapStats)) != cudaSuccess ||
+    if (cudaMallocHost(&s->hreport, sizeof(MapReport)) != cudaSuccess ||
         cudaMallocHost(&s->hdots, sizeof(double) * 32) != cudaSuccess ||
-        cudaMallocHost(&s->hflag, sizeof(int)) != cudaSuccess ||
         cudaMallocHost(&s->hnorm3, sizeof(NormSums) * 3) != cudaSuccess ||
         cudaMallocHost(&s->hloss, sizeof(double)) != cudaSuccess ||
         cudaMallocHost(&s->hcon, sizeof(double) * 4 * (size_t)std::max(1, c->cfg.nonlinear_max_iter)) != cudaSuccess)
         return fail(c, UPIC_ERR_NOMEM, "cudaMallocHost failed");
+    s->hnorm = &s->hreport->norms;
+    s->hstats = &s->hreport->stats;
+    s->hflag = &s->hreport->flag;
     if ((rc = dalloc(c, &s->dcon, 4 * (size_t)std::max(1, c->cfg.nonlinear_max_iter)))) return rc;
     std::vector<unsigned char> ex(N, 0);
     for (int i = 0; i < c->nx; ++i)
@@ -1510,10 +1518,8 @@ int implicit_create(upic_ctx* c) {
 void implicit_destroy(upic_ctx* c) {
     if (!c || !c->imp) return;
     ImplicitState* s = c->imp;
-    if (s->hnorm) cudaFreeHost(s->hnorm);
-    if (s->hstats) cudaFreeHost(s->hstats);
+    if (s->hreport) cudaFreeHost(s->hreport);
     if (s->hdots) cudaFreeHost(s->hdots);
-    if (s->hflag) cudaFreeHost(s->hflag);
     if (s->hnorm3) cudaFreeHost(s->hnorm3);
     if (s->hloss) cudaFreeHost(s->hloss);
     if (s->hcon) cudaFreeHost(s->hcon);
@@ -1696,7 +1702,7 @@ int implicit_init_fields(upic_ctx* c, double* diag_row) {
     // uniform background only enters the k = 0 mode.
     double* rho = s.dreal;
     UPIC_CUDA(c, launch_convert_acc(s.acc, N, s.scaleJ, s.J, rho, 0.0, 3, c->st));
-    if (cf.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(s.J, 3, c->nx, c->ny, c->st));
+    if (cf.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(s.J, s.J, 3, c->nx, c->ny, c->st));
     // spectra: phi from Poisson (solve_periodic_poisson_for_phi :3196), psi = A = U = 0
     UPIC_CUDA(c, cudaMemsetAsync(s.spec, 0, sizeof(double2) * 9 * (size_t)N, c->st));
     UPIC_CUDA(c, fft2d_batched(c->plan, s.spec + 2 * (size_t)N, 1, 0, c->st, rho));
@@ -1999,7 +2005,7 @@ extern "C" int upic_orbit_deposit(upic_ctx* c, long np, const double* x, const d
     }
     double* out = s.dreal;
     UPIC_CUDA(c, launch_convert_acc(s.acc, N, sc4, out, nullptr, 0.0, 1, c->st));
-    if (c->cfg.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(out, 3, c->nx, c->ny, c->st));
+    if (c->cfg.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(out, out, 3, c->nx, c->ny, c->st));
     UPIC_CUDA(c, cudaMemcpyAsync(J, out, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, c->st));
     return orbit_check(c, s);
 }
@@ -2441,7 +2447,7 @@ extern "C" int upic_fft_solve_cn(upic_ctx* c, const double* phi, const double* p
     UPIC_CUDA(c, fft2d_batched(c->plan, sin_, 9, 0, c->st, dreal));
     // J_field: the Nyquist-projected current (:5265-5266)
     UPIC_CUDA(c, cudaMemcpyAsync(dj, J, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->st));
-    if (cf.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(dj, 3, c->nx, c->ny, c->st));
+    if (cf.nyquist_projection) UPIC_CUDA(c, launch_project_nyquist(dj, dj, 3, c->nx, c->ny, c->st));
     UPIC_CUDA(c, fft2d_batched(c->plan, jhat, 3, 0, c->st, dj));
     CnArgs k{};
     k.nx = c->nx;

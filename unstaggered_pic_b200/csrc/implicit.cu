@@ -12,6 +12,7 @@
 // (implicit_solve_kernel, implicit_deposit_kernel).  The grid runs in 2D
 // (nz = 1): the z stencil of the reference then sums to one, so its z factors
 // and z-knot splits only change rounding and are dropped here.
+#include <algorithm>
 #include <climits>
 
 #include "deposit.cuh"
@@ -2298,6 +2299,19 @@ UPIC_D double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y +
 UPIC_D double2 cscale(double s, double2 a) { return make_double2(s * a.x, s * a.y); }
 UPIC_D double2 cik(double k, double2 z) { return make_double2(-k * z.y, k * z.x); }
 
+// What a map evaluation adds to starts at zero: one launch of 1.6 us where
+// four or five clears took 1.1 us each and their gaps.
+__global__ void map_reset_kernel(int N, MapReset r) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *r.stats = MapStats{};
+        r.stats->first_fail_key = ~0ull;
+        *r.flag = 0;
+        *r.perr = 0;
+        if (r.nfailed) *r.nfailed = 0;
+    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 6 * N; i += gridDim.x * blockDim.x) r.acc[i] = 0ull;
+}
+
 __global__ void cn_kspace_kernel(CnArgs a) {
     const int N = a.N;
     const double c2 = a.kappa * a.kappa;
@@ -2398,7 +2412,8 @@ __global__ void momentum_from_v_kernel(long np, const double* vx, const double* 
 // fixed xor tree combines the lanes (the same order on every run).
 // Axis 1 (lines along y) reads rows contiguously; axis 0 (lines along x)
 // makes 32 lines of consecutive j share each warp's columns via the grid.
-__global__ void project_lines_kernel(double* f, int ncomp, int nx, int ny, int axis) {
+// From `src` to `dst`, which may be the same.
+__global__ void project_lines_kernel(const double* src, double* dst, int ncomp, int nx, int ny, int axis) {
     const int n = axis == 0 ? nx : ny;
     const int lines = axis == 0 ? ny : nx;
     const int stride = axis == 0 ? ny : 1;
@@ -2407,15 +2422,17 @@ __global__ void project_lines_kernel(double* f, int ncomp, int nx, int ny, int a
     const long warps = (long)gridDim.x * (blockDim.x >> 5);
     for (long L = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5); L < total; L += warps) {
         const int c = (int)(L / lines), l = (int)(L - (long)c * lines);
-        double* base = f + (size_t)c * nx * ny + (axis == 0 ? l : (size_t)l * ny);
+        const size_t first = (size_t)c * nx * ny + (axis == 0 ? l : (size_t)l * ny);
+        const double* in = src + first;
+        double* out = dst + first;
         DD s{0.0, 0.0};
         for (int j = lane; j < n; j += 32) {
-            const double v = base[(size_t)j * stride];
+            const double v = in[(size_t)j * stride];
             s = dd_add(s, (j & 1) ? -v : v);
         }
         s = warp_sum_dd(s);
         const double mean = (s.hi + s.lo) / (double)n;
-        for (int j = lane; j < n; j += 32) base[(size_t)j * stride] -= (j & 1) ? -mean : mean;
+        for (int j = lane; j < n; j += 32) out[(size_t)j * stride] = in[(size_t)j * stride] - ((j & 1) ? -mean : mean);
     }
 }
 
@@ -2429,9 +2446,53 @@ __global__ void kspace_mask_kernel(double2* f, int ncomp, int N, const unsigned 
 // ---- outer iteration algebra ------------------------------------------------
 constexpr int kRed = 256;
 
+// True in the launch's last block to get here, whose threads then see what
+// every block wrote before; the ticket is back at zero after the launch.
+UPIC_D bool last_block(unsigned* ticket) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// One warp: lane l combines the partials l, l+32, ...; a fixed xor tree
+// combines the lanes.
+UPIC_D void residual_final(const double* partials, int grid, NormSums* out) {
+    DD a{0, 0}, b{0, 0}, c{0, 0};
+    double x = 0.0, y = 0.0;
+    for (int k = threadIdx.x; k < grid; k += 32) {
+        const double* o = partials + (size_t)k * 8;
+        a = dd_add_dd(a, DD{__ldcg(o), __ldcg(o + 1)});
+        b = dd_add_dd(b, DD{__ldcg(o + 2), __ldcg(o + 3)});
+        c = dd_add_dd(c, DD{__ldcg(o + 4), __ldcg(o + 5)});
+        x = fmax(x, __ldcg(o + 6));
+        y = fmax(y, __ldcg(o + 7));
+    }
+    a = warp_sum_dd(a);
+    b = warp_sum_dd(b);
+    c = warp_sum_dd(c);
+    x = warp_max(x);
+    y = warp_max(y);
+    if (threadIdx.x != 0) return;
+    out->r2[0] = a.hi; out->r2[1] = a.lo;
+    out->map2[0] = b.hi; out->map2[1] = b.lo;
+    out->guess2[0] = c.hi; out->guess2[1] = c.lo;
+    out->max_rel = x;
+    out->max_scaled = y;
+}
+
+__global__ void residual_final_kernel(const double* partials, int grid, NormSums* out) {
+    residual_final(partials, grid, out);
+}
+
+// The last block finishes.  A separate one-warp finish over 296 blocks, most
+// of them empty on a small grid, took 7.1 us after 3.8 at 64 x 64.
 __global__ void __launch_bounds__(kRed)
 residual_norms_kernel(int N, const double* map, const double* guess, double floor_rel, double atol,
-                      double rtol, double* partials) {
+                      double rtol, double* partials, unsigned* ticket, NormSums* out) {
     DD r2{0, 0}, m2{0, 0}, g2{0, 0};
     double mrel = 0.0, msc = 0.0;
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < N; id += gridDim.x * blockDim.x) {
@@ -2474,32 +2535,7 @@ residual_norms_kernel(int N, const double* map, const double* guess, double floo
         double* o = partials + (size_t)blockIdx.x * 8;
         o[0] = a.hi; o[1] = a.lo; o[2] = b.hi; o[3] = b.lo; o[4] = c.hi; o[5] = c.lo; o[6] = x; o[7] = y;
     }
-}
-
-// One warp: lane l combines the partials l, l+32, ...; a fixed xor tree
-// combines the lanes.
-__global__ void residual_final_kernel(const double* partials, int grid, NormSums* out) {
-    DD a{0, 0}, b{0, 0}, c{0, 0};
-    double x = 0.0, y = 0.0;
-    for (int k = threadIdx.x; k < grid; k += 32) {
-        const double* o = partials + (size_t)k * 8;
-        a = dd_add_dd(a, DD{o[0], o[1]});
-        b = dd_add_dd(b, DD{o[2], o[3]});
-        c = dd_add_dd(c, DD{o[4], o[5]});
-        x = fmax(x, o[6]);
-        y = fmax(y, o[7]);
-    }
-    a = warp_sum_dd(a);
-    b = warp_sum_dd(b);
-    c = warp_sum_dd(c);
-    x = warp_max(x);
-    y = warp_max(y);
-    if (threadIdx.x != 0) return;
-    out->r2[0] = a.hi; out->r2[1] = a.lo;
-    out->map2[0] = b.hi; out->map2[1] = b.lo;
-    out->guess2[0] = c.hi; out->guess2[1] = c.lo;
-    out->max_rel = x;
-    out->max_scaled = y;
+    if (last_block(ticket) && threadIdx.x < 32) residual_final(partials, gridDim.x, out);
 }
 
 struct RPtrs {
@@ -2509,7 +2545,7 @@ struct RPtrs {
 constexpr int kMaxDots = 14;
 
 __global__ void __launch_bounds__(kRed)
-anderson_dots_kernel(int n, RPtrs rp, int m, double* partials) {
+anderson_dots_kernel(int n, RPtrs rp, int m, double* partials, unsigned* ticket, double* out) {
     DD s[kMaxDots];
     for (int k = 0; k < kMaxDots; ++k) s[k] = DD{0, 0};
     const int ndots = m * (m + 1) / 2 + m;
@@ -2546,17 +2582,18 @@ anderson_dots_kernel(int n, RPtrs rp, int m, double* partials) {
         partials[(size_t)blockIdx.x * 2 * kMaxDots + 2 * threadIdx.x] = t.hi;
         partials[(size_t)blockIdx.x * 2 * kMaxDots + 2 * threadIdx.x + 1] = t.lo;
     }
-}
-
-// One warp per dot (blockDim = 32 * ndots), lanes over the partials.
-__global__ void dots_final_kernel(const double* partials, int grid, int ndots, double* out) {
-    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (k >= ndots) return;
-    DD t{0, 0};
-    for (int b = lane; b < grid; b += 32)
-        t = dd_add_dd(t, DD{partials[(size_t)b * 2 * kMaxDots + 2 * k], partials[(size_t)b * 2 * kMaxDots + 2 * k + 1]});
-    t = warp_sum_dd(t);
-    if (lane == 0) out[k] = t.hi + t.lo;
+    if (!last_block(ticket)) return;
+    // a warp per dot, lanes over the partials
+    const int lane = threadIdx.x & 31;
+    for (int k = w; k < ndots; k += kRed / kWarp) {
+        DD t{0, 0};
+        for (int b = lane; b < (int)gridDim.x; b += 32) {
+            const double* p = partials + (size_t)b * 2 * kMaxDots + 2 * k;
+            t = dd_add_dd(t, DD{__ldcg(p), __ldcg(p + 1)});
+        }
+        t = warp_sum_dd(t);
+        if (lane == 0) out[k] = t.hi + t.lo;
+    }
 }
 
 struct GPtrs {
@@ -2602,6 +2639,17 @@ __global__ void lerp_kernel(int n, const double* a, const double* b, double s, d
 __global__ void axpy_kernel(int n, const double* a, const double* b, double s, double* out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         out[i] = a[i] + s * b[i];
+}
+
+// resid = map - guess, and the pair (guess, resid) into a history slot.
+__global__ void residual_push_kernel(int n, const double* map, const double* guess, double* resid, double* hx,
+                                     double* hr) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double g = guess[i], r = map[i] + -1.0 * g;
+        resid[i] = r;
+        hx[i] = g;
+        hr[i] = r;
+    }
 }
 
 // ---- step diagnostics (compute_subcycled_step_diagnostics :4340 with one
@@ -3605,15 +3653,32 @@ cudaError_t launch_momentum_from_v(long np, const double* vx, const double* vy, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_project_nyquist(double* f, int ncomp, int nx, int ny, cudaStream_t st) {
+cudaError_t launch_project_nyquist(const double* src, double* dst, int ncomp, int nx, int ny, cudaStream_t st) {
     if (nx > 1 && nx % 2 == 0) {
-        project_lines_kernel<<<gsize((long)ncomp * ny, 8), 256, 0, st>>>(f, ncomp, nx, ny, 0);
+        project_lines_kernel<<<gsize((long)ncomp * ny, 8), 256, 0, st>>>(src, dst, ncomp, nx, ny, 0);
         count_launches(1);
+        src = dst;
     }
     if (ny > 1 && ny % 2 == 0) {
-        project_lines_kernel<<<gsize((long)ncomp * nx, 8), 256, 0, st>>>(f, ncomp, nx, ny, 1);
+        project_lines_kernel<<<gsize((long)ncomp * nx, 8), 256, 0, st>>>(src, dst, ncomp, nx, ny, 1);
         count_launches(1);
+        src = dst;
     }
+    if (src != dst)  // no even axis
+        return cudaMemcpyAsync(dst, src, sizeof(double) * ncomp * (size_t)nx * ny, cudaMemcpyDeviceToDevice, st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_map_reset(int N, const MapReset& r, cudaStream_t st) {
+    map_reset_kernel<<<gsize(6L * N), 256, 0, st>>>(N, r);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_residual_push(int n, const double* map, const double* guess, double* resid, double* hx, double* hr,
+                                 cudaStream_t st) {
+    residual_push_kernel<<<gsize(n), 256, 0, st>>>(n, map, guess, resid, hx, hr);
+    count_launches(1);
     return cudaGetLastError();
 }
 
@@ -3625,21 +3690,22 @@ cudaError_t launch_kspace_mask(double2* f, int ncomp, int N, const unsigned char
 }
 
 cudaError_t launch_residual_norms(int N, const double* map, const double* guess, double floor_rel, double atol,
-                                  double rtol, double* partials, int grid, NormSums* out, cudaStream_t st) {
-    residual_norms_kernel<<<grid, kRed, 0, st>>>(N, map, guess, floor_rel, atol, rtol, partials);
-    residual_final_kernel<<<1, 32, 0, st>>>(partials, grid, out);
-    count_launches(2);
+                                  double rtol, double* partials, int grid, unsigned* ticket, NormSums* out,
+                                  cudaStream_t st) {
+    grid = std::min(grid, (N + kRed - 1) / kRed);  // no empty blocks: their zeros change no sum
+    residual_norms_kernel<<<grid, kRed, 0, st>>>(N, map, guess, floor_rel, atol, rtol, partials, ticket, out);
+    count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_anderson_dots(int n, const double* const* r, int m, double* partials, int grid, double* out,
-                                 cudaStream_t st) {
+cudaError_t launch_anderson_dots(int n, const double* const* r, int m, double* partials, int grid, unsigned* ticket,
+                                 double* out, cudaStream_t st) {
     if (m < 1 || m > 4) return cudaErrorInvalidValue;
     RPtrs rp{};
     for (int k = 0; k <= m; ++k) rp.r[k] = r[k];
-    anderson_dots_kernel<<<grid, kRed, 0, st>>>(n, rp, m, partials);
-    dots_final_kernel<<<1, 32 * (m * (m + 1) / 2 + m), 0, st>>>(partials, grid, m * (m + 1) / 2 + m, out);
-    count_launches(2);
+    grid = std::min(grid, (n + kRed - 1) / kRed);
+    anderson_dots_kernel<<<grid, kRed, 0, st>>>(n, rp, m, partials, ticket, out);
+    count_launches(1);
     return cudaGetLastError();
 }
 

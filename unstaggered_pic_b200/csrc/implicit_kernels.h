@@ -229,6 +229,14 @@ cudaError_t launch_add_qA(int order, int nx, int ny, double Lx, double Ly, const
 // k-space map step: J_field spectra -> rho_end, rho_mid, CN (phi, psi), (A, U)
 // and the spectra of grad phi_mid and A_end (continuity_charge_update :3288,
 // cn_potential_update :3249, cn_fft_wave_step_from_spectra :3131).
+// What a map evaluation starts from zero.
+struct MapReset {
+    unsigned long long* acc;  // 6 x N
+    MapStats* stats;
+    int *flag, *perr, *nfailed;  // nfailed may be null
+};
+cudaError_t launch_map_reset(int N, const MapReset& r, cudaStream_t st);
+
 struct CnArgs {
     int nx, ny, N;
     const double *kx, *ky, *k2;
@@ -251,7 +259,8 @@ cudaError_t launch_momentum_from_v(long np, const double* vx, const double* vy, 
 
 // Project every even-grid Nyquist plane out of real fields (project_nyquist
 // :2044): alternating-mean subtraction along x lines then y lines.
-cudaError_t launch_project_nyquist(double* f, int ncomp, int nx, int ny, cudaStream_t st);
+// From src to dst, which may be the same.
+cudaError_t launch_project_nyquist(const double* src, double* dst, int ncomp, int nx, int ny, cudaStream_t st);
 
 // Zero the k = 0 mode and the excluded Nyquist modes of spectra.
 cudaError_t launch_kspace_mask(double2* f, int ncomp, int N, const unsigned char* excl, int zero_mean,
@@ -262,13 +271,18 @@ struct NormSums {
     double r2[2], map2[2], guess2[2];  // double-double sums
     double max_rel, max_scaled;
 };
+// The sums' `partials` (grid x 8, grid x 28 doubles) and `ticket` (zero between
+// launches) belong to one stream.
 cudaError_t launch_residual_norms(int N, const double* map, const double* guess, double floor_rel,
                                   double atol, double rtol, double* partials, int grid,
-                                  NormSums* out, cudaStream_t st);
+                                  unsigned* ticket, NormSums* out, cudaStream_t st);
 // Gram dots of the Anderson history: dr_i = r[i+1]-r[i] for i < m; sums
 // dr_i.dr_j (i>=j, packed) and dr_i.r[m], in double-double.
 cudaError_t launch_anderson_dots(int N3, const double* const* r, int m, double* partials, int grid,
-                                 double* out, cudaStream_t st);
+                                 unsigned* ticket, double* out, cudaStream_t st);
+// resid = map - guess, hx = guess, hr = resid
+cudaError_t launch_residual_push(int n, const double* map, const double* guess, double* resid, double* hx, double* hr,
+                                 cudaStream_t st);
 // out = x[m] + beta r[m] - sum_j gamma_j (dx_j + beta dr_j)
 cudaError_t launch_anderson_candidate(int N3, const double* const* x, const double* const* r, int m,
                                       double beta, const double* gamma, double* out, cudaStream_t st);
