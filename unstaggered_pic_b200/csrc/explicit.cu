@@ -756,18 +756,57 @@ constexpr int kNSums = 8;  // gauge, gauss, cont, Bz, B, E, rho, J
 // sum_x f^2 = (1/N) sum_k |f_hat|^2 (Parseval; double-double, fixed order), so
 // that no field is transformed back: at 64 x 64 the ten inverse transforms,
 // the reduction over their results and its one-warp finish took 60 of a
-// step's 231 us, this launch takes 14 (512 x 512: 44).  Without pairing (a one-cell
-// axis) a field is the real part of its transform, whose spectrum is
-// (f(k) + conj f(-k)) / 2.  The last block to finish adds the blocks'
-// partials and the push kernel's particle partials in index order and writes
-// the row (page-locked host memory).
+// step's 231 us, this launch takes 11 (512 x 512: 40).  Without pairing (a
+// one-cell axis) a field is the real part of its transform, whose spectrum is
+// (f(k) + conj f(-k)) / 2.  One more block adds the push kernel's particle
+// partials meanwhile; the last block to finish adds the blocks' partials in
+// index order and writes the row (page-locked host memory).  A small grid's
+// launch is one chain of latencies, which the particle sums were a part of
+// while the last block took them (14.4 -> 10.6 us at 32 x 32).
 template <bool PAIRED>
 __global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagArgs a) {
     const int N = a.g.nx * a.g.ny;
+    const int nb = gridDim.x - 1;  // blocks of the field sums
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if ((int)blockIdx.x == nb) {
+        __shared__ double part[kRedThreads / kWarp][kDiagPart];
+        DD kin{0.0, 0.0}, gs{0.0, 0.0};
+        double vmax = 0.0;
+        for (int b = threadIdx.x; b < a.pcount; b += blockDim.x) {
+            const double* p = a.pdiag + (size_t)b * kDiagPart;
+            kin = dd_add_dd(kin, DD{p[0], p[1]});
+            gs = dd_add_dd(gs, DD{p[2], p[3]});
+            vmax = fmax(vmax, p[4]);
+        }
+        kin = warp_sum_dd(kin);
+        gs = warp_sum_dd(gs);
+        vmax = warp_max(vmax);
+        if (lane == 0) {
+            part[warp][0] = kin.hi;
+            part[warp][1] = kin.lo;
+            part[warp][2] = gs.hi;
+            part[warp][3] = gs.lo;
+            part[warp][4] = vmax;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            kin = gs = DD{0.0, 0.0};
+            vmax = 0.0;
+            for (int w = 0; w < kRedThreads / kWarp; ++w) {
+                kin = dd_add_dd(kin, DD{part[w][0], part[w][1]});
+                gs = dd_add_dd(gs, DD{part[w][2], part[w][3]});
+                vmax = fmax(vmax, part[w][4]);
+            }
+            double* o = a.partials + (size_t)nb * 16;
+            o[0] = kin.hi + kin.lo;
+            o[1] = gs.hi + gs.lo;
+            o[2] = vmax;
+        }
+    }
     DD s[kNSums];
 #pragma unroll
     for (int k = 0; k < kNSums; ++k) s[k] = DD{0.0, 0.0};
-    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < N; id += gridDim.x * blockDim.x) {
+    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < N && (int)blockIdx.x < nb; id += nb * blockDim.x) {
         double2 o[kDiagTerms];
         diag_terms<PAIRED>(a, id, o);
         if (!PAIRED) {
@@ -785,7 +824,6 @@ __global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagArgs a) {
         s[3] = dd_add_dd(dd_add_dd(s[3], dd_sq(o[8].x)), dd_sq(o[8].y));
     }
     __shared__ double red[kRedThreads / kWarp][kNSums * 2];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
     for (int k = 0; k < kNSums; ++k) {
         s[k] = warp_sum_dd(s[k]);
@@ -795,7 +833,7 @@ __global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagArgs a) {
         }
     }
     __syncthreads();
-    if (threadIdx.x < kNSums) {
+    if (threadIdx.x < kNSums && (int)blockIdx.x < nb) {
         DD t{0.0, 0.0};
         for (int w = 0; w < kRedThreads / kWarp; ++w)
             t = dd_add_dd(t, DD{red[w][2 * threadIdx.x], red[w][2 * threadIdx.x + 1]});
@@ -812,60 +850,31 @@ __global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagArgs a) {
     __syncthreads();
     if (!last) return;
     __threadfence();
-    // one warp per field sum; the particle sums' partials are shared by all
-    // warps and combined in warp order
-    __shared__ double sums[kNSums][2];
-    __shared__ double part[kRedThreads / kWarp][kDiagPart];
+    // one warp per field sum
+    __shared__ double sums[kNSums];
     {
         DD t{0.0, 0.0};
-        for (int b = lane; b < (int)gridDim.x; b += 32) {
+        for (int b = lane; b < nb; b += 32) {
             const volatile double* p = a.partials + (size_t)b * 16 + 2 * warp;
             t = dd_add_dd(t, DD{p[0], p[1]});
         }
         t = warp_sum_dd(t);
-        if (lane == 0) {
-            sums[warp][0] = t.hi;
-            sums[warp][1] = t.lo;
-        }
-    }
-    DD kin{0.0, 0.0}, gs{0.0, 0.0};
-    double vmax = 0.0;
-    for (int b = threadIdx.x; b < a.pcount; b += blockDim.x) {
-        const double* p = a.pdiag + (size_t)b * kDiagPart;
-        kin = dd_add_dd(kin, DD{p[0], p[1]});
-        gs = dd_add_dd(gs, DD{p[2], p[3]});
-        vmax = fmax(vmax, p[4]);
-    }
-    kin = warp_sum_dd(kin);
-    gs = warp_sum_dd(gs);
-    vmax = warp_max(vmax);
-    if (lane == 0) {
-        part[warp][0] = kin.hi;
-        part[warp][1] = kin.lo;
-        part[warp][2] = gs.hi;
-        part[warp][3] = gs.lo;
-        part[warp][4] = vmax;
+        if (lane == 0) sums[warp] = t.hi + t.lo;
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    kin = gs = DD{0.0, 0.0};
-    vmax = 0.0;
-    for (int w = 0; w < kRedThreads / kWarp; ++w) {
-        kin = dd_add_dd(kin, DD{part[w][0], part[w][1]});
-        gs = dd_add_dd(gs, DD{part[w][2], part[w][3]});
-        vmax = fmax(vmax, part[w][4]);
-    }
     const double invN = 1.0 / (double)N;
-    auto tot = [&](int k) { return (sums[k][0] + sums[k][1]) * invN; };  // sum over the nodes
+    auto tot = [&](int k) { return sums[k] * invN; };  // sum over the nodes
     double* r = a.row;
-    for (int k = 0; k < kNSums; ++k) r[k] = sqrt(tot(k) * invN);
+    if (threadIdx.x < kNSums) r[threadIdx.x] = sqrt(tot(threadIdx.x) * invN);
+    if (threadIdx.x != kWarp) return;
+    const volatile double* p = a.partials + (size_t)nb * 16;
+    const double kinetic = p[0], gsum = p[1], vmax = p[2];
     const double field = 0.5 * a.eps0 * (tot(5) * a.dA) + 0.5 / a.mu0 * (tot(4) * a.dA);
-    const double kinetic = kin.hi + kin.lo;
     r[8] = field;
     r[9] = kinetic;
     r[10] = field + kinetic;
     r[11] = vmax;
-    r[12] = a.np > 0 ? (gs.hi + gs.lo) / (double)a.np : 0.0;
+    r[12] = a.np > 0 ? gsum / (double)a.np : 0.0;
 }
 
 __global__ void poisson_kspace_kernel(int N, const double* k2, const double2* rh, double eps0,
@@ -1107,7 +1116,7 @@ cudaError_t launch_diag_field(const DiagArgs& a, int which, double2* out, cudaSt
 
 cudaError_t launch_diag_reduce(const DiagArgs& a, cudaStream_t st) {
     long blocks = ((long)a.g.nx * a.g.ny + kRedThreads - 1) / kRedThreads;
-    const int grid = (int)(blocks < a.max_blocks ? blocks : a.max_blocks);
+    const int grid = 1 + (int)(blocks < a.max_blocks - 1 ? blocks : a.max_blocks - 1);
     if (paired_grid(a.g)) diag_reduce_kernel<true><<<grid, kRedThreads, 0, st>>>(a);
     else diag_reduce_kernel<false><<<grid, kRedThreads, 0, st>>>(a);
     count_launches(1);
