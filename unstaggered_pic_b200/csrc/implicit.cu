@@ -17,6 +17,7 @@
 
 #include "deposit.cuh"
 #include "implicit_kernels.h"
+#include "orbit_knots.h"
 #include "upic_common.cuh"
 
 namespace upic {
@@ -192,7 +193,6 @@ UPIC_D int breakpoints(const Geo& g, double x0, double y0, double dxx, double dx
     b[nb++] = 0.0;
     b[nb++] = 1.0;
     if (split) {
-        const double tol = 1.0e-13;
         const double offset = 0.5 * (double)(ORDER - 1);
 #pragma unroll
         for (int d = 0; d < 2; ++d) {
@@ -201,18 +201,7 @@ UPIC_D int breakpoints(const Geo& g, double x0, double y0, double dxx, double dx
             const double u0 = (wrap1(d == 0 ? x0 : y0, L) + 0.5 * L) / h;
             const double du = (d == 0 ? dxx : dxy) / h;
             if (fabs(du) < 1.0e-300) continue;
-            const double a0 = u0 - offset;
-            const double a1 = a0 + du;
-            const double lo = fmin(a0, a1), hi = fmax(a0, a1);
-            const long long first = (long long)floor(lo) + 1;
-            const long long last = (long long)ceil(hi) - 1;
-            for (long long m = first; m <= last; ++m) {
-                const double s = ((double)m - a0) / du;
-                if (s > tol && s < 1.0 - tol) {
-                    if (nb >= kMaxBreaks) return -1;
-                    b[nb++] = s;
-                }
-            }
+            if (!axis_breaks(u0 - offset, du, b, nb)) return -1;
         }
         // insertion sort, then drop near-duplicates
         for (int i = 1; i < nb; ++i) {
@@ -629,60 +618,6 @@ template <int R>
 UPIC_D double taylor(const double (&w)[R + 1], const double (&G)[R][R + 1], double d, int i, int a) {
     return i == 0 ? w[a] : d * (1.0 / (double)i) * G[i - 1][a];
 }
-
-// The next knot (integer) that an orbit u0 + s du passes along one axis after
-// fraction s (2: none in (0, 1)); s = 0 for the first
-// (path_breakpoints_for_particle :2555).  Only s is kept between calls: the
-// knot passed at s is the integer nearest u0 + s du.
-UPIC_D double next_knot(double u0, double du, double s) {
-    const double step = du > 0.0 ? 1.0 : -1.0;
-    double m = s > 0.0 ? rint(fma(s, du, u0)) + step : du > 0.0 ? floor(u0) + 1.0 : ceil(u0) - 1.0;
-    for (;;) {
-        if (fabs(du) < 1.0e-300 || !((m - (u0 + du)) * step < 0.0)) return 2.0;
-        s = (m - u0) / du;
-        if (s > 1.0e-13) return s < 1.0 - 1.0e-13 ? s : 2.0;
-        m += step;
-    }
-}
-
-// The segments of an orbit between its knots, one after the other; knots
-// closer than 1e-12 count once, and more than kMaxBreaks end points fail.
-struct KnotWalk {
-    double sx, sy, prev;
-    int nb;  // end points so far; 0 when no segment is left, -1 when there were too many
-    UPIC_D void init(double ux, double uy, double dux, double duy) {
-        sx = next_knot(ux, dux, 0.0);
-        sy = next_knot(uy, duy, 0.0);
-        prev = 0.0;
-        nb = 2;
-    }
-    UPIC_D bool more() const { return nb > 0; }
-    UPIC_D bool next(double ux, double uy, double dux, double duy, double& sa, double& sb) {
-        while (nb > 0) {
-            double s = fmin(sx, sy);
-            if (s < 1.0) {
-                const bool ex = sx == s, ey = sy == s;
-                if (ex) sx = next_knot(ux, dux, s);
-                if (ey) sy = next_knot(uy, duy, s);
-                nb += (ex ? 1 : 0) + (ey ? 1 : 0);
-                if (nb > kMaxBreaks) {
-                    nb = -1;
-                    return false;
-                }
-            } else {
-                s = 1.0;
-                nb = 0;
-            }
-            if (s - prev > 1.0e-12) {
-                sa = prev;
-                sb = s;
-                prev = s;
-                return true;
-            }
-        }
-        return false;
-    }
-};
 
 // Grid coordinate less the stencil offset: the stencil of a point starts at
 // node floor of it, its knots are the integers.

@@ -15,9 +15,6 @@ constexpr int kIRecGpm = 0;
 constexpr int kIRecAn = 2;
 constexpr int kIRecAe = 5;
 constexpr int kMaxQuad = 32;
-// Knot crossings per particle orbit that the device kernel can hold
-// (breakpoints of both axes plus the two ends).
-constexpr int kMaxBreaks = 40;
 
 // Failure reasons of the per-particle local fixed point
 // (LocalParticleFailureReason, Project3/ec_pic_nyquist_projected.cpp:204-211).
