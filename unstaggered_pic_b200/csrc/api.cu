@@ -438,34 +438,7 @@ PushArgs push_args(upic_ctx* c, const ParticleSoA& p, long np, bool uniform) {
     return a;
 }
 
-// Fields are paired in the transforms of the FP64 form on grids of at least
-// two cells along each axis (explicit.cu).  The mixed form transforms them one
-// by one: a different rounding of the FP64 spectra would move single FP32
-// node records by an ulp, and the particles with them.
-KGrid kgrid(const upic_ctx* c) {
-    return KGrid{c->nx, c->ny, c->lny, c->nx > 1 && c->ny > 1 && !c->mixed, c->d_kx, c->d_ky, c->d_k2};
-}
-
-// Transforms of the deposited fields and of the gathered ones (explicit.cu
-// bdf_kspace_kernel): pairs of real fields, or one by one on a grid one cell
-// high or wide.  Returns their number.
-int current_map(const upic_ctx* c, FftMap& m) {
-    m = fft_identity_map(3);
-    if (!paired_grid(kgrid(c))) return 3;
-    m.im[0] = 1;
-    m.re[1] = 2;
-    return 2;
-}
-int gather_map(const upic_ctx* c, FftMap& m) {
-    m = fft_identity_map(kGF);
-    if (!paired_grid(kgrid(c))) return kGF;
-    const signed char re[6] = {0, 2, 3, 5, 7, 9}, im[6] = {1, -1, 4, 6, 8, 10};
-    for (int k = 0; k < 6; ++k) {
-        m.re[k] = re[k];
-        m.im[k] = im[k];
-    }
-    return 6;
-}
+KGrid kgrid(const upic_ctx* c) { return KGrid{c->nx, c->ny, c->lny, c->d_kx, c->d_ky, c->d_k2}; }
 
 // J^n (and rho^n with `charge`) of the accumulators and their spectra.
 int transform_deposit(upic_ctx* c, bool charge) {
@@ -477,21 +450,8 @@ int transform_deposit(upic_ctx* c, bool charge) {
     in.n0 = c->cfg.n0;
     in.bg = c->d_bg;
     in.single = c->mixed ? 1 : 0;
-    FftMap m;
-    int n = current_map(c, m);
-    if (charge) {
-        // the charge goes to slot 3 of the spectra: transform 2 when paired
-        m.re[n] = 3;
-        m.im[n] = -1;
-        ++n;
-    }
-    UPIC_CUDA(c, fft2d_from_acc(c->plan, c->d_spec, n, m, in, c->st));
+    UPIC_CUDA(c, fft2d_from_acc(c->plan, c->d_spec, charge ? 4 : 3, in, c->st));
     return 0;
-}
-
-// Spectrum of the naive charge after transform_deposit(c, true).
-const double2* charge_spectrum(const upic_ctx* c) {
-    return c->d_spec + (paired_grid(kgrid(c)) ? 2 : 3) * (size_t)c->N;
 }
 
 // Diagnostics row of the current spectra (hist slot_new with derivatives
@@ -1289,9 +1249,7 @@ int upic_init_fields(upic_ctx* c, double* diag_row) {
     UPIC_CUDA(c, launch_fill_hist(H + 4 * fs, kHistSlots, N, sp + 3 * (size_t)N, c->st));
     c->head = 0;
     // J0 spectra for the step-0 diagnostics
-    FftMap jmap;
-    const int jn = current_map(c, jmap);
-    UPIC_CUDA(c, fft2d_mapped(c->plan, sp, jn, jmap, 0, c->st, c->d_J, 0, nullptr, 0, 0));
+    UPIC_CUDA(c, fft2d_batched(c->plan, sp, 3, 0, c->st, c->d_J));
     if (diag_row) {
         const double a1[3] = {1.0, -1.0, 0.0};
         if ((rc = run_diag(c, c->head, c->head, 2, a1, c->h_row))) return rc;
@@ -1357,7 +1315,7 @@ int explicit_advance(upic_ctx* c, int nsteps, int diag_stride, double* diag, boo
         KspaceArgs k{};
         k.g = kgrid(c);
         k.Jhat = sp;
-        k.rho_dep = naive ? charge_spectrum(c) : nullptr;
+        k.rho_dep = naive ? sp + 3 * (size_t)N : nullptr;
         k.hist = c->d_hist;
         k.R = kHistSlots;
         k.head = c->head;
@@ -1371,10 +1329,10 @@ int explicit_advance(upic_ctx* c, int nsteps, int diag_stride, double* diag, boo
         k.conserving = naive ? 0 : 1;
         k.gspec = sp + 4 * (size_t)N;
         UPIC_CUDA(c, launch_bdf_kspace(k, c->st));
-        FftMap gmap;
-        const int gn = gather_map(c, gmap);
-        UPIC_CUDA(c, fft2d_mapped(c->plan, k.gspec, gn, gmap, 1, c->st, nullptr, c->mixed ? 3 : 2,
-                                  c->mixed ? static_cast<void*>(c->d_gf32) : static_cast<void*>(c->d_gf), kGFStride, 0));
+        if (c->mixed)
+            UPIC_CUDA(c, fft2d_batched(c->plan, k.gspec, kGF, 1, c->st, nullptr, 3, c->d_gf32, kGFStride, 0));
+        else
+            UPIC_CUDA(c, fft2d_batched(c->plan, k.gspec, kGF, 1, c->st, nullptr, 2, c->d_gf, kGFStride, 0));
         if (c->np > 0) {
             if ((rc = launch_push(c, kModePush, grid_ncomp(c), c->P[c->cur], c->np, c->uniform_qm, c->sw,
                                   c->d_pdiag)))

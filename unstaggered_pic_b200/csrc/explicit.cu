@@ -568,20 +568,6 @@ UPIC_D double2 cscale(double s, double2 a) { return make_double2(s * a.x, s * a.
 UPIC_D double2 cik(double k, double2 z) { return make_double2(-k * z.y, k * z.x); }
 
 // ---- k-space step -----------------------------------------------------------
-// Real fields travel in pairs through the transforms: spectrum Z = F + i G of
-// two real fields gives F(k) = (Z(k) + conj Z(-k)) / 2 and
-// G(k) = (Z(k) - conj Z(-k)) / 2i, and the inverse transform of F + i G has F
-// in its real and G in its imaginary part.  A grid one cell high or wide is
-// not paired: its wave number there is that of mode -1
-// (spectral_pic_part3.cpp:320-330), so a derivative's spectrum is not that of
-// a real field and only the real part of each transform is wanted.
-UPIC_D double2 pair_re(double2 z, double2 m) { return make_double2(0.5 * (z.x + m.x), 0.5 * (z.y - m.y)); }
-UPIC_D double2 pair_im(double2 z, double2 m) { return make_double2(0.5 * (z.y + m.y), 0.5 * (m.x - z.x)); }
-// (i kx - ky) z: the pair of i kx z and i ky z
-UPIC_D double2 cgrad(double kx, double ky, double2 z) {
-    return make_double2(-kx * z.y - ky * z.x, kx * z.x - ky * z.y);
-}
-
 // Node (i, j)'s wave numbers from the axes' own rows and columns of the
 // grid-sized tables (16 B per node less to read): kx depends on i alone, ky
 // on j, and k2 = k2(i, 0) + k2(0, j) is the sum the host rounds.
@@ -594,7 +580,6 @@ UPIC_D double2 cmul_add(double s, double2 h, double2 u) {
 
 struct Wave {
     double kx, ky, k2;
-    int mirror;  // node of -k
 };
 UPIC_D Wave wave_at(const KGrid& g, int id) {
     const int i = id >> g.lny, j = id & (g.ny - 1);
@@ -602,31 +587,23 @@ UPIC_D Wave wave_at(const KGrid& g, int id) {
     w.kx = __ldg(g.kx + (i << g.lny));
     w.ky = __ldg(g.ky + j);
     w.k2 = g.nx > 1 && g.ny > 1 ? __dadd_rn(__ldg(g.k2 + (i << g.lny)), __ldg(g.k2 + j)) : __ldg(g.k2 + id);
-    w.mirror = (((g.nx - i) & (g.nx - 1)) << g.lny) + ((g.ny - j) & (g.ny - 1));
     return w;
 }
-
-// Current spectra of mode id.  Paired: transform 0 carries (Jx, Jy), 1 Jz.
-template <bool PAIRED>
-UPIC_D void current_at(const double2* __restrict__ Jhat, int N, int id, int mirror, double2* J) {
-    if (PAIRED) {
-        const double2 z = Jhat[id], m = Jhat[mirror];
-        J[0] = pair_re(z, m);
-        J[1] = pair_im(z, m);
-        J[2] = pair_re(Jhat[N + id], Jhat[N + mirror]);
-    } else {
-        for (int c = 0; c < 3; ++c) J[c] = Jhat[(size_t)c * N + id];
-    }
+// Node of -k
+UPIC_D int mirror_node(const KGrid& g, int id) {
+    const int i = id >> g.lny, j = id & (g.ny - 1);
+    return (((g.nx - i) & (g.nx - 1)) << g.lny) + ((g.ny - j) & (g.ny - 1));
 }
 
 // k-space BDF step: continuity / naive charge, BDF Helmholtz solves for phi
 // and A (spectral_pic_part3.cpp:829-880, 1147-1164), spectra of the eleven
-// gathered fields (:1166-1168), in six transforms when paired: (Ax, Ay), Az,
-// grad phi, grad Ax, grad Ay, grad Az (fields that vanish together share a
-// transform, so a zero component stays exactly zero).  NA: BDF coefficients
-// (2 or 3; the Helmholtz solves take 2 NA - 1), which fixes the number of
-// history slots, so that all loads of a mode are in flight together.
-template <int NA, bool PAIRED>
+// gathered fields (:1166-1168).  Every field has a transform of its own: two
+// real fields that share a complex one (as its real and imaginary parts) both
+// take the rounding of the larger, and a field that is zero does not stay
+// zero.  NA: BDF coefficients (2 or 3; the Helmholtz solves take 2 NA - 1),
+// which fixes the number of history slots, so that all loads of a mode are in
+// flight together.
+template <int NA>
 __global__ void __launch_bounds__(128) bdf_kspace_kernel(KspaceArgs a) {
     constexpr int NB = 2 * NA - 1;
     const int N = a.g.nx * a.g.ny;
@@ -640,7 +617,8 @@ __global__ void __launch_bounds__(128) bdf_kspace_kernel(KspaceArgs a) {
         const Wave w = wave_at(a.g, id);
         const double kx = w.kx, ky = w.ky;
         double2 J[3];
-        current_at<PAIRED>(a.Jhat, N, id, w.mirror, J);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) J[c] = a.Jhat[(size_t)c * N + id];
         double2 H[4][NB - 1];
 #pragma unroll
         for (int f = 0; f < 4; ++f)
@@ -655,7 +633,7 @@ __global__ void __launch_bounds__(128) bdf_kspace_kernel(KspaceArgs a) {
             const double2 num = cmul_add(a.dt, div, hs);
             rho_new = make_double2(-num.x / a.a[0], -num.y / a.a[0]);
         } else {
-            rho_new = PAIRED ? pair_re(a.rho_dep[id], a.rho_dep[w.mirror]) : a.rho_dep[id];
+            rho_new = a.rho_dep[id];
         }
         const double denom = scale * a.b[0] + w.k2;
         // (b0 s + k^2) u = source - s sum b_l u^{n+1-l}: phi from rho / eps0, A from mu0 J
@@ -673,19 +651,12 @@ __global__ void __launch_bounds__(128) bdf_kspace_kernel(KspaceArgs a) {
         }
         a.hist[4 * FS + (size_t)snew * N + id] = rho_new;
         double2* g = a.gspec;
-        if (PAIRED) {
-            g[id] = make_double2(u[1].x - u[2].y, u[1].y + u[2].x);
-            g[(size_t)N + id] = u[3];
 #pragma unroll
-            for (int f = 0; f < 4; ++f) g[(2 + f) * (size_t)N + id] = cgrad(kx, ky, u[f]);
-        } else {
+        for (int c = 0; c < 3; ++c) g[(size_t)c * N + id] = u[1 + c];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) g[(size_t)c * N + id] = u[1 + c];
-#pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                g[(3 + 2 * f) * (size_t)N + id] = cik(kx, u[f]);
-                g[(4 + 2 * f) * (size_t)N + id] = cik(ky, u[f]);
-            }
+        for (int f = 0; f < 4; ++f) {
+            g[(3 + 2 * f) * (size_t)N + id] = cik(kx, u[f]);
+            g[(4 + 2 * f) * (size_t)N + id] = cik(ky, u[f]);
         }
     }
 }
@@ -696,12 +667,21 @@ __global__ void __launch_bounds__(128) bdf_kspace_kernel(KspaceArgs a) {
 // derivatives of the histories; J (3) after them.
 constexpr int kDiagTerms = 13;
 
-template <bool PAIRED>
+// HERM: of the modes' Hermitian parts (f(k) + conj f(-k)) / 2, the spectra of
+// the real fields.
+template <bool HERM>
 UPIC_D void diag_terms(const DiagArgs& a, int id, double2* o) {
     const int N = a.g.nx * a.g.ny;
     const Wave w = wave_at(a.g, id);
     const double kx = w.kx, ky = w.ky;
-    auto H = [&](int field, int slot) -> double2 { return a.hist[((size_t)field * a.R + slot) * N + id]; };
+    const int mir = HERM ? mirror_node(a.g, id) : id;
+    auto val = [&](const double2* __restrict__ f) -> double2 {
+        const double2 z = f[id];
+        if (!HERM) return z;
+        const double2 m = f[mir];
+        return make_double2(0.5 * (z.x + m.x), 0.5 * (z.y - m.y));
+    };
+    auto H = [&](int field, int slot) -> double2 { return val(a.hist + ((size_t)field * a.R + slot) * N); };
     auto ddt = [&](int field) -> double2 {
         double2 r = cscale(a.a[0], H(field, a.slot_new));
         for (int l = 1; l < a.na; ++l) {
@@ -711,7 +691,8 @@ UPIC_D void diag_terms(const DiagArgs& a, int id, double2* o) {
         return make_double2(r.x / a.dt, r.y / a.dt);
     };
     double2* J = o + 10;
-    current_at<PAIRED>(a.Jhat, N, id, w.mirror, J);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) J[c] = val(a.Jhat + (size_t)c * N);
     const double2 phi = H(0, a.slot_new);
     const double2 Ax = H(1, a.slot_new), Ay = H(2, a.slot_new), Az = H(3, a.slot_new);
     const double2 rho = H(4, a.slot_new);
@@ -735,12 +716,11 @@ UPIC_D void diag_terms(const DiagArgs& a, int id, double2* o) {
 }
 
 // Spectrum of one diagnostics field (upic_get_field).
-template <bool PAIRED>
 __global__ void diag_field_kernel(DiagArgs a, int which, double2* out) {
     const int N = a.g.nx * a.g.ny;
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < N; id += gridDim.x * blockDim.x) {
         double2 o[kDiagTerms];
-        diag_terms<PAIRED>(a, id, o);
+        diag_terms<false>(a, id, o);
         double2 r = o[0];
 #pragma unroll
         for (int k = 1; k < 10; ++k)
@@ -756,14 +736,19 @@ constexpr int kNSums = 8;  // gauge, gauss, cont, Bz, B, E, rho, J
 // sum_x f^2 = (1/N) sum_k |f_hat|^2 (Parseval; double-double, fixed order), so
 // that no field is transformed back: at 64 x 64 the ten inverse transforms,
 // the reduction over their results and its one-warp finish took 60 of a
-// step's 231 us, this launch takes 11 (512 x 512: 40).  Without pairing (a
-// one-cell axis) a field is the real part of its transform, whose spectrum is
-// (f(k) + conj f(-k)) / 2.  One more block adds the push kernel's particle
-// partials meanwhile; the last block to finish adds the blocks' partials in
-// index order and writes the row (page-locked host memory).  A small grid's
-// launch is one chain of latencies, which the particle sums were a part of
-// while the last block took them (14.4 -> 10.6 us at 32 x 32).
-template <bool PAIRED>
+// step's 231 us, this launch takes 11 (512 x 512: 40).  A field is the real
+// part of its transform, whose spectrum is (f(k) + conj f(-k)) / 2.  That part
+// is taken of the histories and currents that the fields are formed from
+// (taking it of the fields costs 4.7 us more a row, 32 x 32 and 64 x 64); of
+// the fields themselves on a grid one cell high or wide, where the wave number
+// is that of mode -1 at both k and -k (spectral_pic_part3.cpp:320-330), so
+// that a derivative of a real field is not one.  One more block adds the push
+// kernel's particle partials meanwhile; the last block to finish adds the
+// blocks' partials in index order and writes the row (page-locked host
+// memory).  A small grid's launch is one chain of latencies, which the
+// particle sums were a part of while the last block took them (14.4 -> 10.6 us
+// at 32 x 32).
+template <bool ONE_CELL>
 __global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagArgs a) {
     const int N = a.g.nx * a.g.ny;
     const int nb = gridDim.x - 1;  // blocks of the field sums
@@ -808,12 +793,12 @@ __global__ void __launch_bounds__(kRedThreads) diag_reduce_kernel(DiagArgs a) {
     for (int k = 0; k < kNSums; ++k) s[k] = DD{0.0, 0.0};
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < N && (int)blockIdx.x < nb; id += nb * blockDim.x) {
         double2 o[kDiagTerms];
-        diag_terms<PAIRED>(a, id, o);
-        if (!PAIRED) {
+        diag_terms<!ONE_CELL>(a, id, o);
+        if (ONE_CELL) {
             double2 m[kDiagTerms];
-            diag_terms<PAIRED>(a, wave_at(a.g, id).mirror, m);
+            diag_terms<false>(a, mirror_node(a.g, id), m);
 #pragma unroll
-            for (int k = 0; k < kDiagTerms; ++k) o[k] = pair_re(o[k], m[k]);
+            for (int k = 0; k < kDiagTerms; ++k) o[k] = make_double2(0.5 * (o[k].x + m[k].x), 0.5 * (o[k].y - m[k].y));
         }
         constexpr int which[kDiagTerms] = {0, 5, 5, 5, 1, 2, 4, 4, 4, 6, 7, 7, 7};
 #pragma unroll
@@ -1095,21 +1080,15 @@ cudaError_t launch_convert_acc(unsigned long long* acc, int N, const double* sca
 
 cudaError_t launch_bdf_kspace(const KspaceArgs& a, cudaStream_t st) {
     const int grid = grid_for((long)a.g.nx * a.g.ny, 128);
-    if (a.na == 3) {
-        if (paired_grid(a.g)) bdf_kspace_kernel<3, true><<<grid, 128, 0, st>>>(a);
-        else bdf_kspace_kernel<3, false><<<grid, 128, 0, st>>>(a);
-    } else {
-        if (paired_grid(a.g)) bdf_kspace_kernel<2, true><<<grid, 128, 0, st>>>(a);
-        else bdf_kspace_kernel<2, false><<<grid, 128, 0, st>>>(a);
-    }
+    if (a.na == 3) bdf_kspace_kernel<3><<<grid, 128, 0, st>>>(a);
+    else bdf_kspace_kernel<2><<<grid, 128, 0, st>>>(a);
     count_launches(1);
     return cudaGetLastError();
 }
 
 cudaError_t launch_diag_field(const DiagArgs& a, int which, double2* out, cudaStream_t st) {
     const int grid = grid_for((long)a.g.nx * a.g.ny, 256);
-    if (paired_grid(a.g)) diag_field_kernel<true><<<grid, 256, 0, st>>>(a, which, out);
-    else diag_field_kernel<false><<<grid, 256, 0, st>>>(a, which, out);
+    diag_field_kernel<<<grid, 256, 0, st>>>(a, which, out);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -1117,8 +1096,8 @@ cudaError_t launch_diag_field(const DiagArgs& a, int which, double2* out, cudaSt
 cudaError_t launch_diag_reduce(const DiagArgs& a, cudaStream_t st) {
     long blocks = ((long)a.g.nx * a.g.ny + kRedThreads - 1) / kRedThreads;
     const int grid = 1 + (int)(blocks < a.max_blocks - 1 ? blocks : a.max_blocks - 1);
-    if (paired_grid(a.g)) diag_reduce_kernel<true><<<grid, kRedThreads, 0, st>>>(a);
-    else diag_reduce_kernel<false><<<grid, kRedThreads, 0, st>>>(a);
+    if (a.g.nx > 1 && a.g.ny > 1) diag_reduce_kernel<false><<<grid, kRedThreads, 0, st>>>(a);
+    else diag_reduce_kernel<true><<<grid, kRedThreads, 0, st>>>(a);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -142,10 +142,9 @@ UPIC_D void line_passes(double2* v, int t, double2* sm, const double2* __restric
 
 struct FftArgs {
     double2* data;
-    int nlines;               // y pass: transforms * nx; x pass: transforms
+    int nlines;               // y pass: components * nx; x pass: components
     int lognx, logny;
     const double2* tw;
-    FftMap map;
     const double* rin;        // forward: real planar input or null
     int out_mode;             // inverse
     void* rout;
@@ -200,26 +199,17 @@ __global__ void __launch_bounds__(Shape<LOGN>::ythreads) fft_y_kernel(FftArgs a)
 #pragma unroll
     for (int e = 0; e < S::E; ++e) v[e] = make_double2(0.0, 0.0);
     if (on) {
-        const int cr = a.map.re[p], ci = a.map.im[p];
         if constexpr (PASS == kForwardAcc || PASS == kForwardAcc1) {
             constexpr bool single = PASS == kForwardAcc1;
             const size_t node = (size_t)row * S::n + t;
-            double re[S::E], im[S::E];
-            take_acc<single>(a.acc, cr, N, node, S::T, re);
+            double re[S::E];
+            take_acc<single>(a.acc, p, N, node, S::T, re);
 #pragma unroll
-            for (int e = 0; e < S::E; ++e) im[e] = 0.0;
-            if (ci >= 0) take_acc<single>(a.acc, ci, N, node, S::T, im);
-#pragma unroll
-            for (int e = 0; e < S::E; ++e) v[e] = make_double2(re[e], im[e]);
+            for (int e = 0; e < S::E; ++e) v[e].x = re[e];
         } else if (!INV && a.rin) {
-            const double* r = a.rin + cr * N + (size_t)row * S::n;
+            const double* r = a.rin + (size_t)line * S::n;
 #pragma unroll
             for (int e = 0; e < S::E; ++e) v[e].x = r[t + e * S::T];
-            if (ci >= 0) {
-                const double* q = a.rin + ci * N + (size_t)row * S::n;
-#pragma unroll
-                for (int e = 0; e < S::E; ++e) v[e].y = q[t + e * S::T];
-            }
         } else {
 #pragma unroll
             for (int e = 0; e < S::E; ++e) v[e] = d[t + e * S::T];
@@ -258,7 +248,6 @@ __global__ void __launch_bounds__(Shape<LOGN>::xthreads) fft_x_kernel(FftArgs a,
     line_passes<LOGN, 0, INV>(
         v, t, smem, a.tw, [logcols, col](int i) { return (swizzle(i) << logcols) + col; }, [] { __syncthreads(); });
     constexpr double sc = INV ? 1.0 / (double)S::n : 1.0;
-    const int cr = a.map.re[p], ci = a.map.im[p];
 #pragma unroll
     for (int e = 0; e < S::E; ++e) {
         const size_t at = (size_t)(t + e * S::T) << a.logny, node = at + j;
@@ -266,17 +255,11 @@ __global__ void __launch_bounds__(Shape<LOGN>::xthreads) fft_x_kernel(FftArgs a,
         if (!INV || a.out_mode == 0) {
             d[at] = make_double2(re, im);
         } else if (a.out_mode == 1) {
-            double* o = static_cast<double*>(a.rout);
-            o[cr * N + node] = re;
-            if (ci >= 0) o[ci * N + node] = im;
+            static_cast<double*>(a.rout)[p * N + node] = re;
         } else if (a.out_mode == 2) {
-            double* o = static_cast<double*>(a.rout) + node * a.rec_stride + a.comp_offset;
-            o[cr] = re;
-            if (ci >= 0) o[ci] = im;
+            static_cast<double*>(a.rout)[node * a.rec_stride + a.comp_offset + p] = re;
         } else {
-            float* o = static_cast<float*>(a.rout) + node * a.rec_stride + a.comp_offset;
-            o[cr] = (float)re;
-            if (ci >= 0) o[ci] = (float)im;
+            static_cast<float*>(a.rout)[node * a.rec_stride + a.comp_offset + p] = (float)re;
         }
     }
 }
@@ -360,27 +343,18 @@ void run_x(int logn, const FftArgs& a, bool inverse, cudaStream_t st) {
 
 }  // namespace
 
-FftMap fft_identity_map(int ncomp) {
-    FftMap m{};
-    for (int c = 0; c < ncomp && c < kFftMaxTransforms; ++c) {
-        m.re[c] = (signed char)c;
-        m.im[c] = -1;
-    }
-    return m;
-}
-
 namespace {
 
 // Both passes of `a` (its plan-dependent members are filled in here).
-cudaError_t run_2d(const FftPlan& p, FftArgs a, int ntransforms, int pass, cudaStream_t st) {
+cudaError_t run_2d(const FftPlan& p, FftArgs a, int ncomp, int pass, cudaStream_t st) {
     const int lx = ilog2(p.nx), ly = ilog2(p.ny);
-    if (ntransforms > kFftMaxTransforms || lx > kFftMaxLog || ly > kFftMaxLog) return cudaErrorInvalidValue;
+    if (lx > kFftMaxLog || ly > kFftMaxLog) return cudaErrorInvalidValue;
     a.lognx = lx;
     a.logny = ly;
     FftArgs x = a;
-    a.nlines = ntransforms << lx;
+    a.nlines = ncomp << lx;
     a.tw = p.tw_y;
-    x.nlines = ntransforms;
+    x.nlines = ncomp;
     x.tw = p.tw_x;
     run_y(ly, a, pass, st);
     run_x(lx, x, pass == kInverse, st);
@@ -390,34 +364,23 @@ cudaError_t run_2d(const FftPlan& p, FftArgs a, int ntransforms, int pass, cudaS
 
 }  // namespace
 
-cudaError_t fft2d_mapped(const FftPlan& p, double2* data, int ntransforms, const FftMap& map, int inverse,
-                         cudaStream_t st, const double* real_in, int out_mode, void* real_out, int rec_stride,
-                         int comp_offset) {
+cudaError_t fft2d_batched(const FftPlan& p, double2* data, int ncomp, int inverse, cudaStream_t st,
+                          const double* real_in, int out_mode, void* real_out, int rec_stride, int comp_offset) {
     FftArgs a{};
     a.data = data;
-    a.map = map;
     a.rin = inverse ? nullptr : real_in;
     a.out_mode = out_mode;
     a.rout = real_out;
     a.rec_stride = rec_stride;
     a.comp_offset = comp_offset;
-    return run_2d(p, a, ntransforms, inverse ? kInverse : kForward, st);
+    return run_2d(p, a, ncomp, inverse ? kInverse : kForward, st);
 }
 
-cudaError_t fft2d_from_acc(const FftPlan& p, double2* data, int ntransforms, const FftMap& map, const FftAccIn& acc,
-                           cudaStream_t st) {
+cudaError_t fft2d_from_acc(const FftPlan& p, double2* data, int ncomp, const FftAccIn& acc, cudaStream_t st) {
     FftArgs a{};
     a.data = data;
-    a.map = map;
     a.acc = acc;
-    return run_2d(p, a, ntransforms, acc.single ? kForwardAcc1 : kForwardAcc, st);
-}
-
-cudaError_t fft2d_batched(const FftPlan& p, double2* data, int ncomp, int inverse, cudaStream_t st,
-                          const double* real_in, int out_mode, double* real_out, int rec_stride,
-                          int comp_offset) {
-    return fft2d_mapped(p, data, ncomp, fft_identity_map(ncomp), inverse, st, real_in, out_mode, real_out,
-                        rec_stride, comp_offset);
+    return run_2d(p, a, ncomp, acc.single ? kForwardAcc1 : kForwardAcc, st);
 }
 
 cudaError_t fft_configure_smem() { return raise_one<kFftMaxLog>(); }

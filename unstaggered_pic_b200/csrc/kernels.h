@@ -24,23 +24,15 @@ struct FftPlan {
     const double2* tw_y;  // exp(-2 pi i m / ny), m < ny
 };
 
-// Real components of a batch of transforms: transform p carries component
-// re[p] in its real part and im[p] (-1: none) in its imaginary part.
-constexpr int kFftMaxTransforms = 16;
-struct FftMap {
-    signed char re[kFftMaxTransforms], im[kFftMaxTransforms];
-};
-FftMap fft_identity_map(int ncomp);  // component p alone in transform p
-
-// 2D transforms of stacked complex grids (stride nx*ny).  Forward with
-// real_in != NULL: the input is the components of the real planar array
-// real_in that `map` names, the result lands in data.  Inverse, out_mode 0:
-// complex result in data; 1: the components to real_out planar (stride
-// nx*ny); 2: to interleaved records real_out[node*rec_stride + comp_offset +
-// component]; 3: the same records as floats (float storage).
-cudaError_t fft2d_mapped(const FftPlan& p, double2* data, int ntransforms, const FftMap& map, int inverse,
-                         cudaStream_t st, const double* real_in, int out_mode, void* real_out, int rec_stride,
-                         int comp_offset);
+// 2D transforms of ncomp stacked complex grids (stride nx*ny).  Forward with
+// real_in != NULL: the input is the real planar array real_in (imaginary part
+// 0), the result lands in data.  Inverse, out_mode 0: complex result in data;
+// 1: real parts to real_out planar (stride nx*ny); 2: to interleaved records
+// real_out[node*rec_stride + comp_offset + component]; 3: the same records as
+// floats (float storage).
+cudaError_t fft2d_batched(const FftPlan& p, double2* data, int ncomp, int inverse, cudaStream_t st,
+                          const double* real_in = nullptr, int out_mode = 0, void* real_out = nullptr,
+                          int rec_stride = 0, int comp_offset = 0);
 // Forward transforms straight from the deposit accumulators: component c is
 // J_c (0..2) or rho (3), converted, stored to J / rho and cleared on the way
 // (launch_convert_acc, or launch_convert_acc1 with `single`).
@@ -52,13 +44,7 @@ struct FftAccIn {
     const double* bg;
     int single;
 };
-cudaError_t fft2d_from_acc(const FftPlan& p, double2* data, int ntransforms, const FftMap& map, const FftAccIn& acc,
-                           cudaStream_t st);
-// The same with every component alone in its transform (at most
-// kFftMaxTransforms).
-cudaError_t fft2d_batched(const FftPlan& p, double2* data, int ncomp, int inverse, cudaStream_t st,
-                          const double* real_in = nullptr, int out_mode = 0,
-                          double* real_out = nullptr, int rec_stride = 0, int comp_offset = 0);
+cudaError_t fft2d_from_acc(const FftPlan& p, double2* data, int ncomp, const FftAccIn& acc, cudaStream_t st);
 cudaError_t fft_configure_smem();
 
 // ---------------------------------------------------------------------------
@@ -247,16 +233,13 @@ cudaError_t launch_convert_acc(unsigned long long* acc, int N, const double* sca
 // Grid and wave-number tables (nx x ny each) of the k-space kernels.
 struct KGrid {
     int nx, ny, lny;  // lny = log2(ny)
-    int paired;       // real fields share transforms two by two (explicit.cu)
     const double *kx, *ky, *k2;
 };
 
-inline bool paired_grid(const KGrid& g) { return g.paired != 0; }
-
 struct KspaceArgs {
     KGrid g;
-    const double2* Jhat;       // (Jx, Jy), Jz transforms when paired, else Jx, Jy, Jz
-    const double2* rho_dep;    // naive charge spectrum or null
+    const double2* Jhat;       // 3 x N
+    const double2* rho_dep;    // N (naive charge spectrum) or null
     double2* hist;             // ring: [field(5: phi, Ax, Ay, Az, rho)][slot R][N]
     int R, head;               // slots; head = slot of u^n
     int na;                    // BDF coefficients a[0..na), 2 or 3
@@ -264,7 +247,7 @@ struct KspaceArgs {
     double b[5];               // their convolution, 2 na - 1 of them
     double dt, c, eps0, mu0;
     int conserving;
-    double2* gspec;            // spectra of the gathered fields: 6 transforms when paired, else 11
+    double2* gspec;            // 11 x N gather-field spectra (output)
 };
 cudaError_t launch_bdf_kspace(const KspaceArgs& a, cudaStream_t st);
 
@@ -272,7 +255,7 @@ cudaError_t launch_bdf_kspace(const KspaceArgs& a, cudaStream_t st);
 // 5, B 6..8, rho 9.
 struct DiagArgs {
     KGrid g;
-    const double2* Jhat;          // as in KspaceArgs
+    const double2* Jhat;          // 3 x N
     const double2* hist;
     int R, slot_new, slot_prev0;  // u^{n+1} slot; past(0) slot
     int na;
