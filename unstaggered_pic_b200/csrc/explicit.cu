@@ -34,6 +34,9 @@ constexpr int kPushWarps = kPushThreads / kWarp;
 // With private windows two CTAs fit an SM and their threads keep their values
 // in registers.
 constexpr int push_min_blocks(bool priv) { return priv ? 2 : UPIC_PUSH_MIN_BLOCKS; }
+// Particles staged at a time for private windows: with four components two
+// CTAs fit an SM only with half a warp's (107 KB; 120 KB with all).
+constexpr int push_rows(int ncomp) { return ncomp == 4 ? 16 : 32; }
 constexpr int kKeyNone = -1;
 constexpr int kKeyEscape = -2;
 
@@ -122,7 +125,7 @@ UPIC_D void prefetch_next_batch(const PushArgs& a, const Chunk& ch, int base, in
     prefetch_l2(arr, n0, n1);
 }
 
-// PRIV: warp-private FP64 windows (deposit.cuh); otherwise the CTA shares one
+// PRIV: warp-private windows (deposit.cuh); otherwise the CTA shares one
 // window of fixed-point words, to which each group of equal cells of a warp
 // adds its sums.
 template <int MODE, int NCOMP, bool UNIFORM, bool PRIV>
@@ -139,8 +142,10 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
     const PrivateWindow pw = private_window(tg, 3, 3);
     const int psize = pw.ex * pw.ey * NCOMP;
     double* wins = reinterpret_cast<double*>(smem_u64);
-    constexpr int STAGE = PRIV ? RW * kColStride : StageLayout<NCOMP>::kDoubles;  // doubles staged per warp
-    const int window_words = PRIV ? (kPushWarps * psize + 1) & ~1 : 2 * NCOMP * WN;
+    int* lost = reinterpret_cast<int*>(wins + kPushWarps * psize);
+    constexpr int ROWS = push_rows(NCOMP), CS = col_stride(ROWS);
+    constexpr int STAGE = PRIV ? RW * CS : StageLayout<NCOMP>::kDoubles;  // doubles staged per warp
+    const int window_words = PRIV ? (kPushWarps * psize * 3 / 2 + 1) & ~1 : 2 * NCOMP * WN;
     double* sprod = reinterpret_cast<double*>(smem_u64 + window_words) + warp * STAGE;
     int* sgk = reinterpret_cast<int*>(smem_u64 + window_words + kPushWarps * STAGE) + warp * 32;
     // field records of the tile's window (kModePush): the gathers of
@@ -183,7 +188,7 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
     int cur_tile = -1, ox = 0, oy = 0;
     auto fold = [&]() {
         if constexpr (PRIV)
-            fold_private<NCOMP, kPushWarps>(wins, psize, pw, tg, ox, oy, a.acc, a.scale,
+            fold_private<NCOMP, kPushWarps>(wins, lost, psize, pw, tg, ox, oy, a.acc, a.scale,
                                             [](int c) { return acc_slot(NCOMP, c); });
         else
             fold_window<NCOMP>(whi, wlo, WN, tg, ox, oy, a.acc);
@@ -351,45 +356,56 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                 const unsigned full = 0xffffffffu;
                 const unsigned valid = __ballot_sync(full, key >= 0);
                 const unsigned esc = __ballot_sync(full, key == kKeyEscape);
-                const unsigned heads = run_heads(key, valid);
-                double* mine = sprod + lane;
+                const Groups gr = group_rows(key, valid);
+                double* mine = sprod + gr.row % ROWS;
+                unsigned leaders = gr.leaders;
+                int cur_key = 0;
 #pragma unroll
-                for (int ia = 0; ia < 3; ++ia)
+                for (int first = 0; first < 32; first += ROWS) {
+                    const bool here = gr.row / ROWS * ROWS == first;
+                    if (here) {
 #pragma unroll
-                    for (int ib = 0; ib < 3; ++ib)
-                        mine[(ia * 3 + ib) * kColStride] = key == kKeyNone ? 0.0 : dwx[ia] * dwy[ib];
+                        for (int ia = 0; ia < 3; ++ia)
 #pragma unroll
-                for (int cc = 0; cc < NCOMP; ++cc) mine[(9 + cc) * kColStride] = key == kKeyNone ? 0.0 : dval[cc];
-                __syncwarp();
-                if (esc) {
-                    // stencils that leave the window (rare): exact fixed-point
-                    // adds straight to the grid, then nothing for the window
-                    for (unsigned e = esc; e; e &= e - 1) {
-                        const int j = __ffs(e) - 1;
-                        const int gxj = __shfl_sync(full, gx0, j);
-                        const int gyj = __shfl_sync(full, gy0, j);
+                            for (int ib = 0; ib < 3; ++ib)
+                                mine[(ia * 3 + ib) * CS] = key == kKeyNone ? 0.0 : dwx[ia] * dwy[ib];
 #pragma unroll
-                        for (int r = 0; r < NPER; ++r) {
-                            if (lane + 32 * r < NV) {
-                                const double v = sprod[(9 + t_c[r]) * kColStride + j] * sprod[t_ab[r] * kColStride + j];
-                                if (v != 0.0) {
-                                    const int g = wrap_index(gxj + t_a[r], nx) * ny + wrap_index(gyj + t_b[r], ny);
-                                    const int sl = acc_slot(NCOMP, t_c[r]);
-                                    const Fixed2 f = to_fixed(v, a.scale[sl]);
-                                    atomicAdd(&a.acc[(size_t)(2 * sl) * N + g], f.hi);
-                                    atomicAdd(&a.acc[(size_t)(2 * sl + 1) * N + g], f.lo);
+                        for (int cc = 0; cc < NCOMP; ++cc) mine[(9 + cc) * CS] = key == kKeyNone ? 0.0 : dval[cc];
+                    }
+                    __syncwarp();
+                    if (esc) {
+                        // stencils that leave the window (rare): exact fixed-point
+                        // adds straight to the grid, then nothing for the window
+                        for (unsigned e = __ballot_sync(full, here && key == kKeyEscape); e; e &= e - 1) {
+                            const int l = __ffs(e) - 1, j = __shfl_sync(full, gr.row, l) % ROWS;
+                            const int gxj = __shfl_sync(full, gx0, l);
+                            const int gyj = __shfl_sync(full, gy0, l);
+#pragma unroll
+                            for (int r = 0; r < NPER; ++r) {
+                                if (lane + 32 * r < NV) {
+                                    const double v = sprod[(9 + t_c[r]) * CS + j] * sprod[t_ab[r] * CS + j];
+                                    if (v != 0.0) {
+                                        const int g = wrap_index(gxj + t_a[r], nx) * ny + wrap_index(gyj + t_b[r], ny);
+                                        const int sl = acc_slot(NCOMP, t_c[r]);
+                                        const Fixed2 f = to_fixed(v, a.scale[sl]);
+                                        atomicAdd(&a.acc[(size_t)(2 * sl) * N + g], f.hi);
+                                        atomicAdd(&a.acc[(size_t)(2 * sl + 1) * N + g], f.lo);
+                                    }
                                 }
                             }
                         }
-                    }
-                    __syncwarp();
-                    if (key == kKeyEscape)
+                        __syncwarp();
+                        if (here && key == kKeyEscape)
 #pragma unroll
-                        for (int cc = 0; cc < NCOMP; ++cc) mine[(9 + cc) * kColStride] = 0.0;
+                            for (int cc = 0; cc < NCOMP; ++cc) mine[(9 + cc) * CS] = 0.0;
+                        __syncwarp();
+                    }
+                    const int nrows = min(__popc(valid) - first, ROWS);
+                    if (nrows > 0)
+                        add_columns<NV, 9, ROWS, NPER>(sprod, key, leaders, cur_key, nrows, gr.heads >> first,
+                                                       wins + warp * psize, lost + warp * psize, t_ab, t_c, t_off);
                     __syncwarp();
                 }
-                if (valid)
-                    add_columns<NV, 9, NPER>(sprod, key, valid, heads, wins + warp * psize, t_ab, t_c, t_off);
                 continue;
             }
             // Group the warp's particles by window key: groups in the order of
@@ -928,9 +944,8 @@ int grid_for(long n, int threads) {
 // Shared memory of the push kernels with private or shared windows.
 int push_smem(const TileGeom& tg, int ncomp, bool priv) {
     const int records = 16 + tg.wx * tg.wy * kGFStride * 8;
-    const int windows = priv ? kPushWarps * private_window_doubles(tg, 3, 3, ncomp) * 8 + 8
-                             : 2 * ncomp * tg.wx * tg.wy * 8;
-    const int stage = priv ? kPushWarps * (9 + ncomp) * kColStride * 8
+    const int windows = priv ? private_window_bytes(tg, 3, 3, ncomp, kPushWarps) + 8 : 2 * ncomp * tg.wx * tg.wy * 8;
+    const int stage = priv ? kPushWarps * (9 + ncomp) * col_stride(push_rows(ncomp)) * 8
                            : kPushWarps * (32 * (9 + ncomp) * 8 + 32 * 4);
     const int bytes = windows + stage + records;
     const int red = kPushWarps * 5 * 8;
@@ -938,10 +953,10 @@ int push_smem(const TileGeom& tg, int ncomp, bool priv) {
 }
 
 // Private windows while two CTAs fit an SM, as with the default tile of 8
-// cells (83 KB, 98 KB with the charge); larger windows stay shared.  A launch
-// with shared and with private windows, chunks of 2048: 32 x 32 x 16 36 and 30
-// us, 64 x 64 x 64 64 and 47 us, 256 x 128 x 32 184 and 121 us, 512 x 512 x 64
-// 1480 and 1434 us.
+// cells (99 KB, 107 KB with the charge); larger windows stay shared.  A launch
+// with shared windows and chunks of 2048, and one with private windows:
+// 32 x 32 x 16 36 and 28 us, 64 x 64 x 64 64 and 29 us, 256 x 128 x 32 with the
+// charge 184 and 119 us, 512 x 512 x 64 1480 and 1447 us.
 bool push_private(const TileGeom& tg, int ncomp) { return push_smem(tg, ncomp, true) <= 113 * 1024; }
 
 using PushKernel = void (*)(PushArgs, TileGeom);

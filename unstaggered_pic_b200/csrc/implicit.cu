@@ -38,11 +38,11 @@ constexpr int kMapThreads = 128;
 #endif
 constexpr int solve_min_blocks(bool mom) { return mom ? UPIC_SOLVE_MIN_BLOCKS : UPIC_SOLVE_POINTS_MIN_BLOCKS; }
 // Resident CTAs per SM of the deposit.  With private windows shared memory
-// allows five to six CTAs of a quadratic 2D tile and four of a cubic one,
-// which leaves registers for them; with the shared window 8 for one item per
-// segment and 6 for one per quadrature point measured best.
+// allows four CTAs of a quadratic 2D tile and three of a cubic one, which
+// leaves registers for them; with the shared window 8 for one item per segment
+// and 6 for one per quadrature point measured best.
 constexpr int deposit_min_blocks(int order, bool mom, bool picard, bool priv) {
-    return priv ? (order >= 3 ? 4 : 5) : picard ? 3 : mom ? 8 : 6;
+    return priv ? (order >= 3 ? 3 : 4) : picard ? 3 : mom ? 8 : 6;
 }
 constexpr int kMapWarps = kMapThreads / kWarp;
 constexpr int kKeyNone = -1;
@@ -1200,11 +1200,11 @@ implicit_solve_closed_kernel(ImplicitMapArgs a, int nx, int ny) {
 // fixed-point sums.  PICARD: the deposit of the non-relativistic Picard map
 // (evaluate_picard_map_orbit, Project1/ec_pic_serial_demo.cpp:1455-1474),
 // whose orbit velocity is vbar = (v_guess + v^n) / 2 with no local solve.
-// PRIV: closed-form shape sums into warp-private FP64 windows (deposit.cuh);
+// PRIV: closed-form shape sums into warp-private windows (deposit.cuh);
 // otherwise segment moments (MOM) or quadrature points, and the CTA shares
 // one window of fixed-point words, to which each group of equal cells of a
-// warp adds its sums.  512 x 512 x 16 quadratic 0.70 -> 0.37 ms a launch, 256
-// x 256 x 16 cubic 0.74 -> 0.10 ms (one item per segment instead of four).
+// warp adds its sums.  512 x 512 x 16 quadratic 0.70 -> 0.42 ms a launch, 256
+// x 256 x 16 cubic 0.74 -> 0.13 ms (one item per segment instead of four).
 template <int ORDER, bool UNIFORM, bool MOM, bool PICARD, int SY, bool PRIV>
 __global__ void __launch_bounds__(kMapThreads, deposit_min_blocks(ORDER, MOM, PICARD, PRIV))
 implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
@@ -1212,7 +1212,8 @@ implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
     constexpr int SS = S * SY;
     constexpr int NV = 3 * SS;
     constexpr int RW = SS + 3;
-    constexpr int STAGE = PRIV ? RW * kColStride : 32 * RW;  // doubles staged per warp
+    constexpr int CS = col_stride(32);
+    constexpr int STAGE = PRIV ? RW * CS : 32 * RW;  // doubles staged per warp
     constexpr int NPER = (NV + 31) / 32;
     extern __shared__ unsigned long long smem_u64[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1222,7 +1223,8 @@ implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
     unsigned long long* whi = smem_u64;
     unsigned long long* wlo = whi + 3 * WN;
     double* wins = reinterpret_cast<double*>(smem_u64);
-    const int window_words = PRIV ? kMapWarps * psize : 6 * WN;
+    int* lost = reinterpret_cast<int*>(wins + kMapWarps * psize);
+    const int window_words = PRIV ? kMapWarps * psize * 3 / 2 : 6 * WN;
     double* srow = reinterpret_cast<double*>(smem_u64 + ((window_words + 1) & ~1)) + warp * STAGE;
     int* sgk = reinterpret_cast<int*>(reinterpret_cast<double*>(smem_u64 + ((window_words + 1) & ~1)) +
                                       kMapWarps * STAGE) +
@@ -1256,7 +1258,7 @@ implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
     int cur_tile = -1, ox = 0, oy = 0;
     auto fold = [&]() {
         if constexpr (PRIV) {
-            fold_private<3, kMapWarps>(wins, psize, pw, tg, ox, oy, a.acc, a.scale, [](int c) { return c; });
+            fold_private<3, kMapWarps>(wins, lost, psize, pw, tg, ox, oy, a.acc, a.scale, [](int c) { return c; });
         } else {
             for (int idx = threadIdx.x; idx < 3 * WN; idx += blockDim.x) {
                 const unsigned long long hi = whi[idx], lo = wlo[idx];
@@ -1406,8 +1408,9 @@ implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
                 const unsigned esc = __ballot_sync(full, key == kKeyEscape);
                 int row = -1, nvalid = 0;
                 unsigned heads = 0u;
+                Groups gr{};
                 if constexpr (PRIV) {
-                    heads = run_heads(key, valid);
+                    gr = group_rows(key, valid);
                 } else {
                     const unsigned peers = __match_any_sync(full, key);
                     int ngroups = 0;
@@ -1425,8 +1428,8 @@ implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
                 }
                 if (!PRIV && key == kKeyEscape) row = nvalid + __popc(esc & lt);
                 // value k of this lane's particle goes to mine[k * step]
-                double* mine = PRIV ? srow + lane : srow + row * RW;
-                constexpr int step = PRIV ? kColStride : 1;
+                double* mine = PRIV ? srow + gr.row : srow + row * RW;
+                constexpr int step = PRIV ? CS : 1;
                 if (PRIV && key == kKeyNone) {
 #pragma unroll
                     for (int k = 0; k < RW; ++k) mine[k * step] = 0.0;
@@ -1451,11 +1454,12 @@ implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
                         e &= e - 1;
                         const int gxj = __shfl_sync(full, gx0, j);
                         const int gyj = __shfl_sync(full, gy0, j);
+                        const int rj = PRIV ? __shfl_sync(full, gr.row, j) : 0;
 #pragma unroll
                         for (int r = 0; r < NPER; ++r) {
                             const int t = lane + 32 * r;
                             if (t < NV) {
-                                const double v = PRIV ? srow[(SS + t_c[r]) * step + j] * srow[t_ab[r] * step + j]
+                                const double v = PRIV ? srow[(SS + t_c[r]) * step + rj] * srow[t_ab[r] * step + rj]
                                                       : srow[erow * RW + SS + t_c[r]] * srow[erow * RW + t_ab[r]];
                                 if (v != 0.0) {
                                     const int gi = wrap_index(gxj + t_a[r], nx) * ny + wrap_index(gyj + t_b[r], ny);
@@ -1476,7 +1480,10 @@ implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
                     __syncwarp();
                 }
                 if constexpr (PRIV) {
-                    if (valid) add_columns<NV, SS>(srow, key, valid, heads, wins + warp * psize, t_ab, t_c, t_off);
+                    int cur = 0;
+                    if (valid)
+                        add_columns<NV, SS, 32>(srow, key, gr.leaders, cur, __popc(valid), gr.heads, wins + warp * psize,
+                                                lost + warp * psize, t_ab, t_c, t_off);
                 } else {
                     unsigned h = heads;
                     int gi = 0;
@@ -3244,18 +3251,20 @@ namespace {
 // Shared memory of the deposit launch with private or shared windows.
 int deposit_smem(const TileGeom& tg, int order, bool priv) {
     const int S = order + 1, row = S * S + 3;
-    if (priv) return kMapWarps * (private_window_doubles(tg, S, S, 3) + row * kColStride) * 8 + 8;
+    if (priv) return private_window_bytes(tg, S, S, 3, kMapWarps) + kMapWarps * row * col_stride(32) * 8 + 8;
     return 2 * 3 * tg.wx * tg.wy * 8 + kMapWarps * (32 * row * 8 + 32 * 4);
 }
 
-// Private windows where the closed form holds and four CTAs fit an SM (the
-// default tile of 8 cells takes 30-52 KB); a larger tile, a user's choice,
-// keeps the shared window, which needs a quarter to a half of the memory.  So
-// does a grid one cell high: its few nodes hold many particles each, so that
-// the deposit is small beside the solve (37 and 103 us at 150,000 particles)
-// and the order of its sums shows in the last residual.
+// Private windows where the closed form holds and three CTAs fit an SM (the
+// default tile of 8 cells takes 31-70 KB, more where orbits reach beyond a
+// cell).  A 128 x 128 x 32 quartic step of the non-relativistic method, 70 KB,
+// takes 2.74 ms with private and 7.77 ms with shared windows.
+// A larger tile, a user's choice, keeps the shared window, which needs a
+// quarter to a half of the memory.  So does a grid one cell high: its few
+// nodes hold many particles each, so that the deposit is small beside the
+// solve (37 and 103 us at 150,000 particles).
 bool deposit_private(const TileGeom& tg, int order, bool closed) {
-    return closed && tg.ny > 1 && deposit_smem(tg, order, true) <= 55 * 1024;
+    return closed && tg.ny > 1 && deposit_smem(tg, order, true) <= 75 * 1024;
 }
 
 }  // namespace
