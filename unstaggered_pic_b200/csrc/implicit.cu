@@ -1096,10 +1096,9 @@ implicit_solve_closed_kernel(ImplicitMapArgs a, int nx, int ny) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) in.pstart[c] = in.P0[c] - in.q * in.A0p[c];
             set_local_constants(in, a.kappa);
-            const double* const* start = a.warm_x ? &a.warm_x : &a.vx;
-            guess[0] = start[0][p];
-            guess[1] = start[1][p];
-            guess[2] = start[2][p];
+            guess[0] = a.warm_x ? a.warm_x[p] : a.vx[p];
+            guess[1] = a.warm_x ? a.warm_y[p] : a.vy[p];
+            guess[2] = a.warm_x ? a.warm_z[p] : a.vz[p];
             int reason = kLocalMaxIter, iters = 0;
             double g2 = dot3(guess, guess), r2 = INFINITY, tol = 1.0;
             ClosedOut o;
