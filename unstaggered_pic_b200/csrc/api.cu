@@ -126,12 +126,14 @@ int choose_chunk(long np, int grid, int max_chunk, int unit) {
 }
 
 // Particles per push chunk: 2048, or 1024 while that leaves resident CTAs
-// without a chunk.  Each chunk clears and folds its windows once, which many
-// small runs side by side pay in SM time and one small run alone gains back
-// in latency.  A smallest chunk of 256 / 512 / 1024 / 2048 takes
-//   32 x 32 x 16, 50 steps alone             3.71 / 3.78 / 4.33 / 4.56 ms
-//   64 x 64 x 64, 50 steps alone             5.37 / 5.25 / 5.24 / 6.26 ms
-//   32 runs of 1e4..1e5, 120 steps, a graph  34.2 / 31.7 / 30.5 / 30.2 ms
+// without a chunk.  A CTA clears its windows once and stages the records and
+// folds the windows once per tile it visits; where chunks are fewer than CTAs
+// each chunk has a CTA of its own, so a finer split repeats that work, which
+// many small runs side by side pay in SM time and one small run alone gains
+// back in latency.  A smallest chunk of 256 / 512 / 1024 / 2048 takes
+//   32 x 32 x 16, 50 steps alone             3.43 / 3.62 / 4.16 / 4.41 ms
+//   64 x 64 x 64, 50 steps alone             5.03 / 5.03 / 5.04 / 6.01 ms
+//   32 runs of 1e4..1e5, 120 steps, a graph  35.9 / 33.1 / 31.8 / 31.1 ms
 // A run of an ensemble sums in the same order as the run alone, so both take
 // one rule.
 int push_chunk(const upic_ctx* c) { return choose_chunk(c->np, c->push_grid, 2048, 1024); }
@@ -760,8 +762,8 @@ int upic_create(const upic_config* cfg, upic_ctx** out) {
         (rc = dalloc(c, &c->d_rho, N)) || (rc = dalloc(c, &c->d_gf, (size_t)kGFStride * N)) ||
         (rc = dalloc(c, &c->d_spec, 16 * (size_t)N)) ||
         (rc = dalloc(c, &c->d_hist, 5 * (size_t)kHistSlots * N)) ||
-        (rc = dalloc(c, &c->d_dspec, (size_t)kDiagFields * N)) ||
-        (rc = dalloc(c, &c->d_dreal, (size_t)kDiagFields * N)) ||
+        (rc = dalloc(c, &c->d_dspec, (size_t)kSpecGrids * N)) ||
+        (rc = dalloc(c, &c->d_dreal, (size_t)kRealGrids * N)) ||
         (rc = dalloc(c, &c->d_partials, (size_t)kRedGrid * 16)) ||
         (rc = dalloc(c, &c->d_pdiag, (size_t)c->push_grid * kDiagPart)) ||
         (rc = dalloc(c, &c->d_done, 1)) || (rc = dalloc(c, &c->d_scan, 3)) ||

@@ -2396,7 +2396,6 @@ extern "C" int upic_push_gmhc(upic_ctx* c, long np, const double* x, const doubl
     a.loc_maxit = cf.local_max_iter;
     a.qtab = s.qtab;
     a.nq = s.nq;
-    a.closed = s.closed ? 1 : 0;
     UPIC_CUDA(c, launch_gmhc_push(s.order, a, c->nx, c->ny, np, din, dg, dout, drep, c->st));
     std::vector<double> out(11 * (size_t)np);
     UPIC_CUDA(c, cudaMemcpyAsync(out.data(), dout, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, c->st));

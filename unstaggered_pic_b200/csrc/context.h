@@ -16,7 +16,7 @@
 namespace upic_host {
 
 constexpr int kHistSlots = 5;
-constexpr int kDiagFields = 10;
+constexpr int kSpecGrids = 6, kRealGrids = 5;  // scratch grids of the field entry points
 constexpr int kRedGrid = 148 * 2;
 constexpr int kRowRing = 64;  // diagnostics rows a step call keeps before it hands them over
 

@@ -29,14 +29,9 @@ constexpr int kMapThreads = 128;
 // takes the orbit velocities through global memory: the solve's code and
 // registers stay free of the deposit machinery and each has its own
 // occupancy.
-// Resident CTAs per SM of the local solve.
-#ifndef UPIC_SOLVE_MIN_BLOCKS
-#define UPIC_SOLVE_MIN_BLOCKS 4
-#endif
-#ifndef UPIC_SOLVE_POINTS_MIN_BLOCKS
-#define UPIC_SOLVE_POINTS_MIN_BLOCKS 4
-#endif
-constexpr int solve_min_blocks(bool mom) { return mom ? UPIC_SOLVE_MIN_BLOCKS : UPIC_SOLVE_POINTS_MIN_BLOCKS; }
+// Resident CTAs per SM of the local solve (Gauss rule), and of its closed form.
+constexpr int kSolveMinBlocks = 4;
+constexpr int solve_closed_min_blocks(int order) { return order >= 3 ? 3 : 4; }
 // Resident CTAs per SM of the deposit.  With private windows shared memory
 // allows four CTAs of a quadratic 2D tile and three of a cubic one, which
 // leaves registers for them; with the shared window 8 for one item per segment
@@ -756,47 +751,40 @@ UPIC_D bool orbit_averages(const Geo& g, const double* __restrict__ rec, double 
     return walk.nb == 0;
 }
 
-// Shape sums len <S_a S_b> of the segment [sa, sb] to out[(a SY + b) STEP].
-template <int R, int SY, int STEP>
+// Shape sums len <S_a S_b> of the segment [sa, sb] to out[(a (R + 1) + b) STEP].
+template <int R, int STEP>
 UPIC_D void segment_weights(double ux, double uy, double dux, double duy, double sa, double sb, double* out) {
     const double len = sb - sa, sm = sa + 0.5 * len;
     const double dx = len * dux, dy = len * duy;
-    double tx, ty = 0.0;
+    double tx, ty;
     segment_cell(ux + sm * dux, tx);
-    if constexpr (SY > 1) segment_cell(uy + sm * duy, ty);
+    segment_cell(uy + sm * duy, ty);
     double wx[R + 1], Gx[R][R + 1], wy[R + 1], Gy[R][R + 1];
     spline_taylor<R>(tx, dx, wx, Gx);
-    if constexpr (SY > 1) spline_taylor<R>(ty, dy, wy, Gy);
+    spline_taylor<R>(ty, dy, wy, Gy);
 #pragma unroll 1
-    for (int b = 0; b < SY; ++b) {
+    for (int b = 0; b <= R; ++b) {
         double U[R + 1];
 #pragma unroll
         for (int i = 0; i <= R; ++i) {
-            if constexpr (SY > 1) {
-                double u = 0.0;
+            double u = 0.0;
 #pragma unroll
-                for (int j = 0; j <= R; ++j)
-                    if (!((i + j) & 1)) u = fma(tau_moment(i + j), taylor<R>(wy, Gy, dy, j, 0), u);
-                U[i] = len * u;
-            } else {
-                U[i] = len * tau_moment(i);
-            }
+            for (int j = 0; j <= R; ++j)
+                if (!((i + j) & 1)) u = fma(tau_moment(i + j), taylor<R>(wy, Gy, dy, j, 0), u);
+            U[i] = len * u;
         }
-        if constexpr (SY > 1) {
 #pragma unroll
-            for (int k = 0; k < R; ++k) {
-                wy[k] = wy[k + 1];
+        for (int k = 0; k < R; ++k) {
+            wy[k] = wy[k + 1];
 #pragma unroll
-                for (int i = 0; i < R; ++i) Gy[i][k] = Gy[i][k + 1];
-            }
+            for (int i = 0; i < R; ++i) Gy[i][k] = Gy[i][k + 1];
         }
 #pragma unroll
         for (int a = 0; a <= R; ++a) {
             double m = 0.0;
 #pragma unroll
-            for (int i = 0; i <= R; ++i)
-                if (SY > 1 || !(i & 1)) m = fma(taylor<R>(wx, Gx, dx, i, a), U[i], m);
-            out[(a * SY + b) * STEP] = m;
+            for (int i = 0; i <= R; ++i) m = fma(taylor<R>(wx, Gx, dx, i, a), U[i], m);
+            out[(a * (R + 1) + b) * STEP] = m;
         }
     }
 }
@@ -928,7 +916,7 @@ UPIC_D Geo map_geo(const ImplicitMapArgs& a, int nx, int ny) {
 // segments and so in time, and a fixed stride gave the same CTAs the long
 // ones (SMs active 63% of the launch).
 template <int ORDER, bool UNIFORM, bool MOM, int SY>
-__global__ void __launch_bounds__(kMapThreads, solve_min_blocks(MOM))
+__global__ void __launch_bounds__(kMapThreads, kSolveMinBlocks)
 implicit_solve_kernel(ImplicitMapArgs a, int nx, int ny) {
     const Geo g = map_geo(a, nx, ny);
     unsigned long long it_total = 0;
@@ -1065,10 +1053,11 @@ implicit_solve_kernel(ImplicitMapArgs a, int nx, int ny) {
 // implicit_solve_kernel for large 2D sets (ImplicitMapArgs::closed_solve) with
 // the orbit integrals in closed form.  512 x 512 x 16 quadratic: 2.33 -> 1.38
 // ms a launch, 256 x 256 x 16 cubic 1.22 -> 0.53 ms (FP64 work per segment 410
-// -> 340 instructions quadratic, 64 record loads for 256 cubic; registers 168
-// with 344 B of spills -> 128).
+// -> 340 instructions quadratic, 64 record loads for 256 cubic).  Bound by
+// FP64 issue and the record loads in the chain: 128 registers (168 from cubic
+// splines on) with 0.3-0.8 KB of spills a thread.
 template <int ORDER, bool UNIFORM>
-__global__ void __launch_bounds__(kMapThreads, ORDER >= 3 ? 3 : 4)
+__global__ void __launch_bounds__(kMapThreads, solve_closed_min_blocks(ORDER))
 implicit_solve_closed_kernel(ImplicitMapArgs a, int nx, int ny) {
     const Geo g = map_geo(a, nx, ny);
     const double kappa2 = a.kappa * a.kappa;
@@ -1435,7 +1424,7 @@ implicit_deposit_kernel(ImplicitMapArgs a, TileGeom tg) {
                 }
                 if (PRIV ? key != kKeyNone : row >= 0) {
                     if constexpr (PRIV) {
-                        segment_weights<ORDER, SY, step>(ux, uy, dux, duy, sa, sb, mine);
+                        segment_weights<ORDER, step>(ux, uy, dux, duy, sa, sb, mine);
                     } else {
 #pragma unroll
                         for (int j = 0; j < SS; ++j) mine[j] = wgt[j];
@@ -3299,8 +3288,7 @@ cudaError_t launch_implicit_map(int order, bool uniform, const TileGeom& tg, con
                                               : solve_kernel(order, uniform, a.split != 0, tg.ny == 1);
         if (!ks) return cudaErrorInvalidValue;
         const long blocks = (a.np + kMapThreads - 1) / kMapThreads;
-        const bool mom = a.split && (order <= 2 || tg.ny == 1);
-        const int resident = nsm * (a.closed_solve ? (order >= 3 ? 3 : 4) : solve_min_blocks(mom));
+        const int resident = nsm * (a.closed_solve ? solve_closed_min_blocks(order) : kSolveMinBlocks);
         ks<<<(int)(blocks < resident ? blocks : resident), kMapThreads, 0, st>>>(a, tg.nx, tg.ny);
         count_launches(1);
     }

@@ -119,13 +119,14 @@ cudaError_t implicit_configure_smem(const TileGeom& tg, int order, bool split, b
 // Resident CTAs per SM of the deposit.
 int implicit_deposit_occupancy(const TileGeom& tg, int order, bool split, bool closed, bool picard);
 // The local solves take their orbit integrals in closed form from this many
-// particles on (2D).  Which iterate a particle's fixed point stops at turns on
-// single roundings, and each particle that stops elsewhere than with the Gauss
-// rule's roundings moves the mean iteration count by 1 / np and the last
-// residual, with the convergence rate reported from it, by about 1e-12 / np
-// of the current: from half a million particles on both stay below 1e-9 of
-// the report's values, below it a step is latency (64 x 64 x 16: 71 us of 430
-// per map evaluation).
+// particles on (2D).  The line is drawn by the step's report, neither by
+// accuracy, which is the same, nor by time: at 64 x 64 x 16 a launch takes 41
+// us in closed form and 64 us with the Gauss rule, a step 1.71 and 1.86 ms.
+// Which iterate a particle's fixed point stops at turns on single roundings,
+// and each particle that stops elsewhere than with the Gauss rule's roundings
+// moves the mean iteration count by 1 / np and the last residual, with the
+// convergence rate reported from it, by about 1e-12 / np of the current: from
+// half a million particles on both stay below 1e-9 of the report's values.
 constexpr long kClosedSolveMin = 1L << 19;
 
 // Point deposit of rho (q S / dV, slot 3) and J (q v S / dV, slots 0..2) at
