@@ -700,13 +700,13 @@ def measure(args, name, steps, warmup, world, rank, dist, dev, predictor="previo
         achieved = alg_bytes / (kern_ms / 1e3) / 1e9
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                     "frac": achieved / peak, "traffic": None, "peak_source": peak_kind,
-                    "kernel": "implicit_map_kernel (per-particle local GM-HC solve + orbit-averaged "
-                              "current deposit)",
+                    "kernel": "implicit_solve_closed_kernel + implicit_deposit_kernel (per-particle local "
+                              "GM-HC solve, orbit-averaged current deposit)",
                     "kernel_ms": kern_ms / max(kern_n, 1), "kernel_launches": kern_n,
                     "kernel_share": kern_ms / t_ms,
                     "algorithmic_bytes_per_particle_launch": IMPLICIT_READ_BYTES,
-                    "note": "FP64-issue bound (local fixed point with orbit quadrature per particle "
-                            "per launch); HBM fraction stated for the streamed particle state"}
+                    "note": "bound by the L1 data pipe and FP64 issue (local fixed point over the orbit's "
+                            "node records); HBM fraction stated for the streamed particle state"}
         solve = {"outer_iterations_per_step": float(np.mean(info[:, 0])),
                  "map_evaluations_per_step": kern_n / steps,
                  "local_iterations_mean": float(np.mean(info[:, 5])),

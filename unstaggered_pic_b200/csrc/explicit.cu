@@ -260,7 +260,7 @@ push_deposit_kernel(PushArgs a, TileGeom tg) {
                                 }
                                 // the last field alone: the record's padding would
                                 // take its share of the shared-memory return path,
-                                // which bounds this kernel (75% busy)
+                                // which bounds this kernel (71% busy)
                                 G[kGF - 1] = fma(reinterpret_cast<const double*>(rec)[kGF - 1], w, G[kGF - 1]);
                             }
                         }

@@ -1053,9 +1053,10 @@ implicit_solve_kernel(ImplicitMapArgs a, int nx, int ny) {
 // implicit_solve_kernel for large 2D sets (ImplicitMapArgs::closed_solve) with
 // the orbit integrals in closed form.  512 x 512 x 16 quadratic: 2.33 -> 1.38
 // ms a launch, 256 x 256 x 16 cubic 1.22 -> 0.53 ms (FP64 work per segment 410
-// -> 340 instructions quadratic, 64 record loads for 256 cubic).  Bound by
-// FP64 issue and the record loads in the chain: 128 registers (168 from cubic
-// splines on) with 0.3-0.8 KB of spills a thread.
+// -> 340 instructions quadratic, 64 record loads for 256 cubic).  Bound by the
+// L1 data pipe, 90% busy with the record loads (quadratic), then by FP64 issue,
+// 54%; 128 registers (168 from cubic splines on) with 0.3-0.8 KB of spills a
+// thread.
 template <int ORDER, bool UNIFORM>
 __global__ void __launch_bounds__(kMapThreads, solve_closed_min_blocks(ORDER))
 implicit_solve_closed_kernel(ImplicitMapArgs a, int nx, int ny) {
