@@ -32,6 +32,9 @@ thread_local std::string g_create_error;
 namespace upic_host {
 
 int fail(upic_ctx* c, int code, const std::string& msg) {
+    // a failed runtime call leaves its error behind in this thread, where the
+    // next launch, of another context perhaps, would take it for its own
+    (void)cudaGetLastError();
     if (c) c->err = msg;
     else g_create_error = msg;
     return code;
